@@ -51,6 +51,7 @@ constexpr int kDopThreads = 128;
 constexpr int kDopTriples = 14 * 13 * 12 / 6;  // 364 plane triples of the 14-DOP
 constexpr int kDopBlocks = (kDopTriples + kDopThreads - 1) / kDopThreads;
 constexpr int kDopPer = (kDopTriples + kDopThreads - 1) / kDopThreads;  // triples per thread when merging
+constexpr int kPlocMaxRounds = 64;  // grid-wide PLOC rounds (ploc_grid_rounds stays below it for 2^28 primitives)
 constexpr int kSortItems = 8;
 constexpr uint32_t kSortTile = kSortThreads * kSortItems;
 
@@ -63,9 +64,9 @@ struct BuildState {
     uint32_t error;
     uint32_t depth;
     uint32_t blas_kinds;  // TLAS: kBlasKind* bits of the BLASes its instances enter
-    uint32_t ploc_count[2];  // PLOC clusters entering the round (double-buffered by round parity)
+    uint32_t ploc_round[kPlocMaxRounds + 1];  // PLOC clusters entering each round | kPloc* bits
+    uint32_t ploc_ticket[kPlocMaxRounds];     // next tile of each round
     uint32_t merge_counter;  // PLOC merges so far (internal node ids count down from n - 2)
-    uint32_t ploc_blocks_done;  // blocks of the current merge launch that have finished
     uint32_t radius_bits;    // BLAS: largest vertex distance from the bounds centre (float bits, rounded up)
     uint32_t dop_hi[7], dop_lo[7];  // BLAS: largest / smallest vertex projection on each 14-DOP axis (ordered uint)
     uint32_t dop_blocks_done;       // blocks of k_dop_vertices that have finished
@@ -149,8 +150,10 @@ __device__ void reduce_bounds(BuildState* st, const float cmin[3], const float c
     }
 }
 
-__global__ void k_init_state(BuildState* st) {
+__global__ void k_init_state(BuildState* st, uint32_t n) {
+    for (uint32_t i = threadIdx.x; i < kPlocMaxRounds; i += blockDim.x) st->ploc_ticket[i] = 0;
     if (threadIdx.x == 0) {
+        st->ploc_round[0] = n;
         for (int k = 0; k < 3; k++) {
             st->cb[k] = 0xFFFFFFFFu;
             st->cb[3 + k] = 0u;
@@ -163,9 +166,7 @@ __global__ void k_init_state(BuildState* st) {
         st->error = 0;
         st->depth = 1;
         st->blas_kinds = 0;
-        st->ploc_count[0] = st->ploc_count[1] = 0;
         st->merge_counter = 0;
-        st->ploc_blocks_done = 0;
         st->dop_blocks_done = 0;
         st->radius_bits = 0;
         for (int k = 0; k < 7; k++) {
@@ -219,8 +220,11 @@ __device__ bool fetch_triangle(const BlasInput& in, uint32_t i, int* geom, uint3
     return ok;
 }
 
-__global__ void k_blas_prims(const __grid_constant__ BlasInput in, float4* boxes, BuildState* st) {
+// desc / tiles: the PLOC look-back descriptors to zero (tiles <= n; 0 for other builds).
+__global__ void k_blas_prims(const __grid_constant__ BlasInput in, float4* boxes, BuildState* st,
+                             unsigned long long* desc, uint32_t tiles) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < tiles) desc[i] = 0ull;
     float cmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float bmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, bmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     if (i < in.n) {
@@ -365,8 +369,9 @@ __device__ bool fill_instance(const RtAccelerationStructureInstance& r, uint32_t
 }
 
 __global__ void k_tlas_prims(const RtAccelerationStructureInstance* inst, uint32_t n, float4* boxes,
-                             InstRecord* temp, BuildState* st) {
+                             InstRecord* temp, BuildState* st, unsigned long long* desc, uint32_t tiles) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < tiles) desc[i] = 0ull;
     float cmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float bmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, bmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     uint32_t kinds = 0;
@@ -417,44 +422,6 @@ __global__ void k_morton(const float4* boxes, uint32_t n, const BuildState* st, 
     }
     keys[i] = (expand_bits10(q[0]) << 2) | (expand_bits10(q[1]) << 1) | expand_bits10(q[2]);
     vals[i] = i;
-}
-
-// Exclusive scan of m values in place by one block of 1024 threads (all of
-// them call it); returns the total to every thread.  Values are read through
-// L2: other blocks of the same launch may have written them.
-__device__ uint32_t block_exclusive_scan(uint32_t* data, uint32_t m, uint32_t* warp_sums) {
-    const uint32_t per = (m + 1023) / 1024;
-    const uint32_t b = threadIdx.x * per, e = min(m, b + per);
-    uint32_t sum = 0;
-    for (uint32_t i = b; i < e; i++) sum += __ldcg(&data[i]);
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = sum;
-    for (int off = 1; off < 32; off <<= 1) {
-        uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-        if (lane >= (uint32_t)off) incl += o;
-    }
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = warp_sums[lane];
-        uint32_t wi = w;
-        for (int off = 1; off < 32; off <<= 1) {
-            uint32_t o = __shfl_up_sync(0xFFFFFFFFu, wi, off);
-            if (lane >= (uint32_t)off) wi += o;
-        }
-        warp_sums[lane] = wi - w;
-        if (lane == 31) warp_sums[32] = wi;
-    }
-    __syncthreads();
-    uint32_t run = warp_sums[warp] + incl - sum;
-    for (uint32_t i = b; i < e; i++) {
-        const uint32_t v = __ldcg(&data[i]);
-        data[i] = run;
-        run += v;
-    }
-    const uint32_t total = warp_sums[32];
-    __syncthreads();
-    return total;
 }
 
 struct SortTileShared {
@@ -838,7 +805,8 @@ __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const 
         else load_box_cg(iboxes, nd.x, llo, lhi);
         if (nd.y & kLeafBit) load_box_cg(sboxes, nd.y & ~kLeafBit, rlo, rhi);
         else load_box_cg(iboxes, nd.y, rlo, rhi);
-        iboxes[2 * (size_t)p] = make_float4(fminf(llo[0], rlo[0]), fminf(llo[1], rlo[1]), fminf(llo[2], rlo[2]), 0.0f);
+        iboxes[2 * (size_t)p] = make_float4(fminf(llo[0], rlo[0]), fminf(llo[1], rlo[1]), fminf(llo[2], rlo[2]),
+                                            __uint_as_float(nd.w - nd.z + 1u));  // primitives below
         iboxes[2 * (size_t)p + 1] =
             make_float4(fmaxf(lhi[0], rhi[0]), fmaxf(lhi[1], rhi[1]), fmaxf(lhi[2], rhi[2]), 0.0f);
         p = __ldcg(&iparent[p]);
@@ -854,23 +822,46 @@ __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const 
 // nearest neighbours merge into a new internal node at the lower position,
 // and the surviving clusters are compacted in order.  Internal node ids are
 // handed out from n - 2 down, so the last merge (the root) is node 0, where
-// the collapse starts.  Rounds over more than kPlocSmall clusters run as
-// grid-wide launches (their cluster count stays on the device: a round that
-// finds kPlocSmall or fewer clusters does nothing); one CTA with every
-// cluster in shared memory finishes.  If a round merges nothing (equal or NaN
-// areas), the next one merges neighbour pairs (i, i ^ 1) so the loop always
-// ends.  The host launches ploc_grid_rounds(n) grid-wide rounds: enough
-// nearest-neighbour rounds for the count to fall to kPlocSmall at the
-// measured rate (about 0.58 of the primitives survive the first round, 0.81
-// of the clusters each later one), then pair rounds, each halving the count,
-// in case it has not.
+// the collapse starts.  A cluster is two float4: (lo, binary reference) and
+// (hi, primitives below it).
+//
+// Mutual pairs alone leave 0.81 of the clusters per round, and in fans of
+// slivers (the poles of a sphere), where each cluster's nearest is the next
+// one of a chain, 0.98.  So a cluster at an odd position that has no mutual
+// neighbour also merges with its nearest neighbour j when j is at an even
+// position, has no mutual neighbour either, and its own nearest is hardly
+// nearer (kPlocNear): j takes the best of those that ask.  That leaves 0.75
+// per round (2.6M-triangle sphere: 26 rounds to 1024 clusters instead of 134)
+// at the same surface-area cost: on ten meshes and instance sets within 1 %
+// of mutual pairs only, simulated on the host; for the spheres, where the old
+// builder gave up and merged neighbour pairs, 54 instead of 61.
+//
+// Rounds over more than kPlocSmall clusters are one grid-wide launch each
+// (k_ploc_round; the cluster count stays on the device).  One CTA with every
+// cluster in shared memory finishes (k_ploc_tail).  When a round leaves more
+// than 31/32 of its clusters (many equal or NaN areas), the next one merges
+// neighbour pairs (i, i ^ 1) instead.
 constexpr int kPlocRadius = 16;
-constexpr uint32_t kPlocSmall = 4096;
-constexpr uint32_t kPlocChunk = 256;        // clusters per block of the neighbour search
-constexpr uint32_t kPlocScanBlock = 1024;   // clusters per block of the compaction scan
-constexpr uint32_t kPlocSmallThreads = 1024;
-constexpr uint32_t kPlocSmallPer = kPlocSmall / kPlocSmallThreads;
-constexpr size_t kPlocSmallSmem = (size_t)kPlocSmall * 10 * 4;  // 6 box floats, ref, neighbour, keep, size
+constexpr uint32_t kPlocSmall = 1024;  // clusters the one-CTA tail holds, one per thread
+constexpr float kPlocNear = 1.25f;
+constexpr double kPlocFirstRate = 0.62, kPlocRate = 0.765;  // survivors of the first and of later rounds, at most
+constexpr uint32_t kPlocThreads = 512;
+constexpr uint32_t kPlocTile = kPlocThreads - 6 * kPlocRadius;  // clusters a block owns per tile
+constexpr uint32_t kPlocMaxBlocks = 152 * 3;
+constexpr uint32_t kPlocParity = 1u << 31, kPlocForced = 1u << 30, kPlocCount = (1u << 28) - 1u;
+constexpr uint32_t kPlocSpinLimit = 1u << 22;
+
+struct PlocArgs {
+    const float4* boxes;     // primitive boxes in caller order
+    const uint32_t* vals;    // Morton order -> primitive
+    float4* sboxes;          // primitive boxes in Morton order (written by the first round)
+    float4* cbox[2];         // clusters, double-buffered
+    uint4* inodes;
+    float4* iboxes;
+    BuildState* st;
+    unsigned long long* desc;  // look-back descriptors: (round + 1) << 34 | state << 32 | survivors
+    uint32_t n;
+};
 
 __device__ __forceinline__ float merged_half_area(float ax, float ay, float az, float bx, float by, float bz,
                                                   float cx, float cy, float cz, float dx, float dy, float dz) {
@@ -879,400 +870,481 @@ __device__ __forceinline__ float merged_half_area(float ax, float ay, float az, 
     return ex * ey + ey * ez + ez * ex;
 }
 
-__device__ __forceinline__ uint32_t ploc_size(const uint32_t* counts, uint32_t r) {
-    return (r & kLeafBit) ? 1u : __ldcg(&counts[r]);
+// The internal node of a merge: children a and b, the merged box, the primitives below.
+__device__ __forceinline__ void ploc_write_node(const PlocArgs& a, uint32_t id, uint32_t ra, uint32_t rb, float4 lo,
+                                                float4 hi, uint32_t size) {
+    a.inodes[id] = make_uint4(ra, rb, 0u, 0u);
+    a.iboxes[2 * (size_t)id] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(size));
+    a.iboxes[2 * (size_t)id + 1] = make_float4(hi.x, hi.y, hi.z, 0.0f);
 }
 
-__global__ void k_ploc_init(const float4* sboxes, uint32_t n, uint32_t* cref, float4* cbox, BuildState* st) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) st->ploc_count[0] = n;
-    if (i >= n) return;
-    cref[i] = kLeafBit | i;
-    cbox[2 * (size_t)i] = sboxes[2 * (size_t)i];
-    cbox[2 * (size_t)i + 1] = sboxes[2 * (size_t)i + 1];
+__device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Nearest neighbour of every cluster within kPlocRadius positions (smallest
-// merged-box surface area, the lower position on ties).  The area of a pair
-// does not depend on the order of its boxes (min / max per axis), so each pair
-// is evaluated once: a block stages kPlocChunk clusters' boxes plus the halo in
-// shared memory, every position p of [c0 - R, c0 + kPlocChunk) writes the
-// areas of (p, p + o) for o = 1..R, and then each cluster scans its candidates
-// in ascending position, the pairs below it first.
-__global__ void __launch_bounds__(kPlocChunk) k_ploc_nn(const float4* cbox, uint32_t* nn, const BuildState* st,
-                                                          int round, int forced) {
-    const uint32_t count = st->ploc_count[round & 1];
-    if (count <= kPlocSmall) return;
-    constexpr int R = kPlocRadius;
-    constexpr int kSpan = (int)kPlocChunk + R;  // positions whose forward pairs a tile needs
-    __shared__ float4 slo[kPlocChunk + 2 * R], shi[kPlocChunk + 2 * R];
-    __shared__ float area[R][kSpan];            // area[o - 1][p - (c0 - R)] = area of (p, p + o)
-    for (uint32_t c0 = blockIdx.x * kPlocChunk; c0 < count; c0 += gridDim.x * kPlocChunk) {
-        const uint32_t i = c0 + threadIdx.x;
-        if (forced) {  // pair rounds: neighbours are fixed pairs
-            if (i < count) nn[i] = (i ^ 1u) < count ? (i ^ 1u) : i;
-            continue;
-        }
-        for (uint32_t t = threadIdx.x; t < kPlocChunk + 2 * R; t += blockDim.x) {
-            const int64_t g = (int64_t)c0 - R + t;
-            if (g >= 0 && g < (int64_t)count) {
-                slo[t] = __ldcg(&cbox[2 * g]);
-                shi[t] = __ldcg(&cbox[2 * g + 1]);
-            }
-        }
-        __syncthreads();
-        for (int lp = threadIdx.x; lp < kSpan; lp += blockDim.x) {
-            const int64_t gp = (int64_t)c0 - R + lp;
-            if (gp < 0 || gp >= (int64_t)count) continue;
-            const float4 a = slo[lp], b = shi[lp];
-#pragma unroll
-            for (int o = 1; o <= R; o++) {
-                const float4 c = slo[lp + o], d = shi[lp + o];
-                area[o - 1][lp] = merged_half_area(a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z, d.x, d.y, d.z);
-            }
-        }
-        __syncthreads();
-        if (i < count) {
-            const int li = (int)threadIdx.x + R;
-            uint32_t best = i;
-            float bd = INFINITY;
-            for (int o = R; o >= 1; o--) {  // candidates i - R .. i - 1
-                if ((int64_t)i - o < 0) continue;
-                const float h = area[o - 1][li - o];
-                if (h < bd) {  // ties keep the lower position
-                    bd = h;
-                    best = i - o;
+// Survivors of the tiles before `tile` in this round, by decoupled look-back:
+// the calling warp reads 32 descriptors at a time, waits until each is
+// published, and stops at the first that carries an inclusive prefix.
+// Bounded: after kPlocSpinLimit polls the build records RT_ERR_TIMEOUT.
+__device__ uint32_t ploc_look_back(const unsigned long long* desc, uint32_t round, uint32_t tile, uint32_t* error) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t sum = 0, spins = 0;
+    for (int64_t at = (int64_t)tile - 1;; at -= 32) {
+        const int64_t q = at - lane;
+        uint32_t state = 2u, value = 0u;  // before the first tile: a prefix of 0
+        if (q >= 0) {
+            for (;;) {
+                const unsigned long long v = ld_relaxed64(&desc[q]);
+                if ((uint32_t)(v >> 34) == round + 1u) {
+                    state = (uint32_t)(v >> 32) & 3u;
+                    value = (uint32_t)v;
+                    break;
                 }
-            }
-            for (int o = 1; o <= R; o++) {  // candidates i + 1 .. i + R
-                if (i + o >= count) break;
-                const float h = area[o - 1][li];
-                if (h < bd) {
-                    bd = h;
-                    best = i + o;
+                if (++spins > kPlocSpinLimit) {
+                    atomicOr(error, 1u << RT_ERR_TIMEOUT);
+                    break;  // go on with what was found
                 }
+                __nanosleep(20);
             }
-            nn[i] = best;
         }
-        __syncthreads();
+        __syncwarp();
+        const unsigned prefix = __ballot_sync(0xFFFFFFFFu, state == 2u);
+        const int stop = prefix ? __ffs(prefix) - 1 : 31;  // nearest tile with an inclusive prefix
+        sum += __reduce_add_sync(0xFFFFFFFFu, (int)lane <= stop ? value : 0u);
+        if (prefix) return sum;
     }
 }
 
-// One round's merges and the compaction offsets.  Block b takes tiles of
-// kPlocScanBlock clusters.  Cluster i merges with its nearest neighbour j
-// when j's nearest is i: the lower position keeps the new node, the higher
-// one drops out.  One scan per tile counts survivors (low 16 bits) and merges
-// (high 16 bits): the survivors' offsets go to scan and their total to blk,
-// and the tile claims its merges' node ids (counting down from n - 2) with
-// one atomic.  The block that finishes last turns the tile totals into tile
-// offsets and sets the next round's cluster count (a count of finished
-// blocks: no block waits for another).
-__global__ void __launch_bounds__(kPlocScanBlock) k_ploc_merge(
-    const uint32_t* cref, const float4* cbox, const uint32_t* nn, uint32_t* tref, float4* tbox, uint32_t* keep,
-    uint32_t* scan, uint32_t* blk, uint4* inodes, float4* iboxes, uint32_t* counts, BuildState* st, int round,
-    uint32_t n) {
-    const uint32_t count = st->ploc_count[round & 1];
-    if (count <= kPlocSmall) return;
-    __shared__ uint32_t warp_sums[33];
-    __shared__ uint32_t tile_base, last;
+// The asker that position i (even, without a mutual neighbour) takes: of the
+// odd positions within R whose nearest neighbour is i, the one with the
+// smallest area, the lower one on ties; kNone if there is none near enough.
+// x: i's place in nbr / best; the places x - R .. x + R that lie in
+// [first, last) are looked at.
+__device__ __forceinline__ uint32_t ploc_take(const uint32_t* nbr, const float* best, uint32_t i, int x, int first,
+                                              int last) {
+    const float limit = best[x] * kPlocNear;
+    float bd = INFINITY;
+    uint32_t q = kNone;
+#pragma unroll
+    for (int o = 1 - kPlocRadius; o < kPlocRadius; o += 2) {  // odd offsets, ascending
+        const int y = x + o;
+        if (y >= first && y < last && nbr[y] == i && best[y] <= limit && best[y] < bd) {
+            bd = best[y];
+            q = i + (uint32_t)o;
+        }
+    }
+    return q;
+}
+
+// One round over more than kPlocSmall clusters.  A block takes tiles in
+// ticket order.  Of its 512 threads' positions the middle 416 are its own and
+// 3 R on each side a halo: boxes for all 512, the areas of the pairs
+// (p, p + 1..R) once each (they do not depend on the order of the boxes) in
+// shared memory, the nearest neighbour (smallest area, the lower position on
+// ties) of the positions within 2 R of an own one, the askers taken by those
+// within R, then the merges of the own positions: the lower of a pair keeps
+// the new node, the higher drops out.  The tile claims its merges' node ids with one atomic
+// (counting down from n - 2) and finds its survivors' output position by
+// look-back over the earlier tiles, so one launch reads each cluster once and
+// writes each survivor once: 32 + 0.8 x 32 bytes per cluster.  (Neighbour
+// search, merge and compaction as three launches moved about 200 bytes per
+// cluster: PLOC of 10.5M triangles 3.6 ms; of 164k triangles 410 us.)  Bound:
+// shared-memory and arithmetic issue for large counts, latency for small.
+// The first round gathers the Morton-ordered primitive boxes itself.
+__global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_constant__ PlocArgs a, int round) {
+    BuildState* st = a.st;
+    const uint32_t word = st->ploc_round[round], count = word & kPlocCount;
+    if (count <= kPlocSmall) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->ploc_round[round + 1] = word;
+        return;
+    }
+    constexpr int R = kPlocRadius, T = (int)kPlocThreads;
+    const bool forced = (word & kPlocForced) != 0u;
+    const float4* cin = a.cbox[(word & kPlocParity) ? 1 : 0];
+    float4* cout = a.cbox[(word & kPlocParity) ? 0 : 1];
+    __shared__ float4 s0[T];          // lo, hi.x
+    __shared__ float2 s1[T];          // hi.y, hi.z
+    __shared__ float area[R][T - R];  // area[o - 1][t] = area of the pair (t, t + o)
+    __shared__ uint32_t nbr[T];       // nearest neighbour (position in the round)
+    __shared__ float best_area[T];    // its area
+    uint32_t* take = reinterpret_cast<uint32_t*>(&area[0][0]);  // the asker a position takes (once area is done with)
+    __shared__ uint32_t warp_sums[2 * T / 32];  // each warp's total, then the totals before it
+    __shared__ uint32_t s_tile, s_claim, s_prefix;
+    const int t = (int)threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t tiles = (count + kPlocScanBlock - 1) / kPlocScanBlock;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const uint32_t i = tile * kPlocScanBlock + threadIdx.x;
-        const bool valid = i < count;
-        uint32_t r = 0u, k = 0u, j = i;
-        bool merging = false;
+    const uint32_t tiles = (count + kPlocTile - 1u) / kPlocTile;
+    for (;;) {
+        if (t == 0) s_tile = atomicAdd(&st->ploc_ticket[round], 1u);
+        __syncthreads();
+        const uint32_t tile = s_tile;
+        if (tile >= tiles) return;
+        const int i = (int)(tile * kPlocTile) - 3 * R + t;  // this thread's position
+        const bool inside = i >= 0 && i < (int)count;
+        const bool own = inside && t >= 3 * R && t < T - 3 * R;
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-        if (valid) {
-            j = __ldcg(&nn[i]);
-            r = __ldcg(&cref[i]);
-            lo = __ldcg(&cbox[2 * (size_t)i]);
-            hi = __ldcg(&cbox[2 * (size_t)i + 1]);
-            k = 1u;
-            if (j != i && j < count && __ldcg(&nn[j]) == i) {
-                if (i < j) merging = true;
-                else k = 0u;
+        if (inside) {
+            if (round == 0) {
+                const size_t p = a.vals[i];
+                lo = a.boxes[2 * p];
+                hi = a.boxes[2 * p + 1];
+                if (own) {
+                    a.sboxes[2 * (size_t)i] = lo;
+                    a.sboxes[2 * (size_t)i + 1] = hi;
+                }
+                lo.w = __uint_as_float(kLeafBit | (uint32_t)i);
+                hi.w = __uint_as_float(1u);
+            } else {
+                lo = __ldcg(&cin[2 * (size_t)i]);
+                hi = __ldcg(&cin[2 * (size_t)i + 1]);
             }
         }
+        s0[t] = make_float4(lo.x, lo.y, lo.z, hi.x);
+        s1[t] = make_float2(hi.y, hi.z);
+        __syncthreads();
+        if (t < T - R) {
+#pragma unroll
+            for (int o = 1; o <= R; o++) {
+                const float4 c = s0[t + o];
+                const float2 d = s1[t + o];
+                const float h = merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y, c.z, c.w, d.x, d.y);
+                area[o - 1][t] = i >= 0 && i + o < (int)count ? h : INFINITY;
+            }
+        }
+        __syncthreads();
+        uint32_t near = kNone;
+        if (t >= R && t < T - R) {
+            int best = i;
+            float bd = INFINITY;
+            if (inside && forced) {
+                if ((i ^ 1) < (int)count) best = i ^ 1;
+            } else if (inside) {
+#pragma unroll
+                for (int o = R; o >= 1; o--) {  // candidates i - R .. i - 1
+                    const float h = area[o - 1][t - o];
+                    if (h < bd) {  // ties keep the lower position
+                        bd = h;
+                        best = i - o;
+                    }
+                }
+#pragma unroll
+                for (int o = 1; o <= R; o++) {  // candidates i + 1 .. i + R
+                    const float h = area[o - 1][t];
+                    if (h < bd) {
+                        bd = h;
+                        best = i + o;
+                    }
+                }
+            }
+            near = inside ? (uint32_t)best : kNone;
+            nbr[t] = near;
+            best_area[t] = bd;
+        }
+        __syncthreads();
+        bool mutual = false;
+        if (t >= 2 * R && t < T - 2 * R && inside) {
+            mutual = near != (uint32_t)i && nbr[t + ((int)near - i)] == (uint32_t)i;
+            take[t] = !mutual && !(i & 1) ? ploc_take(nbr, best_area, (uint32_t)i, t, R, T - R) : kNone;
+        }
+        __syncthreads();
+        uint32_t k = 0u;
+        bool merging = false;
+        int tj = t;
+        if (own) {
+            uint32_t j = (uint32_t)i;  // the cluster to merge with; i itself: none
+            if (mutual) j = near;
+            else if (!(i & 1)) j = take[t] != kNone ? take[t] : j;
+            else if (take[t + ((int)near - i)] == (uint32_t)i) j = near;
+            tj = t + ((int)j - i);
+            merging = (int)j > i;
+            k = (int)j < i ? 0u : 1u;
+        }
+        // one scan counts survivors (low 16 bits) and merges (high 16 bits)
         const uint32_t v = k | (merging ? 1u << 16 : 0u);
         uint32_t incl = v;
+#pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
             if (lane >= (uint32_t)off) incl += o;
         }
         if (lane == 31u) warp_sums[warp] = incl;
         __syncthreads();
+        if (warp == 1) {  // beside the look-back: both wait on L2
+            const uint32_t m = __reduce_add_sync(0xFFFFFFFFu, lane < T / 32 ? warp_sums[lane] >> 16 : 0u);
+            if (lane == 0) s_claim = m ? atomicAdd(&st->merge_counter, m) : 0u;
+        }
         if (warp == 0) {
-            const uint32_t w = warp_sums[lane];
+            const uint32_t w = lane < T / 32 ? warp_sums[lane] : 0u;
             uint32_t wi = w;
+#pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
                 const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, wi, off);
                 if (lane >= (uint32_t)off) wi += o;
             }
-            warp_sums[lane] = wi - w;
-            if (lane == 31u) {
-                blk[tile] = wi & 0xFFFFu;
-                tile_base = (wi >> 16) ? atomicAdd(&st->merge_counter, wi >> 16) : 0u;
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, wi, 31);
+            const unsigned long long tag = (unsigned long long)(round + 1) << 34;
+            if (lane == 0) st_relaxed64(&a.desc[tile], tag | (1ull << 32) | (total & 0xFFFFu));
+            if (lane < T / 32) warp_sums[T / 32 + lane] = wi - w;
+            const uint32_t before = ploc_look_back(a.desc, (uint32_t)round, tile, &st->error);
+            if (lane == 0) {
+                const uint32_t after = before + (total & 0xFFFFu);
+                st_relaxed64(&a.desc[tile], tag | (2ull << 32) | after);
+                s_prefix = before;
+                if (tile == tiles - 1u)
+                    st->ploc_round[round + 1] = (after & kPlocCount) | ((word & kPlocParity) ^ kPlocParity) |
+                                                (after > count - count / 32u ? kPlocForced : 0u);
             }
         }
         __syncthreads();
-        const uint32_t excl = warp_sums[warp] + incl - v;
-        if (merging) {
-            const uint32_t claim = tile_base + (excl >> 16);
-            if (claim + 2u > n) {  // more merges than a binary tree over n primitives has
-                atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
-            } else {
-                const uint32_t id = n - 2u - claim;
-                const uint32_t rj = __ldcg(&cref[j]);
-                const float4 lj = __ldcg(&cbox[2 * (size_t)j]), hj = __ldcg(&cbox[2 * (size_t)j + 1]);
-                lo = make_float4(fminf(lo.x, lj.x), fminf(lo.y, lj.y), fminf(lo.z, lj.z), 0.0f);
-                hi = make_float4(fmaxf(hi.x, hj.x), fmaxf(hi.y, hj.y), fmaxf(hi.z, hj.z), 0.0f);
-                inodes[id] = make_uint4(r, rj, 0u, 0u);
-                iboxes[2 * (size_t)id] = lo;
-                iboxes[2 * (size_t)id + 1] = hi;
-                counts[id] = ploc_size(counts, r) + ploc_size(counts, rj);
-                r = id;
-            }
-        }
-        if (valid) {
-            tref[i] = r;
-            tbox[2 * (size_t)i] = lo;
-            tbox[2 * (size_t)i + 1] = hi;
-            keep[i] = k;
-            scan[i] = excl & 0xFFFFu;
-        }
-        __syncthreads();
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&st->ploc_blocks_done, 1u) == gridDim.x - 1 ? 1u : 0u;
-    __syncthreads();
-    if (last) {
-        __threadfence();
-        const uint32_t total = block_exclusive_scan(blk, tiles, warp_sums);
-        if (threadIdx.x == 0) {
-            st->ploc_count[(round + 1) & 1] = total;
-            st->ploc_blocks_done = 0;
-        }
-    }
-}
-
-// Survivors to their compacted positions (tile offset + offset in the tile).
-__global__ void k_ploc_scatter(const uint32_t* tref, const float4* tbox, const uint32_t* keep, const uint32_t* scan,
-                               const uint32_t* blk, uint32_t* cref, float4* cbox, BuildState* st, int round) {
-    const uint32_t count = st->ploc_count[round & 1];
-    if (count <= kPlocSmall) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) st->ploc_count[(round + 1) & 1] = count;
-        return;
-    }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const uint32_t k = __ldcg(&keep[i]);
-        const uint32_t pos = __ldcg(&blk[i / kPlocScanBlock]) + __ldcg(&scan[i]);
         if (k) {
-            cref[pos] = __ldcg(&tref[i]);
-            cbox[2 * (size_t)pos] = __ldcg(&tbox[2 * (size_t)i]);
-            cbox[2 * (size_t)pos + 1] = __ldcg(&tbox[2 * (size_t)i + 1]);
+            const uint32_t excl = warp_sums[T / 32 + warp] + incl - v;
+            const size_t pos = s_prefix + (excl & 0xFFFFu);
+            if (merging) {
+                const uint32_t claim = s_claim + (excl >> 16);
+                if (claim + 2u > a.n) {  // more merges than a binary tree over n primitives has
+                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                } else {
+                    const uint32_t id = a.n - 2u - claim;
+                    const float4 c = s0[tj];
+                    const float2 d = s1[tj];
+                    const size_t j = (size_t)(i + (tj - t));
+                    const uint32_t rj = round == 0 ? kLeafBit | (uint32_t)j : __float_as_uint(__ldcg(&cin[2 * j]).w);
+                    const uint32_t sj = round == 0 ? 1u : __float_as_uint(__ldcg(&cin[2 * j + 1]).w);
+                    const uint32_t ri = __float_as_uint(lo.w), size = __float_as_uint(hi.w) + sj;
+                    lo = make_float4(fminf(lo.x, c.x), fminf(lo.y, c.y), fminf(lo.z, c.z), __uint_as_float(id));
+                    hi = make_float4(fmaxf(hi.x, c.w), fmaxf(hi.y, d.x), fmaxf(hi.z, d.y), __uint_as_float(size));
+                    ploc_write_node(a, id, ri, rj, lo, hi, size);
+                }
+            }
+            if (pos < count) {  // always, unless a look-back gave up
+                cout[2 * pos] = lo;
+                cout[2 * pos + 1] = hi;
+            }
         }
+        if (gridDim.x >= tiles) return;  // a block for each tile: no further one to ask for
+        __syncthreads();                 // the next tile reuses the shared arrays
     }
 }
 
-// The last rounds, in one CTA: every cluster (at most kPlocSmall) in shared
-// memory with its size; node ids are claimed from a shared counter.  With
-// few clusters, G = 2..32 threads share one cluster's neighbour search (each
-// takes every G-th offset, then a shuffle reduction keeps the smallest area,
-// the lower position on ties); otherwise thread t owns the contiguous
-// positions [t * per, t * per + per).
-__global__ void __launch_bounds__(kPlocSmallThreads) k_ploc_small(const uint32_t* cref, const float4* cbox,
-                                                                   uint4* inodes, float4* iboxes, uint32_t* counts,
-                                                                   BuildState* st, int round, uint32_t n) {
-    extern __shared__ float psm[];
-    float* lx = psm;
-    float* ly = lx + kPlocSmall;
-    float* lz = ly + kPlocSmall;
-    float* hx = lz + kPlocSmall;
-    float* hy = hx + kPlocSmall;
-    float* hz = hy + kPlocSmall;
-    uint32_t* ref = reinterpret_cast<uint32_t*>(hz + kPlocSmall);
-    uint32_t* nbr = ref + kPlocSmall;
-    uint32_t* keep = nbr + kPlocSmall;
-    uint32_t* sz = keep + kPlocSmall;
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t s_count, s_forced, s_merges, s_error;
+// The last rounds, in one CTA with every cluster (at most kPlocSmall, one
+// per thread) in shared memory; node ids follow from the round's prefix sums.
+// The areas of the pairs (i, i + 1..R) are computed once each: warp w takes
+// 32 clusters and every S-th offset, S = 1..16 the warps there are per 32
+// clusters, and the other warps only meet at the barriers.  Bound: issue of
+// one SM for the first rounds, then four barriers and the shared-memory
+// latency between them, about 1 us a round.  Meshes with fans of slivers (the
+// poles of a sphere) take many rounds: 163,840 triangles 75, 4,096 triangles
+// 40.  (With both directions evaluated by every thread of the block in each
+// round, the tail of those took 535 and 290 us.)  If the grid-wide rounds
+// left more than kPlocSmall clusters, neighbour pairs are merged in global
+// memory until that few remain.
+struct PlocTailShared {
+    float4 s0[kPlocSmall];   // lo, hi.x
+    float2 s1[kPlocSmall];   // hi.y, hi.z
+    uint2 ref[kPlocSmall];   // binary reference, primitives below
+    uint32_t nbr[kPlocSmall];
+    float best[kPlocSmall];
+    // area[o - 1][i] = area of the pair (i, i + o); then row 0 holds the asker each position takes
+    float area[kPlocRadius][kPlocSmall];
+    uint32_t warp_sums[32];
+};
+__global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant__ PlocArgs a, int round) {
+    extern __shared__ float4 ploc_smem[];
+    PlocTailShared& s = *reinterpret_cast<PlocTailShared*>(ploc_smem);
+    constexpr int R = kPlocRadius;
+    BuildState* st = a.st;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    uint32_t count = st->ploc_count[round & 1];
-    if (count > kPlocSmall || count == 0u) {
+    const uint32_t word = st->ploc_round[round];
+    uint32_t count = word & kPlocCount, merges = st->merge_counter;
+    float4* c = a.cbox[(word & kPlocParity) ? 1 : 0];
+    if (count == 0u) {
         if (tid == 0) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
         return;
     }
-    for (uint32_t t = tid; t < count; t += blockDim.x) {
-        float4 a = __ldcg(&cbox[2 * (size_t)t]), b = __ldcg(&cbox[2 * (size_t)t + 1]);
-        lx[t] = a.x; ly[t] = a.y; lz[t] = a.z;
-        hx[t] = b.x; hy[t] = b.y; hz[t] = b.z;
-        const uint32_t r = __ldcg(&cref[t]);
-        ref[t] = r;
-        sz[t] = ploc_size(counts, r);
+    while (count > kPlocSmall) {  // pair q takes positions 2q, 2q + 1 and is stored at q (behind every later read)
+        const uint32_t pairs = (count + 1u) / 2u;
+        for (uint32_t base = 0; base < pairs; base += blockDim.x) {
+            const uint32_t q = base + tid;
+            float4 lo, hi, l2, h2;
+            const bool on = q < pairs, two = on && 2u * q + 1u < count;
+            if (on) {
+                lo = __ldcg(&c[4 * (size_t)q]);
+                hi = __ldcg(&c[4 * (size_t)q + 1]);
+            }
+            if (two) {
+                l2 = __ldcg(&c[4 * (size_t)q + 2]);
+                h2 = __ldcg(&c[4 * (size_t)q + 3]);
+            }
+            __syncthreads();
+            if (two) {
+                const uint32_t claim = merges + q;
+                const uint32_t ra = __float_as_uint(lo.w), rb = __float_as_uint(l2.w);
+                const uint32_t size = __float_as_uint(hi.w) + __float_as_uint(h2.w);
+                if (claim + 2u <= a.n) {
+                    const uint32_t id = a.n - 2u - claim;
+                    lo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), __uint_as_float(id));
+                    hi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), __uint_as_float(size));
+                    ploc_write_node(a, id, ra, rb, lo, hi, size);
+                } else {
+                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                }
+            }
+            if (on) {
+                c[2 * (size_t)q] = lo;
+                c[2 * (size_t)q + 1] = hi;
+            }
+            __syncthreads();
+        }
+        merges += count / 2u;
+        count = pairs;
     }
-    if (tid == 0) {
-        s_forced = 0u;
-        s_merges = st->merge_counter;
-        s_error = 0u;
+    if (tid < count) {
+        float4 lo, hi;
+        if (round == 0) {  // no grid-wide round: gather the primitives here
+            const size_t p = a.vals[tid];
+            lo = a.boxes[2 * p];
+            hi = a.boxes[2 * p + 1];
+            a.sboxes[2 * (size_t)tid] = lo;
+            a.sboxes[2 * (size_t)tid + 1] = hi;
+            lo.w = __uint_as_float(kLeafBit | tid);
+            hi.w = __uint_as_float(1u);
+        } else {
+            lo = __ldcg(&c[2 * (size_t)tid]);
+            hi = __ldcg(&c[2 * (size_t)tid + 1]);
+        }
+        s.s0[tid] = make_float4(lo.x, lo.y, lo.z, hi.x);
+        s.s1[tid] = make_float2(hi.y, hi.z);
+        s.ref[tid] = make_uint2(__float_as_uint(lo.w), __float_as_uint(hi.w));
     }
     __syncthreads();
-    for (uint32_t guard = 0; count > 1u; guard++) {
-        if (guard > kPlocSmall) {  // every round merges at least one pair: never reached
-            if (tid == 0) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
-            return;
+    bool forced = false;
+    while (count > 1u) {  // a round after one without a merge merges pairs: it ends
+        const uint32_t blocks = (count + 31u) >> 5;  // of 32 clusters
+        if (!forced) {
+            const int lg = min(4, 31 - __clz(32u / blocks));  // log2 S
+            const uint32_t b = warp >> lg;
+            if (b < blocks) {
+                const uint32_t i = b * 32u + lane;
+                const float4 p = s.s0[i];
+                const float2 q = s.s1[i];
+                const uint32_t step = 1u << lg;
+#pragma unroll 4
+                for (uint32_t o = 1u + (warp & (step - 1u)); o <= (uint32_t)R; o += step) {
+                    const uint32_t j = (i + o) & (kPlocSmall - 1u);
+                    const float4 u = s.s0[j];
+                    const float2 v = s.s1[j];
+                    const float h = merged_half_area(p.x, p.y, p.z, p.w, q.x, q.y, u.x, u.y, u.z, u.w, v.x, v.y);
+                    s.area[o - 1u][i] = i + o < count ? h : INFINITY;
+                }
+            }
         }
-        const uint32_t per = (count + blockDim.x - 1) / blockDim.x;
-        const uint32_t b0 = min(count, tid * per), b1 = min(count, b0 + per);
-        const bool forced = s_forced != 0u;
-        uint32_t g = 1;  // threads per cluster in the neighbour search
-        while (g < 32u && count * g * 2u <= blockDim.x) g <<= 1;
-        if (g > 1u) {
-            const uint32_t i = tid / g, sub = tid % g;
-            const bool on = i < count;
-            uint32_t best = i;
+        __syncthreads();
+        const bool here = tid < count;
+        uint32_t near = tid;
+        if (here) {
             float bd = INFINITY;
-            if (on && !forced) {
-                for (uint32_t k = sub; k <= 2u * kPlocRadius; k += g) {
-                    const int64_t j = (int64_t)i - kPlocRadius + k;
-                    if (k == (uint32_t)kPlocRadius || j < 0 || j >= (int64_t)count) continue;
-                    float h = merged_half_area(lx[i], ly[i], lz[i], hx[i], hy[i], hz[i], lx[j], ly[j], lz[j], hx[j],
-                                               hy[j], hz[j]);
+            if (forced) {
+                if ((tid ^ 1u) < count) near = tid ^ 1u;
+            } else {
+#pragma unroll
+                for (int o = R; o >= 1; o--) {  // candidates i - R .. i - 1
+                    const float h = tid >= (uint32_t)o ? s.area[o - 1][tid - o] : INFINITY;
+                    if (h < bd) {  // ties keep the lower position
+                        bd = h;
+                        near = tid - o;
+                    }
+                }
+#pragma unroll
+                for (int o = 1; o <= R; o++) {  // candidates i + 1 .. i + R
+                    const float h = s.area[o - 1][tid];
                     if (h < bd) {
                         bd = h;
-                        best = (uint32_t)j;
+                        near = tid + o;
                     }
                 }
             }
-            // groups of g lanes are aligned inside the warp (g divides 32)
-            for (uint32_t off = 1; off < g; off <<= 1) {
-                const float ob = __shfl_xor_sync(0xFFFFFFFFu, bd, off);
-                const uint32_t oj = __shfl_xor_sync(0xFFFFFFFFu, best, off);
-                if (ob < bd || (ob == bd && oj < best && ob < INFINITY)) {
-                    bd = ob;
-                    best = oj;
-                }
+            s.nbr[tid] = near;
+            s.best[tid] = bd;
+        }
+        __syncthreads();
+        uint32_t* take = reinterpret_cast<uint32_t*>(&s.area[0][0]);
+        bool mutual = false;
+        if (here) {
+            mutual = near != tid && s.nbr[near] == tid;
+            take[tid] = !mutual && !(tid & 1u) ? ploc_take(s.nbr, s.best, tid, (int)tid, 0, (int)count) : kNone;
+        }
+        __syncthreads();
+        bool keep = false, merge = false;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 q = make_float2(0.f, 0.f);
+        uint2 r = make_uint2(0u, 0u);
+        uint32_t partner = 0u;
+        if (here) {
+            uint32_t j = tid;  // the cluster to merge with; tid itself: none
+            if (mutual) j = near;
+            else if (!(tid & 1u)) j = take[tid] != kNone ? take[tid] : j;
+            else if (take[near] == tid) j = near;
+            merge = j > tid;
+            keep = j >= tid;
+            p = s.s0[tid];
+            q = s.s1[tid];
+            r = s.ref[tid];
+            if (merge) {
+                const float4 u = s.s0[j];
+                const float2 v = s.s1[j];
+                const uint2 o = s.ref[j];
+                p = make_float4(fminf(p.x, u.x), fminf(p.y, u.y), fminf(p.z, u.z), fmaxf(p.w, u.w));
+                q = make_float2(fmaxf(q.x, v.x), fmaxf(q.y, v.y));
+                r.y += o.y;
+                partner = o.x;
             }
-            if (on && sub == 0u) nbr[i] = forced ? ((i ^ 1u) < count ? (i ^ 1u) : i) : best;
-        } else {
-            for (uint32_t i = b0; i < b1; i++) {
-                uint32_t best = i;
-                if (forced) {
-                    best = (i ^ 1u) < count ? (i ^ 1u) : i;
+        }
+        const unsigned kb = __ballot_sync(0xFFFFFFFFu, keep), mb = __ballot_sync(0xFFFFFFFFu, merge);
+        if (lane == 0) s.warp_sums[warp] = (uint32_t)__popc(kb) | ((uint32_t)__popc(mb) << 16);
+        __syncthreads();  // every old cluster has been read
+        const uint32_t sum = s.warp_sums[lane];
+        const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, sum);
+        if (tid < blocks * 32u) {
+            const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? sum : 0u);
+            const uint32_t lt = (1u << lane) - 1u;
+            if (merge) {
+                const uint32_t claim = merges + (before >> 16) + (uint32_t)__popc(mb & lt);
+                if (claim + 2u <= a.n) {
+                    const uint32_t id = a.n - 2u - claim;
+                    ploc_write_node(a, id, r.x, partner, make_float4(p.x, p.y, p.z, 0.f),
+                                    make_float4(p.w, q.x, q.y, 0.f), r.y);
+                    r.x = id;
                 } else {
-                    float bd = INFINITY;
-                    const uint32_t j0 = i >= (uint32_t)kPlocRadius ? i - kPlocRadius : 0u;
-                    const uint32_t j1 = min(count - 1u, i + kPlocRadius);
-                    for (uint32_t j = j0; j <= j1; j++) {
-                        if (j == i) continue;
-                        float h = merged_half_area(lx[i], ly[i], lz[i], hx[i], hy[i], hz[i], lx[j], ly[j], lz[j],
-                                                   hx[j], hy[j], hz[j]);
-                        if (h < bd) {
-                            bd = h;
-                            best = j;
-                        }
-                    }
-                }
-                nbr[i] = best;
-            }
-        }
-        __syncthreads();
-        uint32_t local = 0;
-        for (uint32_t i = b0; i < b1; i++) {
-            const uint32_t j = nbr[i];
-            uint32_t k = 1u;
-            if (j != i && nbr[j] == i) {
-                if (i < j) {
-                    const float ax = fminf(lx[i], lx[j]), ay = fminf(ly[i], ly[j]), az = fminf(lz[i], lz[j]);
-                    const float bx = fmaxf(hx[i], hx[j]), by = fmaxf(hy[i], hy[j]), bz = fmaxf(hz[i], hz[j]);
-                    const uint32_t m = atomicAdd(&s_merges, 1u);
-                    if (m + 2u <= n) {
-                        const uint32_t id = n - 2u - m;
-                        const uint32_t size = sz[i] + sz[j];
-                        inodes[id] = make_uint4(ref[i], ref[j], 0u, 0u);
-                        iboxes[2 * (size_t)id] = make_float4(ax, ay, az, 0.0f);
-                        iboxes[2 * (size_t)id + 1] = make_float4(bx, by, bz, 0.0f);
-                        counts[id] = size;
-                        ref[i] = id;
-                        sz[i] = size;
-                    } else {
-                        s_error = 1u;
-                    }
-                    lx[i] = ax; ly[i] = ay; lz[i] = az;
-                    hx[i] = bx; hy[i] = by; hz[i] = bz;
-                } else {
-                    k = 0u;
+                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
                 }
             }
-            keep[i] = k;
-            local += k;
-        }
-        // block-wide exclusive scan of the per-thread survivor counts
-        uint32_t incl = local;
-        for (int off = 1; off < 32; off <<= 1) {
-            uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-            if (lane >= (uint32_t)off) incl += o;
-        }
-        __syncthreads();  // merges done (other threads read ref / box / size of their pair above)
-        if (lane == 31u) warp_sums[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t w = warp_sums[lane], wi = w;
-            for (int off = 1; off < 32; off <<= 1) {
-                uint32_t o = __shfl_up_sync(0xFFFFFFFFu, wi, off);
-                if (lane >= (uint32_t)off) wi += o;
-            }
-            warp_sums[lane] = wi - w;
-            if (lane == 31u) s_count = wi;
-        }
-        __syncthreads();
-        // in-order compaction through registers
-        uint32_t pos = warp_sums[warp] + incl - local;
-        float v[kPlocSmallPer][6];
-        uint32_t rr[kPlocSmallPer], ss[kPlocSmallPer], kk[kPlocSmallPer];
-#pragma unroll
-        for (uint32_t q = 0; q < kPlocSmallPer; q++) {
-            const uint32_t i = b0 + q;
-            kk[q] = i < b1 ? keep[i] : 0u;
-            if (i < b1) {
-                v[q][0] = lx[i]; v[q][1] = ly[i]; v[q][2] = lz[i];
-                v[q][3] = hx[i]; v[q][4] = hy[i]; v[q][5] = hz[i];
-                rr[q] = ref[i];
-                ss[q] = sz[i];
+            if (keep) {
+                const uint32_t pos = (before & 0xFFFFu) + (uint32_t)__popc(kb & lt);
+                s.s0[pos] = p;
+                s.s1[pos] = q;
+                s.ref[pos] = r;
             }
         }
-        __syncthreads();
-#pragma unroll
-        for (uint32_t q = 0; q < kPlocSmallPer; q++) {
-            if (!kk[q]) continue;
-            lx[pos] = v[q][0]; ly[pos] = v[q][1]; lz[pos] = v[q][2];
-            hx[pos] = v[q][3]; hy[pos] = v[q][4]; hz[pos] = v[q][5];
-            ref[pos] = rr[q];
-            sz[pos] = ss[q];
-            pos++;
-        }
-        const uint32_t next = s_count;
-        __syncthreads();
-        if (tid == 0) s_forced = next == count ? 1u : 0u;
-        count = next;
+        merges += total >> 16;
+        forced = (total & 0xFFFFu) == count;
+        count = total & 0xFFFFu;
         __syncthreads();
     }
-    if (tid == 0) {
-        st->merge_counter = s_merges;
-        if (s_error) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
-    }
+    if (tid == 0) st->merge_counter = merges;
 }
 
 // ---- collapse to 8-wide -------------------------------------------------------
 struct CollapseCtx {
     const uint4* inodes;
-    const float4* iboxes;
+    const float4* iboxes;  // (lo, primitives below as bits), (hi, -) of each internal node
     const float4* sboxes;
     WideNode* nodes;
     uint32_t* parents;   // may be null
     BuildState* st;
-    const uint32_t* counts;  // primitives under each internal node (PLOC); null = the Karras ranges
     uint32_t* perm;          // final primitive order: position -> Morton-sorted position
     uint32_t leaf_max;
     uint32_t width;      // children per node: 8, or 4 (RT_BUILD_EXT_NODE_WIDTH_4)
@@ -1283,9 +1355,7 @@ struct CollapseCtx {
 // Primitives under a binary reference.
 __device__ __forceinline__ uint32_t ref_count(const CollapseCtx& c, uint32_t r) {
     if (r & kLeafBit) return 1u;
-    if (c.counts) return c.counts[r];
-    uint4 nd = c.inodes[r];
-    return nd.w - nd.z + 1u;
+    return __float_as_uint(c.iboxes[2 * (size_t)r].w);
 }
 
 // A leaf child's primitives take positions [first, first + count) of the
@@ -2087,13 +2157,22 @@ inline bool uses_ploc(uint32_t n, bool top, uint32_t build_flags) {
            n > (top ? kTlasLeafMax : kBlasLeafMax);
 }
 
-// Grid-wide PLOC rounds for n > kPlocSmall primitives: nearest-neighbour
-// rounds to reach kPlocSmall clusters at the measured survival rates with a
-// margin of 6, then pair rounds that reach it from n even if none merged.
-inline void ploc_grid_rounds(uint32_t n, int* nn_rounds, int* pair_rounds) {
-    const double x = 0.58 * (double)n / (double)kPlocSmall;
-    *nn_rounds = 1 + (x > 1.0 ? (int)std::ceil(std::log(x) / -std::log(0.81)) : 0) + 6;
-    *pair_rounds = 1 + (int)std::ceil(std::log2((double)n / (double)kPlocSmall));
+// Grid-wide PLOC rounds for n > kPlocSmall primitives: enough to reach
+// kPlocSmall clusters at the measured survival rates, and 2 more.  A round
+// that finds kPlocSmall or fewer does nothing (2.5 us); k_ploc_tail finishes
+// any count.
+inline int ploc_grid_rounds(uint32_t n) {
+    if (n <= kPlocSmall) return 0;
+    const double x = kPlocFirstRate * (double)n / (double)kPlocSmall;
+    const int rounds = 1 + (x > 1.0 ? (int)std::ceil(std::log(x) / -std::log(kPlocRate)) : 0) + 2;
+    return std::min(rounds, kPlocMaxRounds);
+}
+// Blocks of round r: the clusters it is expected to find and a third more (a
+// block takes further tiles while there are any, which costs a small round
+// half its time again).
+inline uint32_t ploc_round_blocks(uint32_t n, int r) {
+    const double c = r == 0 ? (double)n : 1.35 * kPlocFirstRate * std::pow(kPlocRate, r - 1) * (double)n;
+    return std::min<uint32_t>((uint32_t)(c / kPlocTile) + 2u, kPlocMaxBlocks);
 }
 
 }  // namespace
@@ -2157,7 +2236,7 @@ ScratchLayout ScratchLayout::make(uint32_t n, bool top, uint32_t build_flags) {
         s.ploc_nn = take(nn * 4);
         s.ploc_keep = take(nn * 4);
         s.ploc_scan = take(nn * 4);
-        s.ploc_blk = take(((nn + kPlocScanBlock - 1) / kPlocScanBlock) * 4);
+        s.ploc_blk = take(((nn + 1023) / 1024) * 4);
         s.counts = take(ni * 4);
     }
     s.refit_counters = 0;
@@ -2199,11 +2278,15 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     uint32_t* flags = reinterpret_cast<uint32_t*>(scratch + sl.flags);
     InstRecord* temp = top ? reinterpret_cast<InstRecord*>(scratch + sl.temp_inst) : nullptr;
     const uint32_t T = 256;
+    // PLOC look-back descriptors, one per tile of the first round (8 bytes per kPlocTile primitives)
+    unsigned long long* desc = sl.ploc ? reinterpret_cast<unsigned long long*>(scratch + sl.ploc_nn) : nullptr;
+    const uint32_t ploc_tiles = sl.ploc ? blocks_for(n, kPlocTile) : 0u;
 
-    note_launch(), k_init_state<<<1, 32, 0, stream>>>(st);
+    note_launch(), k_init_state<<<1, 32, 0, stream>>>(st, n);
     if (n > 0) {
-        if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st);
-        else note_launch(), k_blas_prims<<<blocks_for(n, T), T, 0, stream>>>(*blas, boxes, st);
+        if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st, desc,
+                                                                               ploc_tiles);
+        else note_launch(), k_blas_prims<<<blocks_for(n, T), T, 0, stream>>>(*blas, boxes, st, desc, ploc_tiles);
         note_launch(), k_morton<<<blocks_for(n, T), T, 0, stream>>>(boxes, n, st, keys[0], vals[0]);
         // four stable digit passes: the sorted pairs land back in keys[0] / vals[0]
         const int cur = 0;
@@ -2211,44 +2294,31 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
                                             reinterpret_cast<uint8_t*>(hist), &st->error, stream);
             e != cudaSuccess)
             return e;
-        note_launch(), k_gather_boxes<<<blocks_for(n, T), T, 0, stream>>>(boxes, vals[cur], n, sboxes);
-        uint32_t* counts = nullptr;
         if (sl.ploc) {
-            counts = reinterpret_cast<uint32_t*>(scratch + sl.counts);
-            uint32_t* cref[2] = {reinterpret_cast<uint32_t*>(scratch + sl.ploc_ref0),
-                                 reinterpret_cast<uint32_t*>(scratch + sl.ploc_ref1)};
-            float4* cbox[2] = {reinterpret_cast<float4*>(scratch + sl.ploc_box0),
-                               reinterpret_cast<float4*>(scratch + sl.ploc_box1)};
-            uint32_t* nnb = reinterpret_cast<uint32_t*>(scratch + sl.ploc_nn);
-            uint32_t* keep = reinterpret_cast<uint32_t*>(scratch + sl.ploc_keep);
-            uint32_t* scan = reinterpret_cast<uint32_t*>(scratch + sl.ploc_scan);
-            uint32_t* blk = reinterpret_cast<uint32_t*>(scratch + sl.ploc_blk);
-            note_launch(), k_ploc_init<<<blocks_for(n, T), T, 0, stream>>>(sboxes, n, cref[0], cbox[0], st);
-            int round = 0;
-            if (n > kPlocSmall) {
-                // grid-wide rounds until kPlocSmall clusters remain (later rounds
-                // do nothing); grids of at most one full SM load (152 SMs x 2048
-                // threads), grid-stride beyond
-                const uint32_t g = std::min<uint32_t>(blocks_for(n, kPlocChunk), 1216u);
-                const uint32_t gm = std::min<uint32_t>(blocks_for(n, kPlocScanBlock), 304u);
-                int nn_rounds = 0, pair_rounds = 0;
-                ploc_grid_rounds(n, &nn_rounds, &pair_rounds);
-                for (; round < nn_rounds + pair_rounds; round++) {
-                    const int forced = round >= nn_rounds;
-                    note_launch(), k_ploc_nn<<<g, kPlocChunk, 0, stream>>>(cbox[0], nnb, st, round, forced);
-                    note_launch(), k_ploc_merge<<<gm, kPlocScanBlock, 0, stream>>>(
-                        cref[0], cbox[0], nnb, cref[1], cbox[1], keep, scan, blk, inodes, iboxes, counts, st, round, n);
-                    note_launch(), k_ploc_scatter<<<g, 256, 0, stream>>>(cref[1], cbox[1], keep, scan, blk, cref[0],
-                                                                        cbox[0], st, round);
-                }
-            }
+            PlocArgs pa;
+            pa.boxes = boxes;
+            pa.vals = vals[cur];
+            pa.sboxes = sboxes;
+            pa.cbox[0] = reinterpret_cast<float4*>(scratch + sl.ploc_box0);
+            pa.cbox[1] = reinterpret_cast<float4*>(scratch + sl.ploc_box1);
+            pa.inodes = inodes;
+            pa.iboxes = iboxes;
+            pa.st = st;
+            pa.desc = desc;
+            pa.n = n;
+            const int rounds = ploc_grid_rounds(n);
+            for (int r = 0; r < rounds; r++)
+                note_launch(), k_ploc_round<<<ploc_round_blocks(n, r), kPlocThreads, 0, stream>>>(pa, r);
             // a per-device attribute: set on every build (a host-side call, no device work)
             const cudaError_t smem_ok =
-                cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlocSmallSmem);
+                cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(PlocTailShared));
             if (smem_ok != cudaSuccess) return smem_ok;
-            note_launch(), k_ploc_small<<<1, kPlocSmallThreads, kPlocSmallSmem, stream>>>(cref[0], cbox[0], inodes,
-                                                                                        iboxes, counts, st, round, n);
-        } else if (n > 1) {
+            note_launch(), k_ploc_tail<<<1, kPlocSmall, sizeof(PlocTailShared), stream>>>(pa, rounds);
+        } else {
+            note_launch(), k_gather_boxes<<<blocks_for(n, T), T, 0, stream>>>(boxes, vals[cur], n, sboxes);
+        }
+        if (!sl.ploc && n > 1) {
             note_launch(), k_karras<<<blocks_for(n - 1, T), T, 0, stream>>>(keys[cur], n, inodes, iparent, lparent);
             cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, stream);
             note_launch(), k_bottom_up<<<blocks_for(n, T), T, 0, stream>>>(inodes, lparent, iparent, sboxes, iboxes,
@@ -2259,7 +2329,6 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         cc.inodes = inodes;
         cc.iboxes = iboxes;
         cc.sboxes = sboxes;
-        cc.counts = counts;
         cc.perm = perm;
         cc.nodes = fp32_nodes;
         cc.parents = top ? reinterpret_cast<uint32_t*>(dst + al.parents) : nullptr;
