@@ -11,16 +11,13 @@
 //      boxes and subtree sizes come with each merge), or the Karras LBVH
 //      (index-augmented for ties) with bottom-up boxes from one arrival
 //      counter per internal node
-//   5. collapse to 8-wide nodes: a node takes its binary children and
-//      repeatedly opens the child of largest surface area until it has 8
-//      children or none can open; a subtree of <= leaf_max primitives is a
-//      leaf.  Each task carries the first position of its primitives in the
-//      final order; its children's primitives follow each other in slot
-//      order, and a leaf child writes its primitives' positions (perm).
-//      Levels run breadth-first, one launch each: a task is stashed in its
-//      own (not yet written) wide-node slot, and the nodes one launch
-//      allocates are the next launch's tasks.  The levels past the launched
-//      ones run as one depth-first task per thread.
+//   5. collapse to 8-wide nodes in one launch, a queue of tasks: a node takes
+//      its binary children and repeatedly opens the child of largest surface
+//      area until it has 8 children or none can open; a subtree of <=
+//      leaf_max primitives is a leaf.  Each task carries the first position
+//      of its primitives in the final order; its children's primitives
+//      follow each other in slot order, and a leaf child writes its
+//      primitives' positions (perm).
 //   6. primitive records written in that final order.
 // Everything runs on the caller's stream; no host synchronisation.
 //
@@ -42,10 +39,6 @@ namespace {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kLeafBit = 0x80000000u;
-constexpr int kMinLevels = 6;   // wide levels built breadth-first (more for large n: collapse_levels)
-constexpr int kMaxLevels = 24;
-constexpr uint32_t kCollapseBlocks = 2432;  // 152 SMs x 16 blocks of 128 threads
-constexpr int kTailStack = 192;
 constexpr int kSortThreads = 256;
 constexpr int kDopThreads = 128;
 constexpr int kDopTriples = 14 * 13 * 12 / 6;  // 364 plane triples of the 14-DOP
@@ -58,20 +51,35 @@ constexpr uint32_t kSortTile = kSortThreads * kSortItems;
 struct BuildState {
     uint32_t cb[6];   // centroid bounds, ordered-uint encoding: min xyz, max xyz
     uint32_t bb[6];   // primitive box bounds
-    uint32_t node_counter;
-    uint32_t level_lo, level_hi;  // wide-node slots holding the current collapse level's tasks
-    uint32_t level_blocks_done;   // blocks of the current collapse launch that have finished
     uint32_t error;
     uint32_t depth;
     uint32_t blas_kinds;  // TLAS: kBlasKind* bits of the BLASes its instances enter
-    uint32_t ploc_round[kPlocMaxRounds + 1];  // PLOC clusters entering each round | kPloc* bits
-    uint32_t ploc_ticket[kPlocMaxRounds];     // next tile of each round
     uint32_t merge_counter;  // PLOC merges so far (internal node ids count down from n - 2)
     uint32_t radius_bits;    // BLAS: largest vertex distance from the bounds centre (float bits, rounded up)
     uint32_t dop_hi[7], dop_lo[7];  // BLAS: largest / smallest vertex projection on each 14-DOP axis (ordered uint)
     uint32_t dop_blocks_done;       // blocks of k_dop_vertices that have finished
-    uint32_t dop_state[kDopTriples];  // 1: the triple's planes meet in a point of the 14-DOP
-    double dop_cand[kDopTriples][3];  // that point
+    union {  // the hierarchy is done when the 14-DOP is built
+        struct {
+            uint32_t ploc_round[kPlocMaxRounds + 1];  // PLOC clusters entering each round | kPloc* bits
+            uint32_t ploc_ticket[kPlocMaxRounds];     // next tile of each round
+        };
+        uint32_t dop_state[kDopTriples];  // 1: the triple's planes meet in a point of the 14-DOP
+    };
+    union {
+        // collapse: one cache line each for the two counters that every warp
+        // adds to and the flag that waiting warps read
+        struct {
+            uint32_t _line0[32];
+            unsigned long long progress;  // primitives placed in leaves << 32 | wide nodes allocated
+            uint32_t _line1[30];
+            uint32_t collapse_ticket;     // next wide-node slot to work on
+            uint32_t _line2[31];
+            uint32_t collapse_done;       // 1: every primitive has its leaf
+            uint32_t _line3[31];
+        };
+        double dop_cand[kDopTriples][3];  // that point (written when the collapse is done)
+    };
+    uint32_t node_count;  // wide nodes in use
 };
 
 // The seven 14-DOP axes (unnormalised): x, y, z and the four diagonals.
@@ -160,9 +168,10 @@ __global__ void k_init_state(BuildState* st, uint32_t n) {
             st->bb[k] = 0xFFFFFFFFu;
             st->bb[3 + k] = 0u;
         }
-        st->node_counter = 1;
-        st->level_lo = st->level_hi = 0;
-        st->level_blocks_done = 0;
+        st->progress = 1;
+        st->collapse_ticket = 0;
+        st->collapse_done = 0;
+        st->node_count = 1;
         st->error = 0;
         st->depth = 1;
         st->blas_kinds = 0;
@@ -220,11 +229,21 @@ __device__ bool fetch_triangle(const BlasInput& in, uint32_t i, int* geom, uint3
     return ok;
 }
 
-// desc / tiles: the PLOC look-back descriptors to zero (tiles <= n; 0 for other builds).
-__global__ void k_blas_prims(const __grid_constant__ BlasInput in, float4* boxes, BuildState* st,
-                             unsigned long long* desc, uint32_t tiles) {
+// What a later kernel of the build finds zeroed: the PLOC look-back
+// descriptors and the collapse's tasks.
+struct ZeroedWords {
+    unsigned long long* desc;
+    unsigned long long* tasks;
+    uint32_t descs, task_count;
+};
+__device__ __forceinline__ void zero_words(const ZeroedWords& z, uint32_t i, uint32_t stride) {
+    for (uint32_t k = i; k < z.descs; k += stride) z.desc[k] = 0ull;
+    for (uint32_t k = i; k < z.task_count; k += stride) z.tasks[k] = 0ull;
+}
+
+__global__ void k_blas_prims(const __grid_constant__ BlasInput in, float4* boxes, BuildState* st, ZeroedWords z) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < tiles) desc[i] = 0ull;
+    zero_words(z, i, gridDim.x * blockDim.x);
     float cmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float bmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, bmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     if (i < in.n) {
@@ -369,9 +388,9 @@ __device__ bool fill_instance(const RtAccelerationStructureInstance& r, uint32_t
 }
 
 __global__ void k_tlas_prims(const RtAccelerationStructureInstance* inst, uint32_t n, float4* boxes,
-                             InstRecord* temp, BuildState* st, unsigned long long* desc, uint32_t tiles) {
+                             InstRecord* temp, BuildState* st, ZeroedWords z) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < tiles) desc[i] = 0ull;
+    zero_words(z, i, gridDim.x * blockDim.x);
     float cmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float bmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, bmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     uint32_t kinds = 0;
@@ -750,9 +769,11 @@ __device__ __forceinline__ int kdelta(const uint32_t* k, int n, int i, int j) {
     return __clz(a ^ b);
 }
 
-__global__ void k_karras(const uint32_t* keys, uint32_t n_u, uint4* inodes, uint32_t* iparent, uint32_t* lparent) {
+__global__ void k_karras(const uint32_t* keys, uint32_t n_u, uint4* inodes, uint32_t* iparent, uint32_t* lparent,
+                         ZeroedWords z) {
     int n = (int)n_u;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    zero_words(z, (uint32_t)i, gridDim.x * blockDim.x);
     if (i >= n - 1) return;
     int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = kdelta(keys, n, i, i - d);
@@ -1338,6 +1359,22 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
 }
 
 // ---- collapse to 8-wide -------------------------------------------------------
+// One launch.  A task is a binary node that becomes a wide node: it takes its
+// binary children and repeatedly opens the child of largest surface area
+// until it has `width` children or none can open; a subtree of <= leaf_max
+// primitives is a leaf.  Tasks are queued by wide-node slot: eight lanes (one
+// per child) take the next slot from a ticket counter, wait until its task
+// has been written, and write the tasks of their internal children to slots
+// they claim from the node counter, so the children of a node are neighbours.
+// A task is one 64-bit word (binary node, first primitive position, depth),
+// so nothing else has to be ordered between the lanes that write and read it.
+// A slot is only ever waited for by running warps and written by the owner of
+// a lower slot, which is running too; the launch ends when every primitive is
+// in a leaf (the count travels with the node counter), and every wait is
+// bounded.  Bound: latency, about seven dependent loads per level for small
+// structures; gathers of binary nodes for large ones.  (One launch per level
+// with one thread per task: 15-40 us a level; 163,840 triangles 290 us,
+// 10,485,760 triangles 1.3 ms.)
 struct CollapseCtx {
     const uint4* inodes;
     const float4* iboxes;  // (lo, primitives below as bits), (hi, -) of each internal node
@@ -1345,258 +1382,216 @@ struct CollapseCtx {
     WideNode* nodes;
     uint32_t* parents;   // may be null
     BuildState* st;
+    unsigned long long* tasks;  // one word per wide node, zeroed
     uint32_t* perm;          // final primitive order: position -> Morton-sorted position
     uint32_t leaf_max;
     uint32_t width;      // children per node: 8, or 4 (RT_BUILD_EXT_NODE_WIDTH_4)
     uint32_t max_nodes;
     uint32_t n;          // primitives
 };
+static_assert(kBlasLeafMax <= 2 && kTlasLeafMax <= 2, "a leaf child is one primitive or a pair");
+constexpr int kCollapseThreads = 128;
+constexpr uint32_t kCollapseBlocks = 152 * 8;
+constexpr uint32_t kCollapseSpinLimit = 1u << 22;
 
-// Primitives under a binary reference.
-__device__ __forceinline__ uint32_t ref_count(const CollapseCtx& c, uint32_t r) {
-    if (r & kLeafBit) return 1u;
-    return __float_as_uint(c.iboxes[2 * (size_t)r].w);
-}
-
-// A leaf child's primitives take positions [first, first + count) of the
-// final order, left to right.  The subtree holds at most leaf_max (<= 8)
-// primitives, so the walk needs a few stack entries.
-__device__ void write_leaf_order(const CollapseCtx& c, uint32_t r, uint32_t first) {
-    uint32_t stack[8];
-    int sp = 0;
-    stack[sp++] = r;
-    uint32_t k = first;
-    while (sp > 0) {
-        const uint32_t x = stack[--sp];
-        if (x & kLeafBit) {
-            if (k < c.n) c.perm[k++] = x & ~kLeafBit;
-            continue;
-        }
-        if (x + 1u >= c.n || sp + 2 > 8) {
-            atomicOr(&c.st->error, 1u << RT_ERR_BAD_AS);
-            return;
-        }
-        const uint4 nd = c.inodes[x];
-        stack[sp++] = nd.y;
-        stack[sp++] = nd.x;
-    }
-}
-__device__ __forceinline__ void ref_box(const CollapseCtx& c, uint32_t r, float lo[3], float hi[3]) {
-    const float4* b = (r & kLeafBit) ? c.sboxes : c.iboxes;
-    size_t i = r & ~kLeafBit;
-    float4 l = b[2 * i], h = b[2 * i + 1];
-    lo[0] = l.x; lo[1] = l.y; lo[2] = l.z;
-    hi[0] = h.x; hi[1] = h.y; hi[2] = h.z;
-}
-__device__ __forceinline__ float half_area(const float lo[3], const float hi[3]) {
-    float dx = fmaxf(hi[0] - lo[0], 0.0f), dy = fmaxf(hi[1] - lo[1], 0.0f), dz = fmaxf(hi[2] - lo[2], 0.0f);
+__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
+    float dx = fmaxf(hi.x - lo.x, 0.0f), dy = fmaxf(hi.y - lo.y, 0.0f), dz = fmaxf(hi.z - lo.z, 0.0f);
     return dx * dy + dy * dz + dz * dx;
 }
-
-__device__ void write_node(WideNode* dst, const float lo[8][3], const float hi[8][3], const uint32_t ref[8],
-                           const uint32_t meta[8], int cnt) {
-    WideNode nd;
-    for (int k = 0; k < 8; k++) {
-        bool v = k < cnt && meta[k] != 0u;
-        nd.lox[k] = v ? lo[k][0] : 0.0f;
-        nd.loy[k] = v ? lo[k][1] : 0.0f;
-        nd.loz[k] = v ? lo[k][2] : 0.0f;
-        nd.hix[k] = v ? hi[k][0] : 0.0f;
-        nd.hiy[k] = v ? hi[k][1] : 0.0f;
-        nd.hiz[k] = v ? hi[k][2] : 0.0f;
-        // the traversal's stack entry: node index, or leaf | (count-1) << 28 | first
-        nd.child_ref[k] = !v ? kChildEmpty
-                             : (meta[k] == kMetaInternal ? ref[k] : (kChildLeaf | ((meta[k] - 1u) << 28) | ref[k]));
-    }
-    uint32_t m0 = 0, m1 = 0;
-    for (int k = 0; k < 4; k++) {
-        m0 |= (k < cnt ? meta[k] : 0u) << (8 * k);
-        m1 |= (k + 4 < cnt ? meta[k + 4] : 0u) << (8 * k);
-    }
-    nd.meta[0] = m0;
-    nd.meta[1] = m1;
-    for (int k = 0; k < 6; k++) nd._pad[k] = 0;
-    const uint4* s = reinterpret_cast<const uint4*>(&nd);
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    for (int k = 0; k < 16; k++) d[k] = s[k];
-}
-
 // A binary reference is in range: leaf < n, internal < n - 1.
 __device__ __forceinline__ bool ref_ok(const CollapseCtx& c, uint32_t r) {
     return (r & kLeafBit) ? ((r & ~kLeafBit) < c.n) : (r + 1u < c.n);
 }
+__device__ __forceinline__ unsigned long long collapse_task(uint32_t bref, uint32_t first, uint32_t depth) {
+    return (unsigned long long)bref | ((unsigned long long)first << 28) | ((unsigned long long)(min(depth, 254u) + 1u) << 56);
+}
 
-// One wide node from binary node bref; its primitives take positions
-// [first, first + count) of the final order.
-template <class Push>
-__device__ void collapse_task(const CollapseCtx& c, uint32_t bref, uint32_t slot, uint32_t depth, uint32_t first,
-                              Push push) {
-    // Each child's box, size and surface area are loaded once, when it joins
-    // the node: choosing the child to open reads no memory, and opening one
-    // loads only its two children (independent loads).  area < 0: the child
-    // cannot be opened (a leaf, or a subtree small enough to be one).
-    uint32_t refs[8], size[8];
-    float lo[8][3], hi[8][3], area[8];
-    int cnt = 0;
-    if (bref + 1u >= c.n || slot >= c.max_nodes) {
-        atomicOr(&c.st->error, 1u << RT_ERR_BAD_AS);
+// Child slot `k` of a wide node.  r = its traversal entry, meta = its kind.
+__device__ __forceinline__ void write_child(WideNode* nd, uint32_t k, float4 lo, float4 hi, uint32_t entry, bool used) {
+    const float z = 0.0f;
+    nd->lox[k] = used ? lo.x : z;
+    nd->hix[k] = used ? hi.x : z;
+    nd->loy[k] = used ? lo.y : z;
+    nd->hiy[k] = used ? hi.y : z;
+    nd->loz[k] = used ? lo.z : z;
+    nd->hiz[k] = used ? hi.z : z;
+    nd->child_ref[k] = used ? entry : kChildEmpty;
+}
+
+// The root of a structure of n <= leaf_max primitives (n may be 0): one leaf, or no child.
+__device__ void write_single_leaf(const CollapseCtx& c) {
+    if (c.parents) c.parents[0] = kNone;
+    const float4 lo = make_float4(o2f(c.st->bb[0]), o2f(c.st->bb[1]), o2f(c.st->bb[2]), 0.0f);
+    const float4 hi = make_float4(o2f(c.st->bb[3]), o2f(c.st->bb[4]), o2f(c.st->bb[5]), 0.0f);
+    for (uint32_t k = 0; k < 8; k++)
+        write_child(&c.nodes[0], k, lo, hi, kChildLeaf | ((c.n - 1u) << 28), k == 0 && c.n > 0);
+    c.nodes[0].meta[0] = c.n;
+    c.nodes[0].meta[1] = 0;
+    for (int k = 0; k < 6; k++) c.nodes[0]._pad[k] = 0;
+    for (uint32_t i = 0; i < c.n; i++) c.perm[i] = i;
+}
+
+__global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_constant__ CollapseCtx c) {
+    if (c.n <= c.leaf_max) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) write_single_leaf(c);
         return;
     }
-    auto load = [&](int k, uint32_t r) {
-        refs[k] = r;
-        ref_box(c, r, lo[k], hi[k]);
-        size[k] = ref_count(c, r);
-        area[k] = (!(r & kLeafBit) && size[k] > c.leaf_max) ? half_area(lo[k], hi[k]) : -1.0f;
-    };
-    const uint4 root = c.inodes[bref];
-    if (ref_ok(c, root.x) && ref_ok(c, root.y)) {
-        load(0, root.x);
-        load(1, root.y);
-        cnt = 2;
-    }
-    while (cnt >= 2 && cnt < (int)c.width) {
-        int best = -1;
-        float best_area = -1.0f;
-        for (int k = 0; k < cnt; k++) {
-            if (area[k] > best_area) {
-                best_area = area[k];
-                best = k;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, group = lane & 24u;
+    const uint32_t lt = (1u << lane) - 1u;
+    BuildState* st = c.st;
+    uint32_t slot = kNone, depth_seen = 0, spins = 0;
+    for (;;) {
+        // groups without a slot take the next ones
+        const unsigned want = __ballot_sync(0xFFFFFFFFu, slot == kNone && sub == 0u);
+        if (want) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&st->collapse_ticket, (uint32_t)__popc(want));
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            if (slot == kNone) slot = base + (uint32_t)__popc(want & ((1u << group) - 1u));
+        }
+        unsigned long long task = 0;
+        if (slot == 0u) task = collapse_task(0u, 0u, 0u);
+        else if (slot < c.max_nodes) task = ld_relaxed64(&c.tasks[slot]);
+        const bool ready = task != 0;
+        if (!__any_sync(0xFFFFFFFFu, ready)) {
+            if (ld_relaxed(&st->collapse_done)) break;
+            if (++spins > kCollapseSpinLimit) {
+                if (lane == 0) atomicOr(&st->error, 1u << RT_ERR_TIMEOUT);
+                break;
             }
-        }
-        if (best < 0) break;
-        const uint4 nd = c.inodes[refs[best]];
-        if (!ref_ok(c, nd.x) || !ref_ok(c, nd.y)) {
-            cnt = 0;
-            break;
-        }
-        load(best, nd.x);
-        load(cnt, nd.y);
-        cnt++;
-    }
-    if (cnt == 0) atomicOr(&c.st->error, 1u << RT_ERR_BAD_AS);  // malformed hierarchy: empty node
-    uint32_t ref[8], meta[8];
-    uint32_t at = first;  // the children's primitives follow each other in slot order
-    for (int k = 0; k < cnt; k++) {
-        const uint32_t r = refs[k];
-        const uint32_t sz = size[k];
-        const uint32_t f = at;
-        at += sz;
-        if (sz == 0u || at > c.n) {  // malformed hierarchy
-            atomicOr(&c.st->error, 1u << RT_ERR_BAD_AS);
-            meta[k] = 0;
-            ref[k] = 0;
+            __nanosleep(40);
             continue;
         }
-        if ((r & kLeafBit) || sz <= c.leaf_max) {
-            meta[k] = sz;
-            ref[k] = f;
-            write_leaf_order(c, r, f);
-        } else {
-            uint32_t cs = atomicAdd(&c.st->node_counter, 1u);
-            if (cs >= c.max_nodes) {
-                atomicOr(&c.st->error, 1u << RT_ERR_TOO_LARGE);
-                meta[k] = 0;
-                ref[k] = 0;
-                continue;
-            }
-            meta[k] = kMetaInternal;
-            ref[k] = cs;
-            if (c.parents) c.parents[cs] = slot;
-            push(r, cs, depth + 1, f);
+        spins = 0;
+        const uint32_t bref = (uint32_t)task & 0x0FFFFFFFu, first = (uint32_t)(task >> 28) & 0x0FFFFFFFu;
+        const uint32_t depth = (uint32_t)(task >> 56) - 1u;
+        bool bad = ready && bref + 1u >= c.n;
+        uint4 top = make_uint4(0u, 0u, 0u, 0u);
+        if (ready && !bad) {
+            top = c.inodes[bref];
+            bad = !ref_ok(c, top.x) || !ref_ok(c, top.y);
         }
-    }
-    write_node(&c.nodes[slot], lo, hi, ref, meta, cnt);
-    atomicMax(&c.st->depth, depth + 1);
-}
-
-// A collapse task waiting for its level: the binary node, the wide node's
-// depth and its first primitive position, stashed in the first 16 bytes of
-// the wide-node slot it will write (nothing else writes that slot before).
-__device__ __forceinline__ void stash_task(const CollapseCtx& c, uint32_t slot, uint32_t bref, uint32_t depth,
-                                           uint32_t first) {
-    *reinterpret_cast<uint4*>(&c.nodes[slot]) = make_uint4(bref, depth, first, 0u);
-}
-__device__ __forceinline__ uint4 stashed_task(const CollapseCtx& c, uint32_t slot) {
-    return *reinterpret_cast<const uint4*>(&c.nodes[slot]);
-}
-
-// Root wide node: a single leaf for n <= leaf_max, else the level-0 task.
-__global__ void k_collapse_root(CollapseCtx c, uint32_t n) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (c.parents) c.parents[0] = kNone;
-    if (n == 0 || n <= c.leaf_max) {
-        float lo[8][3], hi[8][3];
-        uint32_t ref[8] = {0}, meta[8] = {0};
-        int cnt = 0;
-        if (n > 0) {
-            for (int k = 0; k < 3; k++) {
-                lo[0][k] = o2f(c.st->bb[k]);
-                hi[0][k] = o2f(c.st->bb[3 + k]);
-            }
-            ref[0] = 0;
-            meta[0] = n;
-            cnt = 1;
-            for (uint32_t i = 0; i < n; i++) c.perm[i] = i;
-        }
-        write_node(&c.nodes[0], lo, hi, ref, meta, cnt);
-        return;
-    }
-    stash_task(c, 0, 0u, 0u, 0u);
-    c.st->level_lo = 0;
-    c.st->level_hi = 1;
-}
-
-// One breadth-first level: the tasks stashed in slots [level_lo, level_hi).
-// Every internal child gets the next slot from node_counter and its task is
-// stashed there, so the slots this launch allocates are the next level.  The
-// block that finishes last publishes that range (a count of finished blocks;
-// no block waits for another).
-__global__ void k_collapse_level(CollapseCtx c) {
-    const uint32_t lo = c.st->level_lo, hi = c.st->level_hi;
-    for (uint32_t t = lo + blockIdx.x * blockDim.x + threadIdx.x; t < hi; t += gridDim.x * blockDim.x) {
-        const uint4 task = stashed_task(c, t);
-        collapse_task(c, task.x, t, task.y, task.z, [&](uint32_t r, uint32_t s, uint32_t d, uint32_t f) {
-            stash_task(c, s, r, d, f);
-        });
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&c.st->level_blocks_done, 1u) == gridDim.x - 1) {
-            __threadfence();
-            const uint32_t allocated = atomicAdd(&c.st->node_counter, 0u);
-            c.st->level_lo = hi;
-            c.st->level_hi = min(allocated, c.max_nodes);
-            c.st->level_blocks_done = 0;
-        }
-    }
-}
-
-// The levels below the last breadth-first launch: each stashed task of the
-// last range is collapsed depth-first by one thread.
-__global__ void k_collapse_tail(CollapseCtx c) {
-    const uint32_t lo = c.st->level_lo, hi = c.st->level_hi;
-    for (uint32_t t = lo + blockIdx.x * blockDim.x + threadIdx.x; t < hi; t += gridDim.x * blockDim.x) {
-        uint2 stack[kTailStack];
-        uint2 dstack[kTailStack];   // depth, first primitive position
-        int sp = 0;
-        const uint4 task = stashed_task(c, t);
-        stack[sp] = make_uint2(task.x, t);
-        dstack[sp++] = make_uint2(task.y, task.z);
-        while (sp > 0) {
-            --sp;
-            uint2 e = stack[sp];
-            uint2 d = dstack[sp];
-            collapse_task(c, e.x, e.y, d.x, d.y, [&](uint32_t r, uint32_t s, uint32_t dd, uint32_t f) {
-                if (sp < kTailStack) {
-                    stack[sp] = make_uint2(r, s);
-                    dstack[sp++] = make_uint2(dd, f);
+        bool open = ready && !bad;  // the group may still open a child
+        uint32_t cnt = open ? 2u : 0u, r = sub == 0u ? top.x : top.y, size = 0, key = 0;
+        uint2 kids = make_uint2(0u, 0u);
+        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+        bool load = sub < cnt;  // the lane has a new child
+        for (uint32_t it = 2;; it++) {
+            if (load) {
+                const size_t x = r & ~kLeafBit;
+                if (r & kLeafBit) {
+                    lo = c.sboxes[2 * x];
+                    hi = c.sboxes[2 * x + 1];
+                    size = 1u;
+                    key = 0u;
                 } else {
-                    atomicOr(&c.st->error, 1u << RT_ERR_STACK_OVERFLOW);
+                    lo = c.iboxes[2 * x];
+                    hi = c.iboxes[2 * x + 1];
+                    const uint4 nd = c.inodes[x];
+                    kids = make_uint2(nd.x, nd.y);
+                    size = __float_as_uint(lo.w);
+                    const float a = half_area(lo, hi);
+                    // 0: cannot be opened (small enough for a leaf, or a NaN area)
+                    key = size > c.leaf_max && a >= 0.0f ? __float_as_uint(a) + 1u : 0u;
                 }
-            });
+            }
+            if (it >= c.width) break;
+            // open the child of largest area, the first of equals
+            uint32_t m = open ? key : 0u;
+            m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+            m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+            m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 4));
+            open = open && m != 0u;
+            const unsigned at = __ballot_sync(0xFFFFFFFFu, open && key == m);
+            if (!at) break;
+            const uint32_t best = open ? (uint32_t)__ffs((at >> group) & 0xFFu) - 1u : 0u;
+            const uint32_t kx = __shfl_sync(0xFFFFFFFFu, kids.x, (int)best, 8);
+            const uint32_t ky = __shfl_sync(0xFFFFFFFFu, kids.y, (int)best, 8);
+            load = false;
+            if (open) {
+                if (!ref_ok(c, kx) || !ref_ok(c, ky)) {
+                    bad = true;
+                    open = false;
+                } else {
+                    load = sub == best || sub == cnt;
+                    if (sub == best) r = kx;
+                    if (sub == cnt) r = ky;
+                    cnt++;
+                }
+            }
+        }
+        if (bad) {  // malformed hierarchy: an empty node, its primitives given up
+            cnt = 0;
+            if (sub == 0u) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+        }
+        // the children's primitives follow each other in slot order
+        const bool child = sub < cnt;
+        uint32_t at = child ? size : 0u;
+        for (uint32_t off = 1; off < 8; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, at, off, 8);
+            if (sub >= off) at += o;
+        }
+        at += first - (child ? size : 0u);
+        const bool leaf = child && ((r & kLeafBit) || size <= c.leaf_max), inner = child && !leaf;
+        const unsigned inners = __ballot_sync(0xFFFFFFFFu, inner);
+        uint32_t placed = leaf ? size : 0u;
+        if (bad && sub == 0u) placed = bref + 1u < c.n ? __float_as_uint(c.iboxes[2 * (size_t)bref].w) : c.n;
+        placed = __reduce_add_sync(0xFFFFFFFFu, placed);
+        unsigned long long before = 0;
+        if (lane == 0) {
+            before = atomicAdd(&st->progress, ((unsigned long long)placed << 32) | (uint32_t)__popc(inners));
+            if ((uint32_t)(before >> 32) + placed >= c.n) {  // the last primitives: no task is left
+                st->node_count = (uint32_t)before + (uint32_t)__popc(inners);
+                st_relaxed(&st->collapse_done, 1u);
+            }
+        }
+        const uint32_t cs = (uint32_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)before, 0) + (uint32_t)__popc(inners & lt);
+        bool used = child;
+        uint32_t meta = 0, entry = 0;
+        if (inner) {
+            meta = kMetaInternal;
+            entry = cs;
+            if (cs >= c.max_nodes) {  // more nodes than any hierarchy of n primitives has: give up
+                atomicOr(&st->error, 1u << RT_ERR_TOO_LARGE);
+                st_relaxed(&st->collapse_done, 1u);
+                used = false;
+            } else {
+                if (c.parents) c.parents[cs] = slot;
+                st_relaxed64(&c.tasks[cs], collapse_task(r, at, depth + 1u));
+            }
+        } else if (leaf) {
+            meta = size;
+            entry = kChildLeaf | ((size - 1u) << 28) | at;
+            if (at + size > c.n || size == 0u) {
+                atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                used = false;
+            } else if (r & kLeafBit) {
+                c.perm[at] = r & ~kLeafBit;
+            } else if ((kids.x & kids.y & kLeafBit) && size == 2u) {
+                c.perm[at] = kids.x & ~kLeafBit;
+                c.perm[at + 1u] = kids.y & ~kLeafBit;
+            } else {
+                atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                used = false;
+            }
+        }
+        // meta bytes of children 0-3 and 4-7
+        uint32_t mw = (used ? meta : 0u) << (8u * (sub & 3u));
+        mw |= __shfl_xor_sync(0xFFFFFFFFu, mw, 1);
+        mw |= __shfl_xor_sync(0xFFFFFFFFu, mw, 2);
+        const uint32_t m1 = __shfl_sync(0xFFFFFFFFu, mw, 4, 8);
+        if (ready) {
+            WideNode* nd = &c.nodes[slot];
+            write_child(nd, sub, lo, hi, entry, used);
+            // the words after child_ref: meta[0], meta[1], six of padding
+            reinterpret_cast<uint32_t*>(nd)[56 + sub] = sub == 0u ? mw : (sub == 1u ? m1 : 0u);
+            if (slot == 0u && sub == 0u && c.parents) c.parents[0] = kNone;
+            depth_seen = max(depth_seen, depth + 1u);
+            slot = kNone;
         }
     }
+    depth_seen = __reduce_max_sync(0xFFFFFFFFu, depth_seen);
+    if (lane == 0 && depth_seen > 1u) atomicMax(&st->depth, depth_seen);
 }
 
 // ---- primitive records ----------------------------------------------------------
@@ -1859,9 +1854,9 @@ __device__ uint32_t quantum_exponent(float L, float ext, uint32_t e_floor) {
     return 254u;
 }
 
-__global__ void k_quantize_nodes(const WideNode* in, const uint32_t* node_count, uint32_t max_nodes, QNode* out) {
+__global__ void k_quantize_nodes(const WideNode* in, const BuildState* st, uint32_t max_nodes, QNode* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t count = min(*node_count, max_nodes);
+    uint32_t count = min(st->node_count, max_nodes);
     if (i >= count) return;
     const WideNode& nd = in[i];
     QNode q;
@@ -1937,7 +1932,7 @@ __global__ void k_finalize(AsHeader* h, const BuildState* st, HeaderStatic hs) {
             break;
         }
     h->status = status;
-    uint32_t nc = st->node_counter;
+    uint32_t nc = st->node_count;
     if (nc > hs.max_nodes) nc = hs.max_nodes;
     h->node_count = nc;
     h->prim_count = hs.prim_count;
@@ -2140,15 +2135,6 @@ __global__ void k_as_copy(const uint8_t* src, uint8_t* dst, uint64_t dst_size, u
 }
 
 inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
-// Breadth-first collapse launches for n primitives and `width` children per
-// node: ceil(log_width n) wide levels plus three for unbalanced trees; deeper
-// subtrees finish depth-first.
-inline int collapse_levels(uint32_t n, uint32_t width) {
-    int l = 0;
-    for (uint64_t c = 1; c < n; c *= width) l++;
-    return std::min(std::max(l + 3, kMinLevels), kMaxLevels);
-}
-
 // PLOC hierarchy for builds that prefer trace speed (the reference's BLAS and
 // TLAS flags); the Karras LBVH for PREFER_FAST_BUILD or no preference, and
 // whenever one leaf holds everything.
@@ -2278,15 +2264,20 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     uint32_t* flags = reinterpret_cast<uint32_t*>(scratch + sl.flags);
     InstRecord* temp = top ? reinterpret_cast<InstRecord*>(scratch + sl.temp_inst) : nullptr;
     const uint32_t T = 256;
-    // PLOC look-back descriptors, one per tile of the first round (8 bytes per kPlocTile primitives)
-    unsigned long long* desc = sl.ploc ? reinterpret_cast<unsigned long long*>(scratch + sl.ploc_nn) : nullptr;
-    const uint32_t ploc_tiles = sl.ploc ? blocks_for(n, kPlocTile) : 0u;
+    // PLOC: one look-back descriptor per tile of the first round.  The collapse's
+    // tasks (8 bytes per possible wide node) take the Karras hierarchy's parent
+    // arrays (12 n bytes) in PLOC builds and the unsorted boxes (32 n bytes, dead
+    // once gathered) in Karras builds, so the scratch holds nothing more for them.
+    unsigned long long* tasks = reinterpret_cast<unsigned long long*>(sl.ploc ? scratch + sl.iparent : scratch + sl.boxes);
+    const uint32_t task_count = n > (top ? kTlasLeafMax : kBlasLeafMax) ? al.max_nodes : 0u;
+    const ZeroedWords zero_ploc = {reinterpret_cast<unsigned long long*>(scratch + sl.ploc_nn), tasks,
+                                   sl.ploc ? blocks_for(n, kPlocTile) : 0u, sl.ploc ? task_count : 0u};
+    const ZeroedWords zero_karras = {nullptr, tasks, 0u, task_count};
 
     note_launch(), k_init_state<<<1, 32, 0, stream>>>(st, n);
     if (n > 0) {
-        if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st, desc,
-                                                                               ploc_tiles);
-        else note_launch(), k_blas_prims<<<blocks_for(n, T), T, 0, stream>>>(*blas, boxes, st, desc, ploc_tiles);
+        if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st, zero_ploc);
+        else note_launch(), k_blas_prims<<<blocks_for(n, T), T, 0, stream>>>(*blas, boxes, st, zero_ploc);
         note_launch(), k_morton<<<blocks_for(n, T), T, 0, stream>>>(boxes, n, st, keys[0], vals[0]);
         // four stable digit passes: the sorted pairs land back in keys[0] / vals[0]
         const int cur = 0;
@@ -2304,7 +2295,7 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
             pa.inodes = inodes;
             pa.iboxes = iboxes;
             pa.st = st;
-            pa.desc = desc;
+            pa.desc = zero_ploc.desc;
             pa.n = n;
             const int rounds = ploc_grid_rounds(n);
             for (int r = 0; r < rounds; r++)
@@ -2319,7 +2310,8 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
             note_launch(), k_gather_boxes<<<blocks_for(n, T), T, 0, stream>>>(boxes, vals[cur], n, sboxes);
         }
         if (!sl.ploc && n > 1) {
-            note_launch(), k_karras<<<blocks_for(n - 1, T), T, 0, stream>>>(keys[cur], n, inodes, iparent, lparent);
+            note_launch(), k_karras<<<blocks_for(n - 1, T), T, 0, stream>>>(keys[cur], n, inodes, iparent, lparent,
+                                                                             zero_karras);
             cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, stream);
             note_launch(), k_bottom_up<<<blocks_for(n, T), T, 0, stream>>>(inodes, lparent, iparent, sboxes, iboxes,
                                                                              flags, n, &st->error);
@@ -2333,24 +2325,14 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         cc.nodes = fp32_nodes;
         cc.parents = top ? reinterpret_cast<uint32_t*>(dst + al.parents) : nullptr;
         cc.st = st;
+        cc.tasks = tasks;
         cc.leaf_max = top ? kTlasLeafMax : kBlasLeafMax;
         cc.width = node_width(build_flags);
         cc.max_nodes = al.max_nodes;
         cc.n = n;
-        note_launch(), k_collapse_root<<<1, 32, 0, stream>>>(cc, n);
-        if (n > cc.leaf_max) {
-            // level lv holds at most width^lv nodes: its grid covers 8^lv tasks
-            // (grid-stride beyond kCollapseBlocks blocks)
-            const int levels = collapse_levels(n, cc.width);
-            uint64_t cap = 1;
-            for (int lv = 0; lv < levels; lv++) {
-                const uint32_t g = blocks_for(std::min<uint64_t>(cap, (uint64_t)kCollapseBlocks * 128), 128);
-                note_launch(), k_collapse_level<<<g, 128, 0, stream>>>(cc);
-                cap = std::min<uint64_t>(cap * 8, al.max_nodes);
-            }
-            const uint32_t g = blocks_for(std::min<uint64_t>(al.max_nodes, (uint64_t)kCollapseBlocks * 128), 128);
-            note_launch(), k_collapse_tail<<<g, 128, 0, stream>>>(cc);
-        }
+        // a group of 8 lanes per possible wide node, up to a full load of the SMs
+        const uint32_t g = std::min<uint32_t>(blocks_for(al.max_nodes, kCollapseThreads / 8), kCollapseBlocks);
+        note_launch(), k_collapse<<<g, kCollapseThreads, 0, stream>>>(cc);
         if (top) {
             note_launch(), k_write_insts<<<blocks_for(n, T), T, 0, stream>>>(temp, vals[cur], perm, n,
                                                               reinterpret_cast<InstRecord*>(dst + al.prims));
@@ -2369,11 +2351,11 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         cc.width = node_width(build_flags);
         cc.max_nodes = al.max_nodes;
         cc.n = n;
-        note_launch(), k_collapse_root<<<1, 32, 0, stream>>>(cc, 0);
+        note_launch(), k_collapse<<<1, kCollapseThreads, 0, stream>>>(cc);
     }
     if (quantized) {
         uint32_t g = blocks_for(al.max_nodes, 128);
-        note_launch(), k_quantize_nodes<<<g, 128, 0, stream>>>(fp32_nodes, &st->node_counter, al.max_nodes,
+        note_launch(), k_quantize_nodes<<<g, 128, 0, stream>>>(fp32_nodes, st, al.max_nodes,
                                                                reinterpret_cast<QNode*>(dst + al.nodes));
     }
     HeaderStatic hs;
