@@ -3,9 +3,9 @@
 // Build = a binary hierarchy over Morton-ordered primitives, collapsed to
 // 8-wide nodes:
 //   1. primitive boxes (triangles, or instance world boxes) + centroid bounds
-//   2. 30-bit Morton codes of the centroids
+//   2. 30-bit Morton codes of the centroids, in the sort's first step
 //   3. stable LSD radix sort, 8-bit digits, 4 passes: one block for up to
-//      kSortTile keys, else onesweep (one upfront histogram of all digits,
+//      kSortBlockMax keys, else onesweep (one upfront histogram of all digits,
 //      then one kernel per digit with decoupled look-back across partitions)
 //   4. the binary hierarchy: PLOC clustering (RT_BUILD_PREFER_FAST_TRACE;
 //      boxes and subtree sizes come with each merge), or the Karras LBVH
@@ -39,14 +39,13 @@ namespace {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kLeafBit = 0x80000000u;
-constexpr int kSortThreads = 256;
+constexpr uint32_t kSortThreads = 1024;
+constexpr uint32_t kSortBlockMax = 8 * kSortThreads;  // keys that one block sorts
 constexpr int kDopThreads = 128;
 constexpr int kDopTriples = 14 * 13 * 12 / 6;  // 364 plane triples of the 14-DOP
 constexpr int kDopBlocks = (kDopTriples + kDopThreads - 1) / kDopThreads;
 constexpr int kDopPer = (kDopTriples + kDopThreads - 1) / kDopThreads;  // triples per thread when merging
 constexpr int kPlocMaxRounds = 64;  // grid-wide PLOC rounds (ploc_grid_rounds stays below it for 2^28 primitives)
-constexpr int kSortItems = 8;
-constexpr uint32_t kSortTile = kSortThreads * kSortItems;
 
 struct BuildState {
     uint32_t cb[6];   // centroid bounds, ordered-uint encoding: min xyz, max xyz
@@ -424,11 +423,10 @@ __device__ __forceinline__ uint32_t expand_bits10(uint32_t x) {
     return x;
 }
 
-__global__ void k_morton(const float4* boxes, uint32_t n, const BuildState* st, uint32_t* keys, uint32_t* vals) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 lo = boxes[2 * (size_t)i], hi = boxes[2 * (size_t)i + 1];
-    float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
+// 30-bit Morton code of the centroid of box i.
+__device__ __forceinline__ uint32_t morton_code(const float4* boxes, uint32_t i, const BuildState* st) {
+    const float4 lo = boxes[2 * (size_t)i], hi = boxes[2 * (size_t)i + 1];
+    const float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
     uint32_t q[3] = {0, 0, 0};
     if (finite3(c)) {
         for (int k = 0; k < 3; k++) {
@@ -439,101 +437,104 @@ __global__ void k_morton(const float4* boxes, uint32_t n, const BuildState* st, 
             q[k] = (uint32_t)s;
         }
     }
-    keys[i] = (expand_bits10(q[0]) << 2) | (expand_bits10(q[1]) << 1) | expand_bits10(q[2]);
-    vals[i] = i;
+    return (expand_bits10(q[0]) << 2) | (expand_bits10(q[1]) << 1) | expand_bits10(q[2]);
 }
 
-struct SortTileShared {
-    uint32_t digit_base[256];
-    uint32_t run[256];
-    uint32_t warp_cnt[kSortThreads / 32][256];
-};
+// Lanes of the (converged) warp whose 8-bit digit equals this lane's: one
+// ballot per bit.  (__match_any_sync takes several times as long.)
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d) {
+    uint32_t peers = 0xFFFFFFFFu;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        const uint32_t bit = (d >> b) & 1u;
+        peers &= __ballot_sync(0xFFFFFFFFu, bit) ^ (bit - 1u);
+    }
+    return peers;
+}
 
-// Stable scatter of tile `tile` (kSortTile keys) by digit (key >> shift) & 255,
-// to digit_base[d] plus the key's rank among the tile's keys of digit d.
-// Expects digit_base filled, run zeroed and a barrier before the call.
-__device__ void scatter_tile(SortTileShared& sm, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
-                             uint32_t* vout, uint32_t n, int shift, uint32_t tile);
-
-// All four passes of the radix sort in one block, for n <= kSortTile keys:
-// k0 / v0 -> k1 / v1 -> k0 / v0 ..., the result in k0 / v0.
-__global__ void __launch_bounds__(kSortThreads) k_radix_sort_small(uint32_t* k0, uint32_t* v0, uint32_t* k1,
-                                                                   uint32_t* v1, uint32_t n) {
-    __shared__ SortTileShared sm;
+// The whole sort in one block, for up to ITEMS * 1024 keys.  A pass ranks each
+// warp's keys by digit in order (so it is stable), scans the counts of all
+// (digit, warp) pairs, and moves the pairs through shared memory.  Keys past n
+// are 2^32 - 1 and come last of equals, so they stay behind the n pairs.
+// MORTON: the keys are the Morton codes of the boxes, the values their
+// indices; otherwise the pairs are in k / v.  The result goes to k / v.
+// Bound: latency and issue of one SM, 3 us and 0.9 us per item and pass (1,024
+// keys 7 us, 4,096 keys 17 us with the codes); at 16 items onesweep's five
+// launches are as fast.
+constexpr uint32_t kSortRow = kSortThreads / 32 + 1;  // counts of one digit by warp, padded against bank conflicts
+constexpr size_t sort_block_smem(int items) { return (256 * kSortRow + 2 * (size_t)items * kSortThreads) * 4; }
+template <bool MORTON, int ITEMS>
+__global__ void __launch_bounds__(kSortThreads) k_sort_block(uint32_t* k, uint32_t* v, uint32_t n, const float4* boxes,
+                                                             const BuildState* st) {
+    extern __shared__ uint32_t sort_smem[];
     __shared__ uint32_t warp_sums[kSortThreads / 32];
-    uint32_t* kin = k0;
-    uint32_t* vin = v0;
-    uint32_t* kout = k1;
-    uint32_t* vout = v1;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (int pass = 0; pass < 4; pass++) {
-        const int shift = pass * 8;
-        for (int d = threadIdx.x; d < 256; d += blockDim.x) {
-            sm.digit_base[d] = 0;
-            sm.run[d] = 0;
+    uint32_t* cnt = sort_smem;
+    uint32_t* skeys = cnt + 256 * kSortRow;
+    uint32_t* svals = skeys + ITEMS * kSortThreads;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = (1u << lane) - 1u;
+    const uint32_t first = warp * ITEMS * 32u + lane;  // item r of this thread: first + 32 r
+    uint32_t key[ITEMS], val[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++) {
+        const uint32_t i = first + 32u * r;
+        key[r] = i < n ? (MORTON ? morton_code(boxes, i, st) : k[i]) : 0xFFFFFFFFu;
+        val[r] = i < n ? (MORTON ? i : v[i]) : 0u;
+    }
+    for (int shift = 0; shift < 32; shift += 8) {
+        for (uint32_t i = tid; i < 256 * kSortRow; i += kSortThreads) cnt[i] = 0;
+        __syncthreads();
+        uint32_t rank[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            const uint32_t d = (key[r] >> shift) & 255u, peers = digit_peers(d);
+            uint32_t* c = &cnt[d * kSortRow + warp];
+            const uint32_t before = *c;
+            __syncwarp();
+            if ((peers & lt) == 0u) *c = before + (uint32_t)__popc(peers);
+            __syncwarp();
+            rank[r] = before + (uint32_t)__popc(peers & lt);
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&sm.digit_base[(kin[i] >> shift) & 255u], 1u);
-        __syncthreads();
-        // exclusive scan of the 256 digit counts (one per thread; kSortThreads == 256)
-        const uint32_t c = sm.digit_base[threadIdx.x];
-        uint32_t incl = c;
+        // exclusive scan over (digit, warp): eight counts per thread
+        uint32_t* row = &cnt[(tid >> 2) * kSortRow + (tid & 3u) * 8u];
+        uint32_t part[8], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            part[j] = sum;
+            sum += row[j];
+        }
+        uint32_t incl = sum;
+#pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
             if (lane >= (uint32_t)off) incl += o;
         }
         if (lane == 31u) warp_sums[warp] = incl;
         __syncthreads();
-        uint32_t before = 0;
-        for (uint32_t w = 0; w < warp; w++) before += warp_sums[w];
-        sm.digit_base[threadIdx.x] = before + incl - c;
+        const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? warp_sums[lane] : 0u) + incl - sum;
+#pragma unroll
+        for (int j = 0; j < 8; j++) row[j] = before + part[j];
         __syncthreads();
-        scatter_tile(sm, kin, vin, kout, vout, n, shift, 0);
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            const uint32_t pos = cnt[((key[r] >> shift) & 255u) * kSortRow + warp] + rank[r];
+            skeys[pos] = key[r];
+            svals[pos] = val[r];
+        }
         __syncthreads();
-        uint32_t* t = kin; kin = kout; kout = t;
-        t = vin; vin = vout; vout = t;
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            key[r] = skeys[first + 32u * r];
+            val[r] = svals[first + 32u * r];
+        }
     }
-}
-
-__device__ void scatter_tile(SortTileShared& sm, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
-                             uint32_t* vout, uint32_t n, int shift, uint32_t tile) {
-    uint32_t* digit_base = sm.digit_base;
-    uint32_t* run = sm.run;
-    auto& warp_cnt = sm.warp_cnt;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
-    uint32_t base = tile * kSortTile;
-    for (int j = 0; j < kSortItems; j++) {
-        for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += blockDim.x) (&warp_cnt[0][0])[i] = 0;
-        __syncthreads();
-        uint32_t idx = base + j * kSortThreads + threadIdx.x;
-        bool valid = idx < n;
-        uint32_t key = valid ? kin[idx] : 0u;
-        uint32_t val = valid ? vin[idx] : 0u;
-        uint32_t d = valid ? ((key >> shift) & 255u) : 256u;
-        uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-        uint32_t rank = __popc(peers & lanemask_lt);
-        if (valid && rank == 0) warp_cnt[warp][d] = __popc(peers);
-        __syncthreads();
-        if (threadIdx.x < 256) {
-            uint32_t dd = threadIdx.x;
-            uint32_t r = run[dd];
-            for (int w = 0; w < kSortThreads / 32; w++) {
-                uint32_t c = warp_cnt[w][dd];
-                warp_cnt[w][dd] = r;
-                r += c;
-            }
-            run[dd] = r;
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++) {
+        const uint32_t i = first + 32u * r;
+        if (i < n) {
+            k[i] = key[r];
+            v[i] = val[r];
         }
-        __syncthreads();
-        if (valid) {
-            uint32_t pos = digit_base[d] + warp_cnt[warp][d] + rank;
-            if (pos < n) {
-                kout[pos] = key;
-                vout[pos] = val;
-            }
-        }
-        __syncthreads();
     }
 }
 
@@ -554,12 +555,13 @@ constexpr int kOsThreads = 256;
 constexpr int kOsItems = 15;
 constexpr uint32_t kOsTile = kOsThreads * kOsItems;  // 3840 keys per partition
 constexpr int kOsWarps = kOsThreads / 32;
+constexpr uint32_t kOsHistBlocks = 152 * 8;  // of the histogram: a full load of the SMs
 constexpr uint32_t kOsAggregate = 1u << 30, kOsPrefix = 2u << 30, kOsValue = (1u << 30) - 1u;
 constexpr uint32_t kOsSpinLimit = 1u << 22;
+constexpr int kOsLook = 8;  // descriptors read at once in a look-back
 
-// The sort's scratch header: digit counts of the four passes (scanned in
-// place to each digit's first output position) and each pass's partition
-// counter.  The partition descriptors follow: [pass][partition][digit].
+// The sort's scratch header: digit counts of the four passes and each pass's
+// partition counter.  The partition descriptors follow: [pass][partition][digit].
 struct OnesweepState {
     uint32_t count[4][256];
     uint32_t next_partition[4];
@@ -576,12 +578,24 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__global__ void __launch_bounds__(kOsThreads) k_onesweep_hist(const uint32_t* keys, uint32_t n, OnesweepState* os) {
+// Digit counts of all four passes.  MORTON: the keys are the Morton codes of
+// the boxes, written here with their indices as values.
+template <bool MORTON>
+__global__ void __launch_bounds__(kOsThreads) k_onesweep_hist(uint32_t* keys, uint32_t* vals, uint32_t n,
+                                                              OnesweepState* os, const float4* boxes,
+                                                              const BuildState* st) {
     __shared__ uint32_t h[4][256];
     for (int i = threadIdx.x; i < 1024; i += blockDim.x) (&h[0][0])[i] = 0;
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = keys[i];
+        uint32_t k;
+        if (MORTON) {
+            k = morton_code(boxes, i, st);
+            keys[i] = k;
+            vals[i] = i;
+        } else {
+            k = keys[i];
+        }
         atomicAdd(&h[0][k & 255u], 1u);
         atomicAdd(&h[1][(k >> 8) & 255u], 1u);
         atomicAdd(&h[2][(k >> 16) & 255u], 1u);
@@ -610,13 +624,6 @@ __device__ __forceinline__ uint32_t block_scan256(uint32_t c, uint32_t* warp_sum
     return before + incl - c;
 }
 
-// Block b: the digit counts of pass b -> each digit's first output position.
-__global__ void __launch_bounds__(256) k_onesweep_scan(OnesweepState* os) {
-    __shared__ uint32_t warp_sums[8];
-    const uint32_t d = threadIdx.x;
-    os->count[blockIdx.x][d] = block_scan256(os->count[blockIdx.x][d], warp_sums);
-}
-
 struct OnesweepShared {
     uint32_t keys[kOsTile];
     uint32_t vals[kOsTile];
@@ -629,7 +636,7 @@ struct OnesweepShared {
 
 // One digit pass (bits pass*8 .. pass*8+7) over n keys: kin / vin -> kout / vout.
 // desc: this pass's descriptors, 256 per partition, zeroed.
-__global__ void __launch_bounds__(kOsThreads) k_onesweep_pass(const uint32_t* kin, const uint32_t* vin,
+__global__ void __launch_bounds__(kOsThreads, 3) k_onesweep_pass(const uint32_t* kin, const uint32_t* vin,
                                                                uint32_t* kout, uint32_t* vout, uint32_t n, int pass,
                                                                OnesweepState* os, uint32_t* desc,
                                                                uint32_t* error) {
@@ -644,14 +651,17 @@ __global__ void __launch_bounds__(kOsThreads) k_onesweep_pass(const uint32_t* ki
     const uint32_t lt = (1u << lane) - 1u;
     uint32_t key[kOsItems], val[kOsItems], rank[kOsItems];
     // warp w ranks keys base + w*32*kOsItems .. in rounds of 32, in order: stable within the tile
+    const uint32_t first = base + (uint32_t)warp * kOsItems * 32u + lane;
+#pragma unroll
+    for (int r = 0; r < kOsItems; r++) key[r] = first + r * 32u < n ? kin[first + r * 32u] : 0u;
+#pragma unroll
+    for (int r = 0; r < kOsItems; r++) val[r] = first + r * 32u < n ? vin[first + r * 32u] : 0u;
+    const uint32_t digit_total = os->count[pass][tid];
 #pragma unroll
     for (int r = 0; r < kOsItems; r++) {
-        const uint32_t idx = base + ((uint32_t)warp * kOsItems + r) * 32u + lane;
-        const bool valid = idx < n;
-        key[r] = valid ? kin[idx] : 0u;
-        val[r] = valid ? vin[idx] : 0u;
-        const uint32_t d = valid ? ((key[r] >> shift) & 255u) : 256u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+        const bool valid = first + r * 32u < n;
+        const uint32_t d = (key[r] >> shift) & 255u;
+        const uint32_t peers = digit_peers(d) & __ballot_sync(0xFFFFFFFFu, valid);
         const uint32_t before = valid ? sm.warp_cnt[warp][d] : 0u;
         __syncwarp();
         if (valid && (peers & lt) == 0u) sm.warp_cnt[warp][d] = before + (uint32_t)__popc(peers);
@@ -674,26 +684,37 @@ __global__ void __launch_bounds__(kOsThreads) k_onesweep_pass(const uint32_t* ki
         st_relaxed(mine, kOsPrefix | total);
     } else {
         st_relaxed(mine, kOsAggregate | total);
-        uint32_t q = p - 1, spins = 0;
-        for (;;) {
-            const uint32_t v = ld_relaxed(desc + (size_t)q * 256u + d);
-            const uint32_t flag = v & ~kOsValue;
-            if (flag == 0u) {
+        // kOsLook descriptors at a time: when all partitions run at once, none
+        // has a prefix yet and one read per step would take p round trips to L2
+        uint32_t q = p, spins = 0;  // the partitions before q are still to be added
+        for (bool more = true; more;) {
+            uint32_t v[kOsLook];
+#pragma unroll
+            for (int j = 0; j < kOsLook; j++)
+                v[j] = q > (uint32_t)j ? ld_relaxed(desc + (size_t)(q - 1u - j) * 256u + d) : kOsPrefix;
+            uint32_t taken = 0;
+#pragma unroll
+            for (int j = 0; j < kOsLook; j++) {
+                const uint32_t flag = v[j] & ~kOsValue;
+                if (!more || taken != (uint32_t)j || flag == 0u) continue;
+                excl += v[j] & kOsValue;
+                taken++;
+                if (flag == kOsPrefix) more = false;
+            }
+            q -= min(taken, q);
+            if (more && taken < (uint32_t)kOsLook) {  // the next one is not published yet
                 if (++spins > kOsSpinLimit) {  // bounded: report and go on with what was found
                     atomicOr(error, 1u << RT_ERR_TIMEOUT);
                     break;
                 }
                 __nanosleep(32);
-                continue;
             }
-            excl += v & kOsValue;
-            if (flag == kOsPrefix || q == 0u) break;
-            q--;
         }
         st_relaxed(mine, kOsPrefix | (excl + total));
     }
     sm.tile_start[d] = block_scan256(total, sm.warp_sums);
-    sm.out_start[d] = os->count[pass][d] + excl;
+    __syncthreads();  // warp_sums is used again
+    sm.out_start[d] = block_scan256(digit_total, sm.warp_sums) + excl;  // every key of a smaller digit comes before
     __syncthreads();
     // stage the tile in digit order, then write it out in that order
 #pragma unroll
@@ -723,21 +744,34 @@ uint64_t key_sort_state_bytes(uint32_t n) {
     return sizeof(OnesweepState) + (uint64_t)4 * onesweep_partitions(n ? n : 1) * 256u * 4u;
 }
 
-cudaError_t launch_key_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t n, uint8_t* state,
-                            uint32_t* error, cudaStream_t stream) {
-    if (n <= 1) return cudaSuccess;
-    if (n <= kSortTile) {
-        // one block sorts all four digits
-        note_launch(), k_radix_sort_small<<<1, kSortThreads, 0, stream>>>(k0, v0, k1, v1, n);
-        return cudaGetLastError();
-    }
+namespace {
+template <bool MORTON, int ITEMS>
+cudaError_t launch_sort_block(uint32_t* k, uint32_t* v, uint32_t n, const float4* boxes, const BuildState* st,
+                              cudaStream_t stream) {
+    const size_t smem = sort_block_smem(ITEMS);
+    // a per-device attribute: set on every sort (a host-side call, no device work)
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_sort_block<MORTON, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    note_launch(), k_sort_block<MORTON, ITEMS><<<1, kSortThreads, smem, stream>>>(k, v, n, boxes, st);
+    return cudaGetLastError();
+}
+
+// Sorts n pairs (MORTON: the boxes' Morton codes and indices) into k0 / v0.
+template <bool MORTON>
+cudaError_t launch_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t n, uint8_t* state,
+                        uint32_t* error, const float4* boxes, const BuildState* st, cudaStream_t stream) {
+    if (n <= kSortThreads) return launch_sort_block<MORTON, 1>(k0, v0, n, boxes, st, stream);
+    if (n <= 2 * kSortThreads) return launch_sort_block<MORTON, 2>(k0, v0, n, boxes, st, stream);
+    if (n <= 4 * kSortThreads) return launch_sort_block<MORTON, 4>(k0, v0, n, boxes, st, stream);
+    if (n <= kSortBlockMax) return launch_sort_block<MORTON, 8>(k0, v0, n, boxes, st, stream);
     OnesweepState* os = reinterpret_cast<OnesweepState*>(state);
     uint32_t* desc = reinterpret_cast<uint32_t*>(state + sizeof(OnesweepState));
     const uint32_t parts = onesweep_partitions(n);
     cudaError_t e = cudaMemsetAsync(state, 0, key_sort_state_bytes(n), stream);
     if (e != cudaSuccess) return e;
-    note_launch(), k_onesweep_hist<<<std::min<uint32_t>(parts, 1024u), kOsThreads, 0, stream>>>(k0, n, os);
-    note_launch(), k_onesweep_scan<<<4, 256, 0, stream>>>(os);
+    note_launch(), k_onesweep_hist<MORTON><<<std::min<uint32_t>((n + kOsThreads - 1) / kOsThreads, kOsHistBlocks),
+                                             kOsThreads, 0, stream>>>(k0, v0, n, os, boxes, st);
     uint32_t* kin = k0;
     uint32_t* vin = v0;
     uint32_t* kout = k1;
@@ -749,6 +783,13 @@ cudaError_t launch_key_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* 
         std::swap(vin, vout);
     }
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_key_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t n, uint8_t* state,
+                            uint32_t* error, cudaStream_t stream) {
+    if (n <= 1) return cudaSuccess;
+    return launch_sort<false>(k0, v0, k1, v1, n, state, error, nullptr, nullptr, stream);
 }
 
 namespace {
@@ -2278,11 +2319,10 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     if (n > 0) {
         if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st, zero_ploc);
         else note_launch(), k_blas_prims<<<blocks_for(n, T), T, 0, stream>>>(*blas, boxes, st, zero_ploc);
-        note_launch(), k_morton<<<blocks_for(n, T), T, 0, stream>>>(boxes, n, st, keys[0], vals[0]);
-        // four stable digit passes: the sorted pairs land back in keys[0] / vals[0]
+        // Morton codes and their stable order: the sorted pairs land in keys[0] / vals[0]
         const int cur = 0;
-        if (cudaError_t e = launch_key_sort(keys[0], vals[0], keys[1], vals[1], n,
-                                            reinterpret_cast<uint8_t*>(hist), &st->error, stream);
+        if (cudaError_t e = launch_sort<true>(keys[0], vals[0], keys[1], vals[1], n, reinterpret_cast<uint8_t*>(hist),
+                                              &st->error, boxes, st, stream);
             e != cudaSuccess)
             return e;
         if (sl.ploc) {
