@@ -41,10 +41,7 @@ constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kSortThreads = 1024;
 constexpr uint32_t kSortBlockMax = 8 * kSortThreads;  // keys that one block sorts
-constexpr int kDopThreads = 128;
 constexpr int kDopTriples = 14 * 13 * 12 / 6;  // 364 plane triples of the 14-DOP
-constexpr int kDopBlocks = (kDopTriples + kDopThreads - 1) / kDopThreads;
-constexpr int kDopPer = (kDopTriples + kDopThreads - 1) / kDopThreads;  // triples per thread when merging
 constexpr int kPlocMaxRounds = 64;  // grid-wide PLOC rounds (ploc_grid_rounds stays below it for 2^28 primitives)
 
 struct BuildState {
@@ -56,30 +53,24 @@ struct BuildState {
     uint32_t merge_counter;  // PLOC merges so far (internal node ids count down from n - 2)
     uint32_t radius_bits;    // BLAS: largest vertex distance from the bounds centre (float bits, rounded up)
     uint32_t dop_hi[7], dop_lo[7];  // BLAS: largest / smallest vertex projection on each 14-DOP axis (ordered uint)
-    uint32_t dop_blocks_done;       // blocks of k_dop_vertices that have finished
-    union {  // the hierarchy is done when the 14-DOP is built
-        struct {
-            uint32_t ploc_round[kPlocMaxRounds + 1];  // PLOC clusters entering each round | kPloc* bits
-            uint32_t ploc_ticket[kPlocMaxRounds];     // next tile of each round
-        };
-        uint32_t dop_state[kDopTriples];  // 1: the triple's planes meet in a point of the 14-DOP
-    };
-    union {
-        // collapse: one cache line each for the two counters that every warp
-        // adds to and the flag that waiting warps read
-        struct {
-            uint32_t _line0[32];
-            unsigned long long progress;  // primitives placed in leaves << 32 | wide nodes allocated
-            uint32_t _line1[30];
-            uint32_t collapse_ticket;     // next wide-node slot to work on
-            uint32_t _line2[31];
-            uint32_t collapse_done;       // 1: every primitive has its leaf
-            uint32_t _line3[31];
-        };
-        double dop_cand[kDopTriples][3];  // that point (written when the collapse is done)
-    };
+    uint32_t ploc_round[kPlocMaxRounds + 1];  // PLOC clusters entering each round | kPloc* bits
+    uint32_t ploc_ticket[kPlocMaxRounds];     // next tile of each round
+    // collapse: one cache line each for the two counters that every warp adds
+    // to and the flag that waiting warps read
+    uint32_t _line0[32];
+    unsigned long long progress;  // primitives placed in leaves << 32 | wide nodes allocated
+    uint32_t _line1[30];
+    uint32_t collapse_ticket;     // next wide-node slot to work on
+    uint32_t _line2[31];
+    uint32_t collapse_done;       // 1: every primitive has its leaf
+    uint32_t _line3[31];
     uint32_t node_count;  // wide nodes in use
 };
+// The state's share of the build scratch.  It is more than the state needs:
+// the scratch sizes that callers query, and the limit of the static-scratch
+// build that follows from them, stay as they are.
+constexpr uint64_t kBuildStateBytes = 10496;
+static_assert(sizeof(BuildState) <= kBuildStateBytes, "build state size");
 
 // The seven 14-DOP axes (unnormalised): x, y, z and the four diagonals.
 __device__ __constant__ const int8_t kDopAxis[7][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 1, 1},
@@ -175,7 +166,6 @@ __global__ void k_init_state(BuildState* st, uint32_t n) {
         st->depth = 1;
         st->blas_kinds = 0;
         st->merge_counter = 0;
-        st->dop_blocks_done = 0;
         st->radius_bits = 0;
         for (int k = 0; k < 7; k++) {
             st->dop_hi[k] = 0u;
@@ -1713,156 +1703,6 @@ __global__ void k_write_tris(const __grid_constant__ BlasInput in, const uint32_
     tris[i] = r;
 }
 
-// The 14-DOP's vertices: every triple of its 14 planes solved in double, one
-// thread per triple over kDopBlocks blocks, kept when the point satisfies all
-// 14 planes (with a relative tolerance).  The block that finishes last (a
-// count of finished blocks: no block waits) gathers the points in triple
-// order and merges duplicates: a point within the tolerance of an earlier one
-// is dropped, one thread per point (a serial pass over all pairs in double
-// took hundreds of microseconds at this part's FP64 rate).  More than
-// kDopMaxVertices distinct points (only through rounding) or a non-finite
-// projection leave the header's dop_count at 0.  The vertices' float rounding
-// (a few 1e-8 relative) is covered by the instance box padding (1e-5
-// relative).
-__global__ void __launch_bounds__(kDopThreads) k_dop_vertices(AsHeader* h, BuildState* st) {
-    __shared__ double pn[14][3], ph[14];
-    __shared__ double cand[kDopTriples][3];  // the points found, in triple order (last block)
-    __shared__ float candf[kDopTriples][3];
-    __shared__ uint8_t dup[kDopTriples];      // 1: within the tolerance of an earlier point
-    __shared__ uint32_t warp_sums[kDopThreads / 32];
-    __shared__ uint32_t npts;
-    __shared__ bool ok;
-    __shared__ uint32_t last;
-    const int t = blockIdx.x * kDopThreads + threadIdx.x;
-    if (threadIdx.x == 0) {
-        ok = true;
-        for (int k = 0; k < 7; k++) {
-            const float hi = o2f(st->dop_hi[k]), lo = o2f(st->dop_lo[k]);
-            if (!(lo <= hi) || !(fabsf(hi) <= FLT_MAX) || !(fabsf(lo) <= FLT_MAX)) ok = false;
-            for (int a = 0; a < 3; a++) {
-                pn[2 * k][a] = (double)kDopAxis[k][a];
-                pn[2 * k + 1][a] = -(double)kDopAxis[k][a];
-            }
-            ph[2 * k] = (double)hi;
-            ph[2 * k + 1] = -(double)lo;
-        }
-        if (blockIdx.x == 0) h->dop_count = 0;
-    }
-    __syncthreads();
-    if (!ok) return;  // the same in every block
-    double scale = 1e-30;
-    for (int j = 0; j < 14; j++) scale = fmax(scale, fabs(ph[j]));
-    if (t < kDopTriples) {
-        int a = 0, b = 1, c = 2;
-        for (int idx = 0; idx < t; idx++) {  // the t-th triple a < b < c in lexicographic order
-            if (++c == 14) {
-                if (++b == 13) {
-                    ++a;
-                    b = a + 1;
-                }
-                c = b + 1;
-            }
-        }
-        uint32_t found = 0;
-        // Cramer's rule on the rows pn[a], pn[b], pn[c]
-        const double* A = pn[a];
-        const double* B = pn[b];
-        const double* C = pn[c];
-        const double det = A[0] * (B[1] * C[2] - B[2] * C[1]) - A[1] * (B[0] * C[2] - B[2] * C[0]) +
-                           A[2] * (B[0] * C[1] - B[1] * C[0]);
-        if (fabs(det) >= 1e-9) {
-            const double x = (ph[a] * (B[1] * C[2] - B[2] * C[1]) - A[1] * (ph[b] * C[2] - B[2] * ph[c]) +
-                              A[2] * (ph[b] * C[1] - B[1] * ph[c])) / det;
-            const double y = (A[0] * (ph[b] * C[2] - B[2] * ph[c]) - ph[a] * (B[0] * C[2] - B[2] * C[0]) +
-                              A[2] * (B[0] * ph[c] - ph[b] * C[0])) / det;
-            const double z = (A[0] * (B[1] * ph[c] - ph[b] * C[1]) - A[1] * (B[0] * ph[c] - ph[b] * C[0]) +
-                              ph[a] * (B[0] * C[1] - B[1] * C[0])) / det;
-            bool inside = true;
-            for (int j = 0; j < 14 && inside; j++)
-                inside = pn[j][0] * x + pn[j][1] * y + pn[j][2] * z <= ph[j] + 1e-9 * scale;
-            if (inside) {
-                st->dop_cand[t][0] = x;
-                st->dop_cand[t][1] = y;
-                st->dop_cand[t][2] = z;
-                found = 1;
-            }
-        }
-        st->dop_state[t] = found;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&st->dop_blocks_done, 1u) == gridDim.x - 1 ? 1u : 0u;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // the points, in triple order (each thread takes kDopPer consecutive triples)
-    const int t0 = threadIdx.x * kDopPer;
-    uint32_t mine = 0;
-    for (int k = 0; k < kDopPer; k++)
-        if (t0 + k < kDopTriples && __ldcg(&st->dop_state[t0 + k])) mine++;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = mine;
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-        if (lane >= (uint32_t)off) incl += o;
-    }
-    if (lane == 31u) warp_sums[warp] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t w = 0; w < kDopThreads / 32; w++) {
-            const uint32_t v = warp_sums[w];
-            warp_sums[w] = run;
-            run += v;
-        }
-        npts = run;
-    }
-    __syncthreads();
-    uint32_t at = warp_sums[warp] + incl - mine;
-    for (int k = 0; k < kDopPer; k++) {
-        const int i = t0 + k;
-        if (i < kDopTriples && __ldcg(&st->dop_state[i])) {
-            for (int a = 0; a < 3; a++) {
-                cand[at][a] = __ldcg(&st->dop_cand[i][a]);
-                candf[at][a] = (float)cand[at][a];
-            }
-            dup[at] = 0;
-            at++;
-        }
-    }
-    __syncthreads();
-    // A pair is a duplicate when every coordinate differs by at most 1e-7
-    // scale (in double).  The float copies screen the pairs first: every
-    // coordinate is within scale (1 + 1e-9) (the axis planes bound it), so
-    // rounding to float moves a difference by at most 2^-23 scale, and a
-    // pair whose float difference exceeds 4e-7 scale cannot pass the double
-    // test.  Only the few pairs that pass the screen use the slow FP64 pipe.
-    const double tol = 1e-7 * scale;
-    const float tolf = 4e-7f * (float)scale;
-    for (uint32_t i = threadIdx.x; i < npts; i += kDopThreads) {
-        bool d = false;
-        for (uint32_t j = 0; j < i && !d; j++) {
-            if (fabsf(candf[i][0] - candf[j][0]) > tolf || fabsf(candf[i][1] - candf[j][1]) > tolf ||
-                fabsf(candf[i][2] - candf[j][2]) > tolf)
-                continue;
-            d = fabs(cand[i][0] - cand[j][0]) <= tol && fabs(cand[i][1] - cand[j][1]) <= tol &&
-                fabs(cand[i][2] - cand[j][2]) <= tol;
-        }
-        dup[i] = d ? 1 : 0;
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    st->dop_blocks_done = 0;
-    uint32_t nv = 0;
-    for (uint32_t i = 0; i < npts; i++) {
-        if (dup[i]) continue;
-        if (nv == kDopMaxVertices) return;  // more points than a 14-DOP has: leave it off
-        for (int a = 0; a < 3; a++) h->dop_vertex[nv][a] = (float)cand[i][a];
-        nv++;
-    }
-    if (nv >= 4u) h->dop_count = nv;
-}
-
 __global__ void k_write_insts(const InstRecord* temp, const uint32_t* vals, const uint32_t* perm, uint32_t n,
                               InstRecord* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1954,25 +1794,20 @@ __global__ void k_quantize_nodes(const WideNode* in, const BuildState* st, uint3
     for (int w = 0; w < 6; w++) dst[w] = src[w];
 }
 
+// ---- header ---------------------------------------------------------------------
 struct HeaderStatic {
     uint32_t type, build_flags, prim_count, max_nodes, geometry_count, leaf_max, node_bytes;
     uint64_t total_size, nodes_offset, prims_offset, parents_offset;
     uint64_t prim_bytes;
 };
 
-__global__ void k_finalize(AsHeader* h, const BuildState* st, HeaderStatic hs) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// The header of a finished build but for the 14-DOP (one thread).
+__device__ void write_header(AsHeader* h, const BuildState* st, const HeaderStatic& hs) {
     h->magic = kAsMagic;
     h->type = hs.type;
     h->build_flags = hs.build_flags;
     uint32_t err = st->error;
-    uint32_t status = RT_OK;
-    for (uint32_t e = 1; e < 32; e++)
-        if (err & (1u << e)) {
-            status = e;
-            break;
-        }
-    h->status = status;
+    h->status = err >> 1 ? (uint32_t)__ffs(err >> 1) : (uint32_t)RT_OK;  // the lowest RT_ERR_* bit
     uint32_t nc = st->node_count;
     if (nc > hs.max_nodes) nc = hs.max_nodes;
     h->node_count = nc;
@@ -2005,6 +1840,180 @@ __global__ void k_finalize(AsHeader* h, const BuildState* st, HeaderStatic hs) {
     uint64_t par = hs.parents_offset ? align_up(nodes_end, 256) : 0;
     uint64_t par_end = par ? par + (uint64_t)nc * 4 : nodes_end;
     h->compacted_size = align_up(align_up(par_end, 256) + hs.prim_count * hs.prim_bytes, 256);
+}
+
+// The plane triples a < b < c of the 14-DOP in lexicographic order.
+struct DopTriples {
+    uint8_t t[kDopTriples][4];
+};
+constexpr DopTriples make_dop_triples() {
+    DopTriples d{};
+    int n = 0;
+    for (int a = 0; a < 14; a++)
+        for (int b = a + 1; b < 14; b++)
+            for (int c = b + 1; c < 14; c++, n++) {
+                d.t[n][0] = (uint8_t)a;
+                d.t[n][1] = (uint8_t)b;
+                d.t[n][2] = (uint8_t)c;
+            }
+    return d;
+}
+__device__ const DopTriples kDopTriple = make_dop_triples();
+
+// Plane j of the 14-DOP: +axis (even) or -axis (odd), and n . p <= its height.
+__device__ __forceinline__ float dop_dot(int j, float x, float y, float z) {
+    const int8_t* a = kDopAxis[j >> 1];
+    const float d = (float)a[0] * x + (float)a[1] * y + (float)a[2] * z;
+    return (j & 1) ? -d : d;
+}
+
+// The header, and for a BLAS its 14-DOP's vertices (0: none), in one block.
+// Every triple of the 14 planes is solved: first in float with a tolerance of
+// 1e-5 of the scale (float rounding moves the point and its projections by a
+// few 1e-6 of it), which leaves the vertices and few others; those are solved
+// in double and kept when the point satisfies all 14 planes (1e-9 relative).
+// Points within 1e-7 of an earlier one (in triple order) are dropped, again
+// screened in float.  This part's double precision runs at two operations per
+// clock and SM: with all 364 triples in double over three blocks the vertices
+// took 28 us and the header another launch of 4 us; together 11.5 us now.  More than kDopMaxVertices
+// distinct points (only through rounding) or a non-finite projection leave
+// the header's dop_count at 0.  The vertices' float rounding (a few 1e-8
+// relative) is covered by the instance box padding (1e-5 relative).
+constexpr int kFinishThreads = 384;
+static_assert(kFinishThreads >= kDopTriples, "one thread per triple");
+__global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const BuildState* st,
+                                                           const __grid_constant__ HeaderStatic hs) {
+    __shared__ float phf[14];
+    __shared__ uint16_t list[kDopTriples];   // triples that pass the float screen, in order
+    __shared__ double cand[kDopTriples][3];  // the points found, by place in the list
+    __shared__ float candf[kDopTriples][3];
+    __shared__ uint8_t found[kDopTriples];   // 1: a point of the 14-DOP; 2: and no earlier one is within the tolerance
+    __shared__ uint32_t warp_sums[kFinishThreads / 32];
+    __shared__ bool ok;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    if (t == kFinishThreads - 1) write_header(h, st, hs);
+    if (hs.type != kAsTypeBottom || hs.prim_count == 0u) {
+        if (t == 0) h->dop_count = 0;
+        return;
+    }
+    if (t == 0) {
+        bool good = true;
+        for (int k = 0; k < 7; k++) {
+            const float hi = o2f(st->dop_hi[k]), lo = o2f(st->dop_lo[k]);
+            if (!(lo <= hi) || !(fabsf(hi) <= FLT_MAX) || !(fabsf(lo) <= FLT_MAX)) good = false;
+            phf[2 * k] = hi;
+            phf[2 * k + 1] = -lo;
+        }
+        ok = good;
+        h->dop_count = 0;
+    }
+    __syncthreads();
+    if (!ok) return;
+    float scale_f = 0.0f;
+    for (int j = 0; j < 14; j++) scale_f = fmaxf(scale_f, fabsf(phf[j]));
+    const double scale = fmax(1e-30, (double)scale_f);
+    bool pass = false;
+    if (t < (uint32_t)kDopTriples) {
+        const int a = kDopTriple.t[t][0], b = kDopTriple.t[t][1], c = kDopTriple.t[t][2];
+        int A[3], B[3], C[3];
+        for (int k = 0; k < 3; k++) {
+            A[k] = (a & 1) ? -kDopAxis[a >> 1][k] : kDopAxis[a >> 1][k];
+            B[k] = (b & 1) ? -kDopAxis[b >> 1][k] : kDopAxis[b >> 1][k];
+            C[k] = (c & 1) ? -kDopAxis[c >> 1][k] : kDopAxis[c >> 1][k];
+        }
+        // rows of the adjugate: point = (ha (B x C) + hb (C x A) + hc (A x B)) / det
+        const int bc[3] = {B[1] * C[2] - B[2] * C[1], B[2] * C[0] - B[0] * C[2], B[0] * C[1] - B[1] * C[0]};
+        const int ca[3] = {C[1] * A[2] - C[2] * A[1], C[2] * A[0] - C[0] * A[2], C[0] * A[1] - C[1] * A[0]};
+        const int ab[3] = {A[1] * B[2] - A[2] * B[1], A[2] * B[0] - A[0] * B[2], A[0] * B[1] - A[1] * B[0]};
+        const int det = A[0] * bc[0] + A[1] * bc[1] + A[2] * bc[2];
+        if (det != 0) {
+            // heights / 32: no sum below can overflow, and every comparison is relative
+            const float ha = phf[a] / 32.0f, hb = phf[b] / 32.0f, hc = phf[c] / 32.0f, r = 1.0f / (float)det;
+            const float x = (ha * (float)bc[0] + hb * (float)ca[0] + hc * (float)ab[0]) * r;
+            const float y = (ha * (float)bc[1] + hb * (float)ca[1] + hc * (float)ab[1]) * r;
+            const float z = (ha * (float)bc[2] + hb * (float)ca[2] + hc * (float)ab[2]) * r;
+            pass = true;
+            for (int j = 0; j < 14; j++)
+                pass = pass && !(dop_dot(j, x, y, z) > phf[j] / 32.0f + 3.125e-7f * scale_f + 1e-37f);
+        }
+    }
+    // the triples that pass, in order
+    const unsigned pb = __ballot_sync(0xFFFFFFFFu, pass);
+    if (lane == 0) warp_sums[warp] = (uint32_t)__popc(pb);
+    __syncthreads();
+    uint32_t before = 0, npts = 0;
+    for (uint32_t w = 0; w < kFinishThreads / 32; w++) {
+        if (w < warp) before += warp_sums[w];
+        npts += warp_sums[w];
+    }
+    if (pass) list[before + (uint32_t)__popc(pb & lt)] = (uint16_t)t;
+    __syncthreads();
+    for (uint32_t i = t; i < npts; i += kFinishThreads) {
+        const int id = list[i];
+        int P[3][3];
+        double H[3];
+        for (int q = 0; q < 3; q++) {
+            const int a = kDopTriple.t[id][q];
+            for (int k = 0; k < 3; k++) P[q][k] = (a & 1) ? -kDopAxis[a >> 1][k] : kDopAxis[a >> 1][k];
+            H[q] = (double)phf[a];
+        }
+        // Cramer's rule on the rows A, B, C.  Their entries are 0 or +-1 and the
+        // determinant is +-1, +-2 or +-4, so its reciprocal is exact and only the
+        // sums below round.
+        const int *A = P[0], *B = P[1], *C = P[2];
+        const int det = A[0] * (B[1] * C[2] - B[2] * C[1]) - A[1] * (B[0] * C[2] - B[2] * C[0]) +
+                        A[2] * (B[0] * C[1] - B[1] * C[0]);
+        const double r = (double)(1.0f / (float)det);
+        const double x = (H[0] * (B[1] * C[2] - B[2] * C[1]) - A[1] * (H[1] * C[2] - B[2] * H[2]) +
+                          A[2] * (H[1] * C[1] - B[1] * H[2])) * r;
+        const double y = (A[0] * (H[1] * C[2] - B[2] * H[2]) - H[0] * (B[0] * C[2] - B[2] * C[0]) +
+                          A[2] * (B[0] * H[2] - H[1] * C[0])) * r;
+        const double z = (A[0] * (B[1] * H[2] - H[1] * C[1]) - A[1] * (B[0] * H[2] - H[1] * C[0]) +
+                          H[0] * (B[0] * C[1] - B[1] * C[0])) * r;
+        const double slack = 1e-9 * scale;
+        const double along[7] = {x, y, z, x + y + z, x + y - z, x - y + z, y - x + z};  // kDopAxis
+        bool inside = true;
+        for (int k = 0; k < 7; k++)
+            inside = inside && along[k] <= (double)phf[2 * k] + slack && -along[k] <= (double)phf[2 * k + 1] + slack;
+        cand[i][0] = x;
+        cand[i][1] = y;
+        cand[i][2] = z;
+        candf[i][0] = (float)x;
+        candf[i][1] = (float)y;
+        candf[i][2] = (float)z;
+        found[i] = inside ? 1 : 0;
+    }
+    __syncthreads();
+    // A pair is a duplicate when every coordinate differs by at most 1e-7
+    // scale (in double).  The float copies screen the pairs first: every
+    // coordinate is within scale (1 + 1e-9) (the axis planes bound it), so
+    // rounding to float moves a difference by at most 2^-23 scale, and a
+    // pair whose float difference exceeds 4e-7 scale cannot pass the double
+    // test.
+    const double tol = 1e-7 * scale;
+    const float tolf = 4e-7f * (float)scale;
+    bool keep = t < npts && found[t] != 0;
+    for (uint32_t j = 0; j < t && keep; j++) {
+        if (!found[j] || fabsf(candf[t][0] - candf[j][0]) > tolf || fabsf(candf[t][1] - candf[j][1]) > tolf ||
+            fabsf(candf[t][2] - candf[j][2]) > tolf)
+            continue;
+        keep = !(fabs(cand[t][0] - cand[j][0]) <= tol && fabs(cand[t][1] - cand[j][1]) <= tol &&
+                 fabs(cand[t][2] - cand[j][2]) <= tol);
+    }
+    const unsigned kb = __ballot_sync(0xFFFFFFFFu, keep);
+    if (lane == 0) warp_sums[warp] = (uint32_t)__popc(kb);
+    __syncthreads();
+    before = 0;
+    uint32_t nv = 0;
+    for (uint32_t w = 0; w < kFinishThreads / 32; w++) {
+        if (w < warp) before += warp_sums[w];
+        nv += warp_sums[w];
+    }
+    if (nv < 4u || nv > kDopMaxVertices) return;  // more points than a 14-DOP has, or too few: leave it off
+    if (keep)
+        for (int a = 0; a < 3; a++) h->dop_vertex[before + (uint32_t)__popc(kb & lt)][a] = candf[t][a];
+    if (t == 0) h->dop_count = nv;
 }
 
 // ---- TLAS refit ---------------------------------------------------------------------
@@ -2238,7 +2247,7 @@ ScratchLayout ScratchLayout::make(uint32_t n, bool top, uint32_t build_flags) {
         return r;
     };
     s.sort_blocks = onesweep_partitions((uint32_t)nn);
-    s.state = take(sizeof(BuildState));
+    s.state = take(kBuildStateBytes);
     s.boxes = take(nn * 32);
     s.sboxes = take(nn * 32);
     s.keys0 = take(nn * 4);
@@ -2380,7 +2389,6 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
             note_launch(), k_write_tris<<<blocks_for(n, T), T, 0, stream>>>(*blas, vals[cur], perm,
                                                                              reinterpret_cast<TriRecord*>(dst + al.prims),
                                                                              st);
-            note_launch(), k_dop_vertices<<<kDopBlocks, kDopThreads, 0, stream>>>(reinterpret_cast<AsHeader*>(dst), st);
         }
     } else {
         CollapseCtx cc{};
@@ -2411,7 +2419,7 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     hs.prims_offset = al.prims;
     hs.parents_offset = al.parents;
     hs.prim_bytes = top ? kInstBytes : kTriBytes;
-    note_launch(), k_finalize<<<1, 32, 0, stream>>>(reinterpret_cast<AsHeader*>(dst), st, hs);
+    note_launch(), k_finish<<<1, kFinishThreads, 0, stream>>>(reinterpret_cast<AsHeader*>(dst), st, hs);
     return cudaGetLastError();
 }
 
