@@ -19,6 +19,8 @@
 //      follow each other in slot order, and a leaf child writes its
 //      primitives' positions (perm).
 //   6. primitive records written in that final order.
+// A TLAS of 2 to kTlasSmall instances goes through all of it in one block
+// (k_tlas_small), whatever the build flags.
 // Everything runs on the caller's stream; no host synchronisation.
 //
 // Replaces vkCmdBuildAccelerationStructuresKHR as called by
@@ -148,7 +150,7 @@ __device__ void reduce_bounds(BuildState* st, const float cmin[3], const float c
     }
 }
 
-__global__ void k_init_state(BuildState* st, uint32_t n) {
+__device__ __forceinline__ void init_state(BuildState* st, uint32_t n) {
     for (uint32_t i = threadIdx.x; i < kPlocMaxRounds; i += blockDim.x) st->ploc_ticket[i] = 0;
     if (threadIdx.x == 0) {
         st->ploc_round[0] = n;
@@ -173,6 +175,7 @@ __global__ void k_init_state(BuildState* st, uint32_t n) {
         }
     }
 }
+__global__ void k_init_state(BuildState* st, uint32_t n) { init_state(st, n); }
 
 __device__ __forceinline__ int find_geometry(const BlasInput& in, uint32_t i) {
     int lo = 0, hi = (int)in.geometry_count - 1;
@@ -376,10 +379,9 @@ __device__ bool fill_instance(const RtAccelerationStructureInstance& r, uint32_t
     return valid;
 }
 
-__global__ void k_tlas_prims(const RtAccelerationStructureInstance* inst, uint32_t n, float4* boxes,
-                             InstRecord* temp, BuildState* st, ZeroedWords z) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    zero_words(z, i, gridDim.x * blockDim.x);
+// Instance i's record and box; every thread of the block takes part in the bounds.
+__device__ __forceinline__ void tlas_prim(const RtAccelerationStructureInstance* inst, uint32_t i, uint32_t n,
+                                          InstRecord* temp, BuildState* st, float4& blo, float4& bhi) {
     float cmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float bmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, bmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     uint32_t kinds = 0;
@@ -397,12 +399,24 @@ __global__ void k_tlas_prims(const RtAccelerationStructureInstance* inst, uint32
             kinds = blas_kind(rec.node_count);
         }
         temp[i] = rec;
-        boxes[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-        boxes[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        blo = make_float4(lo[0], lo[1], lo[2], 0.0f);
+        bhi = make_float4(hi[0], hi[1], hi[2], 0.0f);
     }
     kinds = __reduce_or_sync(0xFFFFFFFFu, kinds);
     if ((threadIdx.x & 31u) == 0 && kinds) atomicOr(&st->blas_kinds, kinds);
     reduce_bounds(st, cmin, cmax, bmin, bmax);
+}
+
+__global__ void k_tlas_prims(const RtAccelerationStructureInstance* inst, uint32_t n, float4* boxes,
+                             InstRecord* temp, BuildState* st, ZeroedWords z) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    zero_words(z, i, gridDim.x * blockDim.x);
+    float4 lo, hi;
+    tlas_prim(inst, i, n, temp, st, lo, hi);
+    if (i < n) {
+        boxes[2 * (size_t)i] = lo;
+        boxes[2 * (size_t)i + 1] = hi;
+    }
 }
 
 __device__ __forceinline__ uint32_t expand_bits10(uint32_t x) {
@@ -413,9 +427,8 @@ __device__ __forceinline__ uint32_t expand_bits10(uint32_t x) {
     return x;
 }
 
-// 30-bit Morton code of the centroid of box i.
-__device__ __forceinline__ uint32_t morton_code(const float4* boxes, uint32_t i, const BuildState* st) {
-    const float4 lo = boxes[2 * (size_t)i], hi = boxes[2 * (size_t)i + 1];
+// 30-bit Morton code of a box's centroid.
+__device__ __forceinline__ uint32_t morton_code(float4 lo, float4 hi, const BuildState* st) {
     const float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
     uint32_t q[3] = {0, 0, 0};
     if (finite3(c)) {
@@ -453,23 +466,16 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d) {
 // launches are as fast.
 constexpr uint32_t kSortRow = kSortThreads / 32 + 1;  // counts of one digit by warp, padded against bank conflicts
 constexpr size_t sort_block_smem(int items) { return (256 * kSortRow + 2 * (size_t)items * kSortThreads) * 4; }
-template <bool MORTON, int ITEMS>
-__global__ void __launch_bounds__(kSortThreads) k_sort_block(uint32_t* k, uint32_t* v, uint32_t n, const float4* boxes,
-                                                             const BuildState* st) {
-    extern __shared__ uint32_t sort_smem[];
-    __shared__ uint32_t warp_sums[kSortThreads / 32];
+// The calling block (kSortThreads threads) sorts the pairs it holds: item r of
+// a thread is number warp * ITEMS * 32 + 32 r + lane, before and after.
+template <int ITEMS>
+__device__ __forceinline__ void block_sort(uint32_t (&key)[ITEMS], uint32_t (&val)[ITEMS], uint32_t* sort_smem,
+                                           uint32_t* warp_sums) {
     uint32_t* cnt = sort_smem;
     uint32_t* skeys = cnt + 256 * kSortRow;
     uint32_t* svals = skeys + ITEMS * kSortThreads;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = (1u << lane) - 1u;
-    const uint32_t first = warp * ITEMS * 32u + lane;  // item r of this thread: first + 32 r
-    uint32_t key[ITEMS], val[ITEMS];
-#pragma unroll
-    for (int r = 0; r < ITEMS; r++) {
-        const uint32_t i = first + 32u * r;
-        key[r] = i < n ? (MORTON ? morton_code(boxes, i, st) : k[i]) : 0xFFFFFFFFu;
-        val[r] = i < n ? (MORTON ? i : v[i]) : 0u;
-    }
+    const uint32_t first = warp * ITEMS * 32u + lane;
     for (int shift = 0; shift < 32; shift += 8) {
         for (uint32_t i = tid; i < 256 * kSortRow; i += kSortThreads) cnt[i] = 0;
         __syncthreads();
@@ -518,6 +524,26 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_block(uint32_t* k, uint32
             val[r] = svals[first + 32u * r];
         }
     }
+}
+
+template <bool MORTON, int ITEMS>
+__global__ void __launch_bounds__(kSortThreads) k_sort_block(uint32_t* k, uint32_t* v, uint32_t n, const float4* boxes,
+                                                             const BuildState* st) {
+    extern __shared__ uint32_t sort_smem[];
+    __shared__ uint32_t warp_sums[kSortThreads / 32];
+    const uint32_t first = (threadIdx.x >> 5) * ITEMS * 32u + (threadIdx.x & 31u);  // item r of this thread: first + 32 r
+    uint32_t key[ITEMS], val[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++) {
+        const uint32_t i = first + 32u * r;
+        key[r] = 0xFFFFFFFFu;
+        val[r] = 0u;
+        if (i < n) {
+            key[r] = MORTON ? morton_code(boxes[2 * (size_t)i], boxes[2 * (size_t)i + 1], st) : k[i];
+            val[r] = MORTON ? i : v[i];
+        }
+    }
+    block_sort<ITEMS>(key, val, sort_smem, warp_sums);
 #pragma unroll
     for (int r = 0; r < ITEMS; r++) {
         const uint32_t i = first + 32u * r;
@@ -580,7 +606,7 @@ __global__ void __launch_bounds__(kOsThreads) k_onesweep_hist(uint32_t* keys, ui
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t k;
         if (MORTON) {
-            k = morton_code(boxes, i, st);
+            k = morton_code(boxes[2 * (size_t)i], boxes[2 * (size_t)i + 1], st);
             keys[i] = k;
             vals[i] = i;
         } else {
@@ -1204,75 +1230,13 @@ struct PlocTailShared {
     float area[kPlocRadius][kPlocSmall];
     uint32_t warp_sums[32];
 };
-__global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant__ PlocArgs a, int round) {
-    extern __shared__ float4 ploc_smem[];
-    PlocTailShared& s = *reinterpret_cast<PlocTailShared*>(ploc_smem);
+// Rounds until one of the `count` clusters in s is left; returns the merges
+// so far.  write_node(id, a, b, lo, hi, size) stores an internal node.
+template <class W>
+__device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t count, uint32_t merges, uint32_t n,
+                                                     uint32_t* error, W write_node) {
     constexpr int R = kPlocRadius;
-    BuildState* st = a.st;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t word = st->ploc_round[round];
-    uint32_t count = word & kPlocCount, merges = st->merge_counter;
-    float4* c = a.cbox[(word & kPlocParity) ? 1 : 0];
-    if (count == 0u) {
-        if (tid == 0) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
-        return;
-    }
-    while (count > kPlocSmall) {  // pair q takes positions 2q, 2q + 1 and is stored at q (behind every later read)
-        const uint32_t pairs = (count + 1u) / 2u;
-        for (uint32_t base = 0; base < pairs; base += blockDim.x) {
-            const uint32_t q = base + tid;
-            float4 lo, hi, l2, h2;
-            const bool on = q < pairs, two = on && 2u * q + 1u < count;
-            if (on) {
-                lo = __ldcg(&c[4 * (size_t)q]);
-                hi = __ldcg(&c[4 * (size_t)q + 1]);
-            }
-            if (two) {
-                l2 = __ldcg(&c[4 * (size_t)q + 2]);
-                h2 = __ldcg(&c[4 * (size_t)q + 3]);
-            }
-            __syncthreads();
-            if (two) {
-                const uint32_t claim = merges + q;
-                const uint32_t ra = __float_as_uint(lo.w), rb = __float_as_uint(l2.w);
-                const uint32_t size = __float_as_uint(hi.w) + __float_as_uint(h2.w);
-                if (claim + 2u <= a.n) {
-                    const uint32_t id = a.n - 2u - claim;
-                    lo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), __uint_as_float(id));
-                    hi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), __uint_as_float(size));
-                    ploc_write_node(a, id, ra, rb, lo, hi, size);
-                } else {
-                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
-                }
-            }
-            if (on) {
-                c[2 * (size_t)q] = lo;
-                c[2 * (size_t)q + 1] = hi;
-            }
-            __syncthreads();
-        }
-        merges += count / 2u;
-        count = pairs;
-    }
-    if (tid < count) {
-        float4 lo, hi;
-        if (round == 0) {  // no grid-wide round: gather the primitives here
-            const size_t p = a.vals[tid];
-            lo = a.boxes[2 * p];
-            hi = a.boxes[2 * p + 1];
-            a.sboxes[2 * (size_t)tid] = lo;
-            a.sboxes[2 * (size_t)tid + 1] = hi;
-            lo.w = __uint_as_float(kLeafBit | tid);
-            hi.w = __uint_as_float(1u);
-        } else {
-            lo = __ldcg(&c[2 * (size_t)tid]);
-            hi = __ldcg(&c[2 * (size_t)tid + 1]);
-        }
-        s.s0[tid] = make_float4(lo.x, lo.y, lo.z, hi.x);
-        s.s1[tid] = make_float2(hi.y, hi.z);
-        s.ref[tid] = make_uint2(__float_as_uint(lo.w), __float_as_uint(hi.w));
-    }
-    __syncthreads();
     bool forced = false;
     while (count > 1u) {  // a round after one without a merge merges pairs: it ends
         const uint32_t blocks = (count + 31u) >> 5;  // of 32 clusters
@@ -1365,13 +1329,13 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
             const uint32_t lt = (1u << lane) - 1u;
             if (merge) {
                 const uint32_t claim = merges + (before >> 16) + (uint32_t)__popc(mb & lt);
-                if (claim + 2u <= a.n) {
-                    const uint32_t id = a.n - 2u - claim;
-                    ploc_write_node(a, id, r.x, partner, make_float4(p.x, p.y, p.z, 0.f),
-                                    make_float4(p.w, q.x, q.y, 0.f), r.y);
+                if (claim + 2u <= n) {
+                    const uint32_t id = n - 2u - claim;
+                    write_node(id, r.x, partner, make_float4(p.x, p.y, p.z, 0.f),
+                               make_float4(p.w, q.x, q.y, 0.f), r.y);
                     r.x = id;
                 } else {
-                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                    atomicOr(error, 1u << RT_ERR_BAD_AS);
                 }
             }
             if (keep) {
@@ -1386,6 +1350,80 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
         count = total & 0xFFFFu;
         __syncthreads();
     }
+    return merges;
+}
+__global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant__ PlocArgs a, int round) {
+    extern __shared__ float4 ploc_smem[];
+    PlocTailShared& s = *reinterpret_cast<PlocTailShared*>(ploc_smem);
+    BuildState* st = a.st;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t word = st->ploc_round[round];
+    uint32_t count = word & kPlocCount, merges = st->merge_counter;
+    float4* c = a.cbox[(word & kPlocParity) ? 1 : 0];
+    if (count == 0u) {
+        if (tid == 0) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+        return;
+    }
+    while (count > kPlocSmall) {  // pair q takes positions 2q, 2q + 1 and is stored at q (behind every later read)
+        const uint32_t pairs = (count + 1u) / 2u;
+        for (uint32_t base = 0; base < pairs; base += blockDim.x) {
+            const uint32_t q = base + tid;
+            float4 lo, hi, l2, h2;
+            const bool on = q < pairs, two = on && 2u * q + 1u < count;
+            if (on) {
+                lo = __ldcg(&c[4 * (size_t)q]);
+                hi = __ldcg(&c[4 * (size_t)q + 1]);
+            }
+            if (two) {
+                l2 = __ldcg(&c[4 * (size_t)q + 2]);
+                h2 = __ldcg(&c[4 * (size_t)q + 3]);
+            }
+            __syncthreads();
+            if (two) {
+                const uint32_t claim = merges + q;
+                const uint32_t ra = __float_as_uint(lo.w), rb = __float_as_uint(l2.w);
+                const uint32_t size = __float_as_uint(hi.w) + __float_as_uint(h2.w);
+                if (claim + 2u <= a.n) {
+                    const uint32_t id = a.n - 2u - claim;
+                    lo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), __uint_as_float(id));
+                    hi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), __uint_as_float(size));
+                    ploc_write_node(a, id, ra, rb, lo, hi, size);
+                } else {
+                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                }
+            }
+            if (on) {
+                c[2 * (size_t)q] = lo;
+                c[2 * (size_t)q + 1] = hi;
+            }
+            __syncthreads();
+        }
+        merges += count / 2u;
+        count = pairs;
+    }
+    if (tid < count) {
+        float4 lo, hi;
+        if (round == 0) {  // no grid-wide round: gather the primitives here
+            const size_t p = a.vals[tid];
+            lo = a.boxes[2 * p];
+            hi = a.boxes[2 * p + 1];
+            a.sboxes[2 * (size_t)tid] = lo;
+            a.sboxes[2 * (size_t)tid + 1] = hi;
+            lo.w = __uint_as_float(kLeafBit | tid);
+            hi.w = __uint_as_float(1u);
+        } else {
+            lo = __ldcg(&c[2 * (size_t)tid]);
+            hi = __ldcg(&c[2 * (size_t)tid + 1]);
+        }
+        s.s0[tid] = make_float4(lo.x, lo.y, lo.z, hi.x);
+        s.s1[tid] = make_float2(hi.y, hi.z);
+        s.ref[tid] = make_uint2(__float_as_uint(lo.w), __float_as_uint(hi.w));
+    }
+    __syncthreads();
+    merges = ploc_tail_rounds(s, count, merges, a.n, &st->error, [&](uint32_t id, uint32_t ra, uint32_t rb, float4 lo,
+                                                                     float4 hi, uint32_t size) {
+        ploc_write_node(a, id, ra, rb, lo, hi, size);
+    });
     if (tid == 0) st->merge_counter = merges;
 }
 
@@ -1462,11 +1500,24 @@ __device__ void write_single_leaf(const CollapseCtx& c) {
     for (uint32_t i = 0; i < c.n; i++) c.perm[i] = i;
 }
 
-__global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_constant__ CollapseCtx c) {
-    if (c.n <= c.leaf_max) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) write_single_leaf(c);
-        return;
-    }
+// Words that other lanes write while this one waits: in the memory of the GPU,
+// or (SHARED) in the shared memory of a build that one block does alone.
+template <bool SHARED, class T>
+__device__ __forceinline__ T queue_load(const T* p) {
+    if constexpr (SHARED) return *const_cast<const volatile T*>(p);
+    else if constexpr (sizeof(T) == 8) return ld_relaxed64(p);
+    else return ld_relaxed(p);
+}
+template <bool SHARED, class T>
+__device__ __forceinline__ void queue_store(T* p, T v) {
+    if constexpr (SHARED) *const_cast<volatile T*>(p) = v;
+    else if constexpr (sizeof(T) == 8) st_relaxed64(p, v);
+    else st_relaxed(p, v);
+}
+
+// Works on tasks until every primitive is in a leaf (n > leaf_max; all lanes of the warp).
+template <bool SHARED>
+__device__ __forceinline__ void collapse_loop(const CollapseCtx& c) {
     const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, group = lane & 24u;
     const uint32_t lt = (1u << lane) - 1u;
     BuildState* st = c.st;
@@ -1482,10 +1533,10 @@ __global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_c
         }
         unsigned long long task = 0;
         if (slot == 0u) task = collapse_task(0u, 0u, 0u);
-        else if (slot < c.max_nodes) task = ld_relaxed64(&c.tasks[slot]);
+        else if (slot < c.max_nodes) task = queue_load<SHARED>(&c.tasks[slot]);
         const bool ready = task != 0;
         if (!__any_sync(0xFFFFFFFFu, ready)) {
-            if (ld_relaxed(&st->collapse_done)) break;
+            if (queue_load<SHARED>(&st->collapse_done)) break;
             if (++spins > kCollapseSpinLimit) {
                 if (lane == 0) atomicOr(&st->error, 1u << RT_ERR_TIMEOUT);
                 break;
@@ -1573,7 +1624,7 @@ __global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_c
             before = atomicAdd(&st->progress, ((unsigned long long)placed << 32) | (uint32_t)__popc(inners));
             if ((uint32_t)(before >> 32) + placed >= c.n) {  // the last primitives: no task is left
                 st->node_count = (uint32_t)before + (uint32_t)__popc(inners);
-                st_relaxed(&st->collapse_done, 1u);
+                queue_store<SHARED>(&st->collapse_done, 1u);
             }
         }
         const uint32_t cs = (uint32_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)before, 0) + (uint32_t)__popc(inners & lt);
@@ -1584,11 +1635,11 @@ __global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_c
             entry = cs;
             if (cs >= c.max_nodes) {  // more nodes than any hierarchy of n primitives has: give up
                 atomicOr(&st->error, 1u << RT_ERR_TOO_LARGE);
-                st_relaxed(&st->collapse_done, 1u);
+                queue_store<SHARED>(&st->collapse_done, 1u);
                 used = false;
             } else {
                 if (c.parents) c.parents[cs] = slot;
-                st_relaxed64(&c.tasks[cs], collapse_task(r, at, depth + 1u));
+                queue_store<SHARED>(&c.tasks[cs], collapse_task(r, at, depth + 1u));
             }
         } else if (leaf) {
             meta = size;
@@ -1623,6 +1674,11 @@ __global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_c
     }
     depth_seen = __reduce_max_sync(0xFFFFFFFFu, depth_seen);
     if (lane == 0 && depth_seen > 1u) atomicMax(&st->depth, depth_seen);
+}
+
+__global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_constant__ CollapseCtx c) {
+    if (c.n > c.leaf_max) collapse_loop<false>(c);
+    else if (blockIdx.x == 0 && threadIdx.x == 0) write_single_leaf(c);
 }
 
 // ---- primitive records ----------------------------------------------------------
@@ -2016,6 +2072,99 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const Bu
     if (t == 0) h->dop_count = nv;
 }
 
+// ---- small TLAS in one block ----------------------------------------------------------
+// A TLAS of 2 to 1,024 instances, one thread each: records and boxes, Morton
+// sort, PLOC and the collapse in shared memory, one launch.  A frame rebuilds
+// such a TLAS before it traces, and eight launches that each work on a few
+// hundred instances were mostly launch and L2 latency.  Bound: latency, the
+// rounds of the clustering first.  (17 instances 117 -> 33 us,
+// 256 instances 190 -> 66 us.)  Above 1,024 the grid-wide path takes over, with
+// its first round on more than one SM.
+constexpr uint32_t kTlasSmall = 1024;
+static_assert(kTlasSmall == kPlocSmall && kTlasSmall == kSortThreads, "one thread per instance");
+struct TlasSmallArgs {
+    const RtAccelerationStructureInstance* inst;
+    InstRecord* temp;      // records in caller order (scratch)
+    AsHeader* header;
+    WideNode* nodes;
+    uint32_t* parents;
+    InstRecord* out;
+    uint32_t n, width, max_nodes;
+};
+struct TlasSmallShared {
+    BuildState st;
+    union {
+        struct {
+            uint32_t sort[(256 * kSortRow + 2 * kTlasSmall)];
+            float4 boxes[2 * kTlasSmall];  // in caller order
+        };
+        PlocTailShared ploc;
+        unsigned long long tasks[kTlasSmall + 2];
+    };
+    uint32_t vals[kTlasSmall], perm[kTlasSmall];
+    float4 sboxes[2 * kTlasSmall], iboxes[2 * kTlasSmall];
+    uint4 inodes[kTlasSmall];
+    uint32_t warp_sums[32];
+};
+__global__ void __launch_bounds__(kTlasSmall) k_tlas_small(const __grid_constant__ TlasSmallArgs a,
+                                                           const __grid_constant__ HeaderStatic hs) {
+    extern __shared__ float4 tlas_smem[];
+    TlasSmallShared& s = *reinterpret_cast<TlasSmallShared*>(tlas_smem);
+    const uint32_t tid = threadIdx.x, n = a.n;
+    init_state(&s.st, n);
+    __syncthreads();
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+    tlas_prim(a.inst, tid, n, a.temp, &s.st, lo, hi);
+    s.boxes[2 * tid] = lo;
+    s.boxes[2 * tid + 1] = hi;
+    __syncthreads();
+    uint32_t key[1] = {tid < n ? morton_code(lo, hi, &s.st) : 0xFFFFFFFFu}, val[1] = {tid};
+    block_sort<1>(key, val, s.sort, s.warp_sums);  // threads past n keep the last places
+    if (tid < n) {
+        lo = s.boxes[2 * val[0]];
+        hi = s.boxes[2 * val[0] + 1];
+        s.vals[tid] = val[0];
+        s.sboxes[2 * tid] = lo;
+        s.sboxes[2 * tid + 1] = hi;
+    }
+    __syncthreads();  // the boxes have been read: their place is the clusters' now
+    if (tid < n) {
+        s.ploc.s0[tid] = make_float4(lo.x, lo.y, lo.z, hi.x);
+        s.ploc.s1[tid] = make_float2(hi.y, hi.z);
+        s.ploc.ref[tid] = make_uint2(kLeafBit | tid, 1u);
+    }
+    __syncthreads();
+    ploc_tail_rounds(s.ploc, n, 0u, n, &s.st.error, [&](uint32_t id, uint32_t ra, uint32_t rb, float4 l, float4 h,
+                                                        uint32_t size) {
+        s.inodes[id] = make_uint4(ra, rb, 0u, 0u);
+        s.iboxes[2 * id] = make_float4(l.x, l.y, l.z, __uint_as_float(size));
+        s.iboxes[2 * id + 1] = h;
+    });
+    for (uint32_t i = tid; i < a.max_nodes; i += kTlasSmall) s.tasks[i] = 0ull;
+    __syncthreads();
+    CollapseCtx c;
+    c.inodes = s.inodes;
+    c.iboxes = s.iboxes;
+    c.sboxes = s.sboxes;
+    c.nodes = a.nodes;
+    c.parents = a.parents;
+    c.st = &s.st;
+    c.tasks = s.tasks;
+    c.perm = s.perm;
+    c.leaf_max = kTlasLeafMax;
+    c.width = a.width;
+    c.max_nodes = a.max_nodes;
+    c.n = n;
+    if ((tid >> 5) * 4u < a.max_nodes) collapse_loop<true>(c);  // a warp works on four nodes
+    __syncthreads();
+    if (tid == 0) write_header(a.header, &s.st, hs);
+    // eight lanes copy a record (temp was written by this block)
+    for (uint32_t i = tid >> 3; i < n; i += kTlasSmall / 8u) {
+        const uint32_t from = s.vals[min(s.perm[i], n - 1u)];
+        reinterpret_cast<uint4*>(&a.out[i])[tid & 7u] = __ldcg(reinterpret_cast<const uint4*>(&a.temp[from]) + (tid & 7u));
+    }
+}
+
 // ---- TLAS refit ---------------------------------------------------------------------
 __global__ void k_refit_insts(const RtAccelerationStructureInstance* inst, uint32_t n, AsHeader* h,
                               float4* sboxes, uint32_t* err) {
@@ -2324,6 +2473,38 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
                                    sl.ploc ? blocks_for(n, kPlocTile) : 0u, sl.ploc ? task_count : 0u};
     const ZeroedWords zero_karras = {nullptr, tasks, 0u, task_count};
 
+    HeaderStatic hs;
+    hs.node_bytes = al.node_bytes;
+    hs.type = top ? kAsTypeTop : kAsTypeBottom;
+    hs.build_flags = build_flags;
+    hs.prim_count = n;
+    hs.max_nodes = al.max_nodes;
+    hs.geometry_count = geometry_count;
+    hs.leaf_max = top ? kTlasLeafMax : kBlasLeafMax;
+    hs.total_size = al.total;
+    hs.nodes_offset = al.nodes;
+    hs.prims_offset = al.prims;
+    hs.parents_offset = al.parents;
+    hs.prim_bytes = top ? kInstBytes : kTriBytes;
+
+    if (top && n > kTlasLeafMax && n <= kTlasSmall) {
+        // a per-device attribute: set on every build (a host-side call, no device work)
+        const cudaError_t smem_ok = cudaFuncSetAttribute(k_tlas_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)sizeof(TlasSmallShared));
+        if (smem_ok != cudaSuccess) return smem_ok;
+        TlasSmallArgs ta;
+        ta.inst = inst;
+        ta.temp = temp;
+        ta.header = reinterpret_cast<AsHeader*>(dst);
+        ta.nodes = fp32_nodes;
+        ta.parents = reinterpret_cast<uint32_t*>(dst + al.parents);
+        ta.out = reinterpret_cast<InstRecord*>(dst + al.prims);
+        ta.n = n;
+        ta.width = node_width(build_flags);
+        ta.max_nodes = al.max_nodes;
+        note_launch(), k_tlas_small<<<1, kTlasSmall, sizeof(TlasSmallShared), stream>>>(ta, hs);
+        return cudaGetLastError();
+    }
     note_launch(), k_init_state<<<1, 32, 0, stream>>>(st, n);
     if (n > 0) {
         if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st, zero_ploc);
@@ -2406,19 +2587,6 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         note_launch(), k_quantize_nodes<<<g, 128, 0, stream>>>(fp32_nodes, st, al.max_nodes,
                                                                reinterpret_cast<QNode*>(dst + al.nodes));
     }
-    HeaderStatic hs;
-    hs.node_bytes = al.node_bytes;
-    hs.type = top ? kAsTypeTop : kAsTypeBottom;
-    hs.build_flags = build_flags;
-    hs.prim_count = n;
-    hs.max_nodes = al.max_nodes;
-    hs.geometry_count = geometry_count;
-    hs.leaf_max = top ? kTlasLeafMax : kBlasLeafMax;
-    hs.total_size = al.total;
-    hs.nodes_offset = al.nodes;
-    hs.prims_offset = al.prims;
-    hs.parents_offset = al.parents;
-    hs.prim_bytes = top ? kInstBytes : kTriBytes;
     note_launch(), k_finish<<<1, kFinishThreads, 0, stream>>>(reinterpret_cast<AsHeader*>(dst), st, hs);
     return cudaGetLastError();
 }
