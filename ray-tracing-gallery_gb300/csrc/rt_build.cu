@@ -1238,7 +1238,7 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
     constexpr int R = kPlocRadius;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     bool forced = false;
-    while (count > 1u) {  // a round after one without a merge merges pairs: it ends
+    while (count > 1u) {  // a round after one with next to no merges merges pairs: it ends
         const uint32_t blocks = (count + 31u) >> 5;  // of 32 clusters
         if (!forced) {
             const int lg = min(4, 31 - __clz(32u / blocks));  // log2 S
@@ -1346,7 +1346,7 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
             }
         }
         merges += total >> 16;
-        forced = (total & 0xFFFFu) == count;
+        forced = (total & 0xFFFFu) > count - 1u - count / 32u;
         count = total & 0xFFFFu;
         __syncthreads();
     }

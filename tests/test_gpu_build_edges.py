@@ -80,7 +80,9 @@ def _check(device, sc, blas_flags, tlas_flags, walk):
     gs = host.GpuScene(device, sc, blas_flags=blas_flags, tlas_flags=tlas_flags)
     rays = scenes.random_rays(3000, 17, 8.0)
     rays["tmax"] = 1e4
+    device.read_stats(reset=True)
     g = host.trace_ray_buffer(device, gs, rays, with_models=False)
+    assert device.read_stats(reset=True)["status"] == 0
     o, _ = O.OracleScene(sc).trace(rays, with_models=False)
     for f in ("t", "u", "v", "instance_id", "geometry_index", "primitive_index", "hit_kind"):
         assert (np.asarray(g[f]).view(np.uint32) == np.asarray(o[f]).view(np.uint32)).all(), f
