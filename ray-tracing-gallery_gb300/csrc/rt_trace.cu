@@ -134,13 +134,6 @@ __device__ __forceinline__ uint32_t octant_offsets(V3 inv) {
     return (inv.x < 0.0f ? 2u : 0u) | ((inv.y < 0.0f ? 6u : 4u) << 8) | ((inv.z < 0.0f ? 10u : 8u) << 16);
 }
 
-__device__ __forceinline__ uint32_t pick8(const uint32_t v[8], uint32_t s) {
-    uint32_t r = v[0];
-#pragma unroll
-    for (int j = 1; j < 8; j++) r = (s == (uint32_t)j) ? v[j] : r;
-    return r;
-}
-
 #define RT_CSWAP(a, b)                  \
     {                                   \
         uint32_t lo_ = min(k[a], k[b]); \
@@ -257,55 +250,54 @@ __device__ __forceinline__ uint32_t child_key(float tn, float tf, uint32_t ref, 
     return hit ? ((__float_as_uint(fmaxf(tn, 0.0f)) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
 }
 
-// Slab tests of four children (base 0 or 4) of an FP32 node from their
-// near / far plane float4s.
-__device__ __forceinline__ void fnode_keys4(const Trav& s, float4 nx, float4 fx, float4 ny, float4 fy, float4 nz,
-                                            float4 fz, uint4 r, int base, uint32_t keys[8], uint32_t refs[8]) {
-    const float a_nx[4] = {nx.x, nx.y, nx.z, nx.w}, a_fx[4] = {fx.x, fx.y, fx.z, fx.w};
-    const float a_ny[4] = {ny.x, ny.y, ny.z, ny.w}, a_fy[4] = {fy.x, fy.y, fy.z, fy.w};
-    const float a_nz[4] = {nz.x, nz.y, nz.z, nz.w}, a_fz[4] = {fz.x, fz.y, fz.z, fz.w};
-    const uint32_t a_r[4] = {r.x, r.y, r.z, r.w};
-    const float tcap = s.t;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        float tnx = (a_nx[j] - s.o.x) * s.inv.x, tfx = (a_fx[j] - s.o.x) * s.inv.x;
-        float tny = (a_ny[j] - s.o.y) * s.inv.y, tfy = (a_fy[j] - s.o.y) * s.inv.y;
-        float tnz = (a_nz[j] - s.o.z) * s.inv.z, tfz = (a_fz[j] - s.o.z) * s.inv.z;
-        refs[base + j] = a_r[j];
-        keys[base + j] =
-            child_key(fmax3(fmaxf(tnx, s.tmin), tny, tnz), fmin3(fminf(tfx, tcap), tfy, tfz), a_r[j], base + j);
-    }
+// (a - o) * inv of two planes at once: the packed operations round each half
+// as the single ones do.
+__device__ __forceinline__ float2 slab2(float a0, float a1, float neg_o, float inv) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, i;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tmov.b64 i, {%5, %5};\n\t"
+        "add.rn.f32x2 p, p, q;\n\tmul.rn.f32x2 p, p, i;\n\tmov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a0), "f"(a1), "f"(neg_o), "f"(inv));
+    return r;
 }
 
-// Slab tests of an FP32 node.  Near / far planes were chosen per ray by the
-// direction signs (s.oct): the loads fetch them directly, so each child needs
-// one subtract and one multiply per plane and no per-axis min/max.  All eight
-// slots are tested (empty ones never hit): skipping children 4-7 of nodes
-// with at most four children measured slower than the branch saves, 4-wide
-// builds included.
-// Node loads: read-only global loads, or plain loads of a copy the warp
-// staged in shared memory (packet traversal, RT_PACKET_STAGE).
-template <bool GLOBAL, class T>
-__device__ __forceinline__ T ldn(const T* p) {
-    if constexpr (GLOBAL) return __ldg(p);
-    else return *p;
+// Slab tests of children base, base + 1 of an FP32 node.
+__device__ __forceinline__ void fnode_keys2(const Trav& s, float nx0, float nx1, float fx0, float fx1, float ny0,
+                                            float ny1, float fy0, float fy1, float nz0, float nz1, float fz0,
+                                            float fz1, uint32_t r0, uint32_t r1, int base, uint32_t keys[8]) {
+    const float2 tnx = slab2(nx0, nx1, -s.o.x, s.inv.x), tfx = slab2(fx0, fx1, -s.o.x, s.inv.x);
+    const float2 tny = slab2(ny0, ny1, -s.o.y, s.inv.y), tfy = slab2(fy0, fy1, -s.o.y, s.inv.y);
+    const float2 tnz = slab2(nz0, nz1, -s.o.z, s.inv.z), tfz = slab2(fz0, fz1, -s.o.z, s.inv.z);
+    keys[base] = child_key(fmax3(fmaxf(tnx.x, s.tmin), tny.x, tnz.x), fmin3(fminf(tfx.x, s.t), tfy.x, tfz.x), r0, base);
+    keys[base + 1] =
+        child_key(fmax3(fmaxf(tnx.y, s.tmin), tny.y, tnz.y), fmin3(fminf(tfx.y, s.t), tfy.y, tfz.y), r1, base + 1);
 }
 
-template <bool GLOBAL = true>
-__device__ __forceinline__ void fnode_keys_at(const Trav& s, const float4* np, uint32_t keys[8], uint32_t refs[8]) {
+// Slab tests of an FP32 node; refs = its child references, which the caller
+// reads again for the few children it enters or pushes (an L1 hit each).
+// Near / far planes were chosen per ray by the direction signs (s.oct): the
+// loads fetch them directly, so each pair of children needs one packed
+// subtract and one packed multiply per plane and no per-axis min/max.  All
+// eight slots are tested (empty ones never hit): skipping children 4-7 of
+// nodes with at most four children measured slower than the branch saves,
+// 4-wide builds included.  The step is bound by the latency of its dependent
+// instructions and loads at six warps per scheduler (issue 52-62 %): packed
+// arithmetic and references picked by a load instead of seven selects took
+// the 1080p frame from 5.13 to 4.85 ms and serving bursts from 20.1 to 19.1
+// ms; 256-bit plane loads (two registers quads at once) were 1-2 % slower.
+__device__ __forceinline__ const uint32_t* fnode_keys(const Trav& s, uint32_t entry, uint32_t keys[8]) {
+    const float4* np = reinterpret_cast<const float4*>(s.nodes + entry);
     const uint32_t ox = s.oct & 0xFFu, oy = (s.oct >> 8) & 0xFFu, oz = s.oct >> 16;
-    const uint4 r0 = ldn<GLOBAL>(reinterpret_cast<const uint4*>(np + 12));
-    const uint4 r1 = ldn<GLOBAL>(reinterpret_cast<const uint4*>(np + 13));
-    const float4 nx0 = ldn<GLOBAL>(np + ox), fx0 = ldn<GLOBAL>(np + (ox ^ 2u)), ny0 = ldn<GLOBAL>(np + oy);
-    const float4 fy0 = ldn<GLOBAL>(np + (oy ^ 2u)), nz0 = ldn<GLOBAL>(np + oz), fz0 = ldn<GLOBAL>(np + (oz ^ 2u));
-    const float4 nx1 = ldn<GLOBAL>(np + ox + 1), fx1 = ldn<GLOBAL>(np + (ox ^ 2u) + 1), ny1 = ldn<GLOBAL>(np + oy + 1);
-    const float4 fy1 = ldn<GLOBAL>(np + (oy ^ 2u) + 1), nz1 = ldn<GLOBAL>(np + oz + 1);
-    const float4 fz1 = ldn<GLOBAL>(np + (oz ^ 2u) + 1);
-    fnode_keys4(s, nx0, fx0, ny0, fy0, nz0, fz0, r0, 0, keys, refs);
-    fnode_keys4(s, nx1, fx1, ny1, fy1, nz1, fz1, r1, 4, keys, refs);
-}
-__device__ __forceinline__ void fnode_keys(const Trav& s, uint32_t entry, uint32_t keys[8], uint32_t refs[8]) {
-    fnode_keys_at<true>(s, reinterpret_cast<const float4*>(s.nodes + entry), keys, refs);
+    const uint4 r0 = __ldg(reinterpret_cast<const uint4*>(np + 12)), r1 = __ldg(reinterpret_cast<const uint4*>(np + 13));
+    const float4 nx0 = __ldg(np + ox), fx0 = __ldg(np + (ox ^ 2u)), ny0 = __ldg(np + oy);
+    const float4 fy0 = __ldg(np + (oy ^ 2u)), nz0 = __ldg(np + oz), fz0 = __ldg(np + (oz ^ 2u));
+    const float4 nx1 = __ldg(np + ox + 1), fx1 = __ldg(np + (ox ^ 2u) + 1), ny1 = __ldg(np + oy + 1);
+    const float4 fy1 = __ldg(np + (oy ^ 2u) + 1), nz1 = __ldg(np + oz + 1), fz1 = __ldg(np + (oz ^ 2u) + 1);
+    fnode_keys2(s, nx0.x, nx0.y, fx0.x, fx0.y, ny0.x, ny0.y, fy0.x, fy0.y, nz0.x, nz0.y, fz0.x, fz0.y, r0.x, r0.y, 0, keys);
+    fnode_keys2(s, nx0.z, nx0.w, fx0.z, fx0.w, ny0.z, ny0.w, fy0.z, fy0.w, nz0.z, nz0.w, fz0.z, fz0.w, r0.z, r0.w, 2, keys);
+    fnode_keys2(s, nx1.x, nx1.y, fx1.x, fx1.y, ny1.x, ny1.y, fy1.x, fy1.y, nz1.x, nz1.y, fz1.x, fz1.y, r1.x, r1.y, 4, keys);
+    fnode_keys2(s, nx1.z, nx1.w, fx1.z, fx1.w, ny1.z, ny1.w, fy1.z, fy1.w, nz1.z, nz1.w, fz1.z, fz1.w, r1.z, r1.w, 6, keys);
+    return reinterpret_cast<const uint32_t*>(np + 12);
 }
 
 // Byte j of w as the float 1 + q 2^-15: q lands in mantissa bits 8..15 of
@@ -361,20 +353,19 @@ __device__ __noinline__ Keys8 qnode_keys_exact(const uint8_t* node, float ox, fl
 // (the builder rounds every plane outward): every child an FP32 traversal
 // would need is visited, so the hits are identical, whatever the distance
 // between the ray origin and the node.
-template <bool GLOBAL = true>
-__device__ __forceinline__ void qnode_keys_at(const Trav& s, const uint8_t* node, uint32_t keys[8],
-                                              uint32_t refs[8]) {
+__device__ __forceinline__ const uint32_t* qnode_keys(const Trav& s, uint32_t entry, uint32_t keys[8]) {
+    const uint8_t* node = reinterpret_cast<const uint8_t*>(s.nodes) + (size_t)entry * kQNodeBytes;
     const uint4* qp = reinterpret_cast<const uint4*>(node);
     const uint2* q2 = reinterpret_cast<const uint2*>(node);
-    uint4 h = ldn<GLOBAL>(qp), r0 = ldn<GLOBAL>(qp + 1), r1 = ldn<GLOBAL>(qp + 2);
+    const uint32_t* child_ref = reinterpret_cast<const uint32_t*>(node + 16);
+    const uint4 h = __ldg(qp), r0 = __ldg(qp + 1), r1 = __ldg(qp + 2);
     // uint2 index of the near-plane words: qlo at 6 + 2a, qhi at 7 + 2a
     const uint32_t ix = 6u + ((s.oct & 0xFFu) >> 1), iy = 6u + (((s.oct >> 8) & 0xFFu) >> 1),
                    iz = 6u + ((s.oct >> 16) >> 1);
-    uint2 nx = ldn<GLOBAL>(q2 + ix), fx = ldn<GLOBAL>(q2 + (ix ^ 1u));
-    uint2 ny = ldn<GLOBAL>(q2 + iy), fy = ldn<GLOBAL>(q2 + (iy ^ 1u));
-    uint2 nz = ldn<GLOBAL>(q2 + iz), fz = ldn<GLOBAL>(q2 + (iz ^ 1u));
-    refs[0] = r0.x; refs[1] = r0.y; refs[2] = r0.z; refs[3] = r0.w;
-    refs[4] = r1.x; refs[5] = r1.y; refs[6] = r1.z; refs[7] = r1.w;
+    const uint2 nx = __ldg(q2 + ix), fx = __ldg(q2 + (ix ^ 1u));
+    const uint2 ny = __ldg(q2 + iy), fy = __ldg(q2 + (iy ^ 1u));
+    const uint2 nz = __ldg(q2 + iz), fz = __ldg(q2 + (iz ^ 1u));
+    const uint32_t refs[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
     const float Ax = __uint_as_float((h.w & 0xFFu) << 23) * s.inv.x;
     const float Ay = __uint_as_float(((h.w >> 8) & 0xFFu) << 23) * s.inv.y;
     const float Az = __uint_as_float(((h.w >> 16) & 0xFFu) << 23) * s.inv.z;
@@ -383,7 +374,7 @@ __device__ __forceinline__ void qnode_keys_at(const Trav& s, const uint8_t* node
         Keys8 kk = qnode_keys_exact(node, s.o.x, s.o.y, s.o.z, s.inv.x, s.inv.y, s.inv.z, s.tmin, s.t);
 #pragma unroll
         for (int k = 0; k < 8; k++) keys[k] = kk.k[k];
-        return;
+        return child_ref;
     }
     const float Bx = (__uint_as_float(h.x) - s.o.x) * s.inv.x;
     const float By = (__uint_as_float(h.y) - s.o.y) * s.inv.y;
@@ -404,11 +395,8 @@ __device__ __forceinline__ void qnode_keys_at(const Trav& s, const uint8_t* node
         keys[k] = child_key(fmaxf(fmaf(-kQuantRelative, fabsf(tn), tn), tlo),
                             fminf(fmaf(kQuantRelative, fabsf(tf), tf), tcap), refs[k], k);
     }
+    return child_ref;
 }
-__device__ __forceinline__ void qnode_keys(const Trav& s, uint32_t entry, uint32_t keys[8], uint32_t refs[8]) {
-    qnode_keys_at<true>(s, reinterpret_cast<const uint8_t*>(s.nodes) + (size_t)entry * kQNodeBytes, keys, refs);
-}
-
 // (inst, geom, prim) below the best hit's, comparing caller instance indices
 // (only reached on an exact tie in t).
 __device__ __noinline__ bool ids_below_best(const InstRecord* insts, uint32_t c_inst, uint32_t hit_inst,
@@ -558,13 +546,14 @@ __device__ __forceinline__ bool trav_step(Trav& s, STK& stack, const SV& sv, con
             atomicOr(status, 1u << RT_ERR_BAD_AS);  // malformed reference: skip it
         } else {
             if (STATS) cnt.nodes++;
-            uint32_t keys[8], refs[8];
+            uint32_t keys[8];
+            const uint32_t* refs;  // the node's child references
             // TLAS nodes are always FP32
             if ((KINDS & kBlasKindQ8) && s.in_blas && (KINDS == kBlasKindQ8 || s.quant)) {
                 if (STATS) cnt.qnodes++;
-                qnode_keys(s, entry, keys, refs);
+                refs = qnode_keys(s, entry, keys);
             } else {
-                fnode_keys(s, entry, keys, refs);
+                refs = fnode_keys(s, entry, keys);
             }
             if (ray_flags & RT_RAY_FLAG_TERMINATE_ON_FIRST_HIT) {
                 // Any accepted hit ends the ray and t never shrinks before
@@ -574,12 +563,12 @@ __device__ __forceinline__ bool trav_step(Trav& s, STK& stack, const SV& sv, con
 #pragma unroll
                 for (int k = 0; k < 8; k++) mask |= (keys[k] != 0xFFFFFFFFu ? 1u : 0u) << k;
                 if (mask) {
-                    s.entry = pick8(refs, (uint32_t)(__ffs(mask) - 1));
+                    s.entry = __ldg(refs + (__ffs(mask) - 1));
                     mask &= mask - 1u;
                     while (mask) {
                         const uint32_t k = (uint32_t)(__ffs(mask) - 1);
                         mask &= mask - 1u;
-                        if (s.sp < (int)kStackSize) stack.put(s.sp++, make_uint2(pick8(refs, k), 0u));
+                        if (s.sp < (int)kStackSize) stack.put(s.sp++, make_uint2(__ldg(refs + k), 0u));
                         else atomicOr(status, 1u << RT_ERR_STACK_OVERFLOW);
                     }
                     return false;
@@ -594,11 +583,11 @@ __device__ __forceinline__ bool trav_step(Trav& s, STK& stack, const SV& sv, con
                     for (int q = 7; q >= 1; q--) {
                         uint32_t key = keys[q];
                         if (key == 0xFFFFFFFFu) continue;
-                        const uint32_t ref = pick8(refs, key & 7u);
+                        const uint32_t ref = __ldg(refs + (key & 7u));
                         if (s.sp < (int)kStackSize) stack.put(s.sp++, make_uint2(ref, key & ~7u));
                         else atomicOr(status, 1u << RT_ERR_STACK_OVERFLOW);
                     }
-                    s.entry = pick8(refs, keys[0] & 7u);
+                    s.entry = __ldg(refs + (keys[0] & 7u));
                     return false;
                 }
             }
@@ -730,18 +719,23 @@ __device__ __forceinline__ uint32_t scene_of(const WfParams& P, uint32_t v) {
 // take their next rays from that chunk, so the rays one warp works on stay
 // neighbours in the list (the shadow rays of neighbouring pixels, which meet
 // the same instances).  The chunk is RT_FETCH_CHUNK entries, less for short
-// lists (at least 32, and about 8 chunks per resident warp), so a small frame
+// lists (about 8 chunks per resident warp, at least one round of rays_per_warp), so a small frame
 // still spreads over every warp.  Measured on the 64-scene batch: shadow
 // launch 11.65 -> 10.38 ms with chunks of 128 (512: 10.85); the closest-hit
 // lists keep the whole-list counter (chunks made them 6 % slower).
 #ifndef RT_FETCH_CHUNK
 #define RT_FETCH_CHUNK 128
 #endif
-// Packet traversal: each node is staged through shared memory by the
-// sub-packet (1) or read by every lane from global memory (0).
-#ifndef RT_PACKET_STAGE
-#define RT_PACKET_STAGE 0
-#endif
+
+// Rays that a warp of a persistent launch works on at a time: all its lanes,
+// or fewer when the list is shorter than the lanes of the grid, so that it
+// spreads over every warp.  A ray is bound by the latency of its own steps,
+// and a warp with fewer rays has fewer different steps to run in each
+// iteration (1,024 rays of a ray buffer: 47 -> 34 us at one ray per warp).
+__device__ __forceinline__ uint32_t rays_per_warp(uint32_t total) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    return min(32u, max(1u, (total + warps - 1u) / warps));
+}
 
 struct WarpChunk {
     uint32_t next = 0, end = 0;  // the same in every lane of the warp
@@ -749,7 +743,7 @@ struct WarpChunk {
     bool exhausted = false;
     __device__ explicit WarpChunk(uint32_t total) {
         const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-        size = min((uint32_t)RT_FETCH_CHUNK, max(32u, total / (8u * warps)));
+        size = min((uint32_t)RT_FETCH_CHUNK, max(rays_per_warp(total), total / (8u * warps)));
     }
 };
 // All 32 lanes call it, converged.  Returns the list entry of a lane that
@@ -947,6 +941,8 @@ __device__ __forceinline__ void trace_wavefront(const WfParams& P) {
     uint32_t t0 = 0;  // clock() at the ray's start (heatmap only)
     uint32_t depth = 0;  // bits 0-7: depth of the ray being traced; 8-15: depth the slot started at
     WarpChunk chunk(total);
+    // (any-hit lists were 3 % slower so: frame of 256x256)
+    if (MODE == kModeBounce && (threadIdx.x & 31u) >= rays_per_warp(total)) return;
     for (;;) {
         uint32_t my;
         if (MODE == kModeShadow && RT_FETCH_CHUNK) {
@@ -1050,8 +1046,8 @@ __global__ void __launch_bounds__(BLOCK, trace_warps_per_sm(KINDS) * 32 / BLOCK)
 // Traverses the sub-packet `act` (the calling lanes, converged, one scene,
 // each at the TLAS root).  ws: the warp's stack (kStackSize entries).
 template <bool STATS, uint32_t KINDS>
-__device__ __forceinline__ void packet_traverse(Trav& s, uint2* ws, float4* nb, const unsigned act,
-                                                const SceneTable& sv, const RtShaderBindingTable* sbt,
+__device__ __forceinline__ void packet_traverse(Trav& s, uint2* ws, const unsigned act, const SceneTable& sv,
+                                                const RtShaderBindingTable* sbt,
                                                 uint32_t* status, uint32_t ray_flags, uint32_t ray_sbt_offset,
                                                 Counters& cnt) {
     const bool any_hit = (ray_flags & RT_RAY_FLAG_TERMINATE_ON_FIRST_HIT) != 0u;
@@ -1073,30 +1069,14 @@ __device__ __forceinline__ void packet_traverse(Trav& s, uint2* ws, float4* nb, 
                 if (leader) atomicOr(status, 1u << RT_ERR_BAD_AS);
             } else {
                 if (STATS) cnt.nodes++;
-                uint32_t keys[8], refs[8];
+                uint32_t keys[8];
+                const uint32_t* refs;  // the node's child references
                 const bool qn = (KINDS & kBlasKindQ8) && s.in_blas && (KINDS == kBlasKindQ8 || s.quant);
-                if (RT_PACKET_STAGE) {
-                    // the sub-packet's lanes copy the node into the warp's buffer with one
-                    // 16-byte load each, then every lane reads its planes from there
-                    const float4* src = qn ? reinterpret_cast<const float4*>(reinterpret_cast<const uint8_t*>(s.nodes) +
-                                                                             (size_t)entry * kQNodeBytes)
-                                           : reinterpret_cast<const float4*>(s.nodes + entry);
-                    const uint32_t n16 = qn ? kQNodeBytes / 16u : kNodeBytes / 16u;
-                    const uint32_t r = (uint32_t)__popc(act & lanemask_lt()), na = (uint32_t)__popc(act);
-                    __syncwarp(act);  // every lane has read the previous node
-                    for (uint32_t q = r; q < n16; q += na) nb[q] = __ldg(src + q);
-                    __syncwarp(act);
-                    if (qn) {
-                        if (STATS) cnt.qnodes++;
-                        qnode_keys_at<false>(s, reinterpret_cast<const uint8_t*>(nb), keys, refs);
-                    } else {
-                        fnode_keys_at<false>(s, nb, keys, refs);
-                    }
-                } else if (qn) {
+                if (qn) {
                     if (STATS) cnt.qnodes++;
-                    qnode_keys(s, entry, keys, refs);
+                    refs = qnode_keys(s, entry, keys);
                 } else {
-                    fnode_keys(s, entry, keys, refs);
+                    refs = fnode_keys(s, entry, keys);
                 }
                 // the nearest lane's key of each child; every lane has read its
                 // last popped entry before this point, so the pushes below
@@ -1108,12 +1088,12 @@ __device__ __forceinline__ void packet_traverse(Trav& s, uint2* ws, float4* nb, 
 #pragma unroll
                     for (int k = 0; k < 8; k++) mask |= (keys[k] != 0xFFFFFFFFu ? 1u : 0u) << k;
                     if (mask) {
-                        entry = pick8(refs, (uint32_t)(__ffs(mask) - 1));
+                        entry = __ldg(refs + (__ffs(mask) - 1));
                         mask &= mask - 1u;
                         while (mask) {
                             const uint32_t k = (uint32_t)(__ffs(mask) - 1);
                             mask &= mask - 1u;
-                            if (sp < (int)kStackSize) ws[sp++] = make_uint2(pick8(refs, k), 0u);
+                            if (sp < (int)kStackSize) ws[sp++] = make_uint2(__ldg(refs + k), 0u);
                             else if (leader) atomicOr(status, 1u << RT_ERR_STACK_OVERFLOW);
                         }
                         pop = false;
@@ -1125,10 +1105,10 @@ __device__ __forceinline__ void packet_traverse(Trav& s, uint2* ws, float4* nb, 
                         for (int q = 7; q >= 1; q--) {
                             const uint32_t key = keys[q];
                             if (key == 0xFFFFFFFFu) continue;
-                            if (sp < (int)kStackSize) ws[sp++] = make_uint2(pick8(refs, key & 7u), key & ~7u);
+                            if (sp < (int)kStackSize) ws[sp++] = make_uint2(__ldg(refs + (key & 7u)), key & ~7u);
                             else if (leader) atomicOr(status, 1u << RT_ERR_STACK_OVERFLOW);
                         }
-                        entry = pick8(refs, keys[0] & 7u);
+                        entry = __ldg(refs + (keys[0] & 7u));
                         pop = false;
                     }
                 }
@@ -1195,7 +1175,6 @@ __device__ __forceinline__ void packet_traverse(Trav& s, uint2* ws, float4* nb, 
 template <int MODE, bool STATS, uint32_t KINDS, int BLOCK, bool LANE_BOUNCES>
 __device__ __forceinline__ void trace_packets(const WfParams& P) {
     __shared__ uint2 stacks[BLOCK / 32][kStackSize];
-    __shared__ float4 nbuf[BLOCK / 32][RT_PACKET_STAGE ? kNodeBytes / 16 : 1];  // staged node per warp
     uint2* ws = stacks[threadIdx.x >> 5];
     const SceneTable sv{P.B.scenes};
     const uint32_t lane = threadIdx.x & 31u;
@@ -1252,8 +1231,7 @@ __device__ __forceinline__ void trace_packets(const WfParams& P) {
             pending &= ~act;
             bool cont = false;
             if ((act >> lane) & 1u) {
-                packet_traverse<STATS, KINDS>(s, ws, nbuf[threadIdx.x >> 5], act, sv, &P.sbt, P.status, ray_flags,
-                                              sbt_offset, cnt);
+                packet_traverse<STATS, KINDS>(s, ws, act, sv, &P.sbt, P.status, ray_flags, sbt_offset, cnt);
                 if (MODE == kModeBounce && LANE_BOUNCES) {
                     // every further bounce of the lane's ray, traced by the lane
                     // alone (the closest-hit program's arithmetic, bit for bit)
@@ -1497,6 +1475,7 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->traversals), (unsigned long long)L.count);
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->primary_rays), (unsigned long long)L.count);
     }
+    if ((threadIdx.x & 31u) >= rays_per_warp(L.count)) return;
     for (;;) {
         uint32_t my = warp_append(L.work, item == kNoItem);
         if (item == kNoItem) {
