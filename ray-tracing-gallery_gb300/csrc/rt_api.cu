@@ -25,7 +25,7 @@ constexpr uint32_t kWorkSlots = 256;
 
 struct CtxDevice {
     RtStats stats;
-    uint32_t work[kWorkSlots];
+    uint32_t work[kWorkSlots], done[kWorkSlots];  // ray-buffer launches (zero between them)
 };
 
 thread_local std::string g_last_error;
@@ -797,7 +797,9 @@ RTCORE_API int32_t rt_cmd_trace_ray_buffer(rt_ctx* ctx, uint64_t tlas, const RtP
     p.collect_stats = (ray_flags & RT_RAY_FLAG_EXT_COLLECT_STATS) ? 1u : 0u;
     p.stats = &ctx->dev->stats;
     p.status = &ctx->dev->stats.status;
-    p.work = &ctx->dev->work[ctx->work_slot.fetch_add(1) % kWorkSlots];
+    const uint32_t slot = ctx->work_slot.fetch_add(1) % kWorkSlots;
+    p.work = &ctx->dev->work[slot];
+    p.done = &ctx->dev->done[slot];
     p.kinds_built = blas_kinds_built();
     cudaError_t e = launch_trace_ray_buffer(p, ctx->num_sms, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "rt_cmd_trace_ray_buffer");

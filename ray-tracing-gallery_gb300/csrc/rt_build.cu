@@ -175,7 +175,9 @@ __device__ __forceinline__ void init_state(BuildState* st, uint32_t n) {
         }
     }
 }
-__global__ void k_init_state(BuildState* st, uint32_t n) { init_state(st, n); }
+__global__ void k_init_state(BuildState* st, uint32_t n) {
+    after_previous();
+    init_state(st, n); }
 
 __device__ __forceinline__ int find_geometry(const BlasInput& in, uint32_t i) {
     int lo = 0, hi = (int)in.geometry_count - 1;
@@ -222,18 +224,21 @@ __device__ bool fetch_triangle(const BlasInput& in, uint32_t i, int* geom, uint3
 }
 
 // What a later kernel of the build finds zeroed: the PLOC look-back
-// descriptors and the collapse's tasks.
+// descriptors, the collapse's tasks, and the state of a onesweep sort.
 struct ZeroedWords {
     unsigned long long* desc;
     unsigned long long* tasks;
-    uint32_t descs, task_count;
+    unsigned long long* sort;
+    uint32_t descs, task_count, sort_words;
 };
 __device__ __forceinline__ void zero_words(const ZeroedWords& z, uint32_t i, uint32_t stride) {
+    for (uint32_t k = i; k < z.sort_words; k += stride) z.sort[k] = 0ull;
     for (uint32_t k = i; k < z.descs; k += stride) z.desc[k] = 0ull;
     for (uint32_t k = i; k < z.task_count; k += stride) z.tasks[k] = 0ull;
 }
 
 __global__ void k_blas_prims(const __grid_constant__ BlasInput in, float4* boxes, BuildState* st, ZeroedWords z) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     zero_words(z, i, gridDim.x * blockDim.x);
     float cmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
@@ -409,6 +414,7 @@ __device__ __forceinline__ void tlas_prim(const RtAccelerationStructureInstance*
 
 __global__ void k_tlas_prims(const RtAccelerationStructureInstance* inst, uint32_t n, float4* boxes,
                              InstRecord* temp, BuildState* st, ZeroedWords z) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     zero_words(z, i, gridDim.x * blockDim.x);
     float4 lo, hi;
@@ -529,6 +535,7 @@ __device__ __forceinline__ void block_sort(uint32_t (&key)[ITEMS], uint32_t (&va
 template <bool MORTON, int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_sort_block(uint32_t* k, uint32_t* v, uint32_t n, const float4* boxes,
                                                              const BuildState* st) {
+    after_previous();
     extern __shared__ uint32_t sort_smem[];
     __shared__ uint32_t warp_sums[kSortThreads / 32];
     const uint32_t first = (threadIdx.x >> 5) * ITEMS * 32u + (threadIdx.x & 31u);  // item r of this thread: first + 32 r
@@ -600,6 +607,7 @@ template <bool MORTON>
 __global__ void __launch_bounds__(kOsThreads) k_onesweep_hist(uint32_t* keys, uint32_t* vals, uint32_t n,
                                                               OnesweepState* os, const float4* boxes,
                                                               const BuildState* st) {
+    after_previous();
     __shared__ uint32_t h[4][256];
     for (int i = threadIdx.x; i < 1024; i += blockDim.x) (&h[0][0])[i] = 0;
     __syncthreads();
@@ -656,6 +664,7 @@ __global__ void __launch_bounds__(kOsThreads, 3) k_onesweep_pass(const uint32_t*
                                                                uint32_t* kout, uint32_t* vout, uint32_t n, int pass,
                                                                OnesweepState* os, uint32_t* desc,
                                                                uint32_t* error) {
+    after_previous();
     __shared__ OnesweepShared sm;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const int shift = pass * 8;
@@ -769,7 +778,7 @@ cudaError_t launch_sort_block(uint32_t* k, uint32_t* v, uint32_t n, const float4
     const cudaError_t e =
         cudaFuncSetAttribute(k_sort_block<MORTON, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    note_launch(), k_sort_block<MORTON, ITEMS><<<1, kSortThreads, smem, stream>>>(k, v, n, boxes, st);
+    launch(k_sort_block<MORTON, ITEMS>, 1, kSortThreads, smem, stream, k, v, n, boxes, st);
     return cudaGetLastError();
 }
 
@@ -784,17 +793,17 @@ cudaError_t launch_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, 
     OnesweepState* os = reinterpret_cast<OnesweepState*>(state);
     uint32_t* desc = reinterpret_cast<uint32_t*>(state + sizeof(OnesweepState));
     const uint32_t parts = onesweep_partitions(n);
-    cudaError_t e = cudaMemsetAsync(state, 0, key_sort_state_bytes(n), stream);
-    if (e != cudaSuccess) return e;
-    note_launch(), k_onesweep_hist<MORTON><<<std::min<uint32_t>((n + kOsThreads - 1) / kOsThreads, kOsHistBlocks),
-                                             kOsThreads, 0, stream>>>(k0, v0, n, os, boxes, st);
+    if (!MORTON) {  // a build's first kernel has zeroed it
+        const cudaError_t e = cudaMemsetAsync(state, 0, key_sort_state_bytes(n), stream);
+        if (e != cudaSuccess) return e;
+    }
+    launch(k_onesweep_hist<MORTON>, std::min<uint32_t>((n + kOsThreads - 1) / kOsThreads, kOsHistBlocks), kOsThreads, 0, stream, k0, v0, n, os, boxes, st);
     uint32_t* kin = k0;
     uint32_t* vin = v0;
     uint32_t* kout = k1;
     uint32_t* vout = v1;
     for (int pass = 0; pass < 4; pass++) {
-        note_launch(), k_onesweep_pass<<<parts, kOsThreads, 0, stream>>>(kin, vin, kout, vout, n, pass, os,
-                                                                          desc + (size_t)pass * parts * 256u, error);
+        launch(k_onesweep_pass, parts, kOsThreads, 0, stream, kin, vin, kout, vout, n, pass, os, desc + (size_t)pass * parts * 256u, error);
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
@@ -811,6 +820,7 @@ cudaError_t launch_key_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* 
 namespace {
 
 __global__ void k_gather_boxes(const float4* boxes, const uint32_t* vals, uint32_t n, float4* sboxes) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t p = vals[i];
@@ -827,11 +837,13 @@ __device__ __forceinline__ int kdelta(const uint32_t* k, int n, int i, int j) {
 }
 
 __global__ void k_karras(const uint32_t* keys, uint32_t n_u, uint4* inodes, uint32_t* iparent, uint32_t* lparent,
-                         ZeroedWords z) {
+                         uint32_t* flags, ZeroedWords z) {
+    after_previous();
     int n = (int)n_u;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     zero_words(z, (uint32_t)i, gridDim.x * blockDim.x);
     if (i >= n - 1) return;
+    flags[i] = 0;  // arrivals at the node, for k_bottom_up
     int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = kdelta(keys, n, i, i - d);
     int lmax = 2;
@@ -867,6 +879,7 @@ __device__ __forceinline__ void load_box_cg(const float4* b, size_t i, float lo[
 
 __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const uint32_t* iparent,
                             const float4* sboxes, float4* iboxes, uint32_t* flags, uint32_t n, uint32_t* err) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t p = lparent[i];
@@ -1035,6 +1048,7 @@ __device__ __forceinline__ uint32_t ploc_take(const uint32_t* nbr, const float* 
 // shared-memory and arithmetic issue for large counts, latency for small.
 // The first round gathers the Morton-ordered primitive boxes itself.
 __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_constant__ PlocArgs a, int round) {
+    after_previous();
     BuildState* st = a.st;
     const uint32_t word = st->ploc_round[round], count = word & kPlocCount;
     if (count <= kPlocSmall) {
@@ -1353,6 +1367,7 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
     return merges;
 }
 __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant__ PlocArgs a, int round) {
+    after_previous();
     extern __shared__ float4 ploc_smem[];
     PlocTailShared& s = *reinterpret_cast<PlocTailShared*>(ploc_smem);
     BuildState* st = a.st;
@@ -1677,6 +1692,7 @@ __device__ __forceinline__ void collapse_loop(const CollapseCtx& c) {
 }
 
 __global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_constant__ CollapseCtx c) {
+    after_previous();
     if (c.n > c.leaf_max) collapse_loop<false>(c);
     else if (blockIdx.x == 0 && threadIdx.x == 0) write_single_leaf(c);
 }
@@ -1684,6 +1700,7 @@ __global__ void __launch_bounds__(kCollapseThreads, 8) k_collapse(const __grid_c
 // ---- primitive records ----------------------------------------------------------
 __global__ void k_write_tris(const __grid_constant__ BlasInput in, const uint32_t* vals, const uint32_t* perm,
                              TriRecord* tris, BuildState* st) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool here = i < in.n;  // every thread takes part in the block's reductions below
     uint32_t p = here ? vals[min(perm[i], in.n - 1u)] : 0u;
@@ -1761,6 +1778,7 @@ __global__ void k_write_tris(const __grid_constant__ BlasInput in, const uint32_
 
 __global__ void k_write_insts(const InstRecord* temp, const uint32_t* vals, const uint32_t* perm, uint32_t n,
                               InstRecord* out) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = temp[vals[min(perm[i], n - 1u)]];
@@ -1792,6 +1810,7 @@ __device__ uint32_t quantum_exponent(float L, float ext, uint32_t e_floor) {
 }
 
 __global__ void k_quantize_nodes(const WideNode* in, const BuildState* st, uint32_t max_nodes, QNode* out) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t count = min(st->node_count, max_nodes);
     if (i >= count) return;
@@ -1939,6 +1958,7 @@ constexpr int kFinishThreads = 384;
 static_assert(kFinishThreads >= kDopTriples, "one thread per triple");
 __global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const BuildState* st,
                                                            const __grid_constant__ HeaderStatic hs) {
+    after_previous();
     __shared__ float phf[14];
     __shared__ uint16_t list[kDopTriples];   // triples that pass the float screen, in order
     __shared__ double cand[kDopTriples][3];  // the points found, by place in the list
@@ -2108,6 +2128,7 @@ struct TlasSmallShared {
 };
 __global__ void __launch_bounds__(kTlasSmall) k_tlas_small(const __grid_constant__ TlasSmallArgs a,
                                                            const __grid_constant__ HeaderStatic hs) {
+    after_previous();
     extern __shared__ float4 tlas_smem[];
     TlasSmallShared& s = *reinterpret_cast<TlasSmallShared*>(tlas_smem);
     const uint32_t tid = threadIdx.x, n = a.n;
@@ -2168,6 +2189,7 @@ __global__ void __launch_bounds__(kTlasSmall) k_tlas_small(const __grid_constant
 // ---- TLAS refit ---------------------------------------------------------------------
 __global__ void k_refit_insts(const RtAccelerationStructureInstance* inst, uint32_t n, AsHeader* h,
                               float4* sboxes, uint32_t* err) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     InstRecord* recs = reinterpret_cast<InstRecord*>(reinterpret_cast<uint8_t*>(h) + h->prims_offset);
@@ -2191,6 +2213,114 @@ __global__ void k_refit_insts(const RtAccelerationStructureInstance* inst, uint3
     sboxes[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
 }
 
+// Refit of a TLAS of up to 512 instances in one block: the records, then the
+// nodes from the leaves up, eight lanes (one per child) to a node, with the
+// instance boxes, the node boxes and the arrival counts in shared memory.  A
+// node is done by the group that brings the last of its internal children.
+// (105 instances: 48 us as a memset and three launches, 12 us now; bound
+// by the latency of the instance transforms and of about four levels.)
+constexpr uint32_t kRefitSmall = 512;
+constexpr uint32_t kRefitNodes = kRefitSmall + 2;  // max_wide_nodes(n, 4)
+__global__ void __launch_bounds__(kRefitSmall) k_refit_small(const RtAccelerationStructureInstance* inst, uint32_t n,
+                                                             AsHeader* h) {
+    __shared__ float4 ibox[2 * kRefitSmall];
+    __shared__ float nbox[kRefitNodes][6];
+    __shared__ uint32_t arrived[kRefitNodes];
+    __shared__ uint32_t err, kinds_seen;
+    const uint32_t tid = threadIdx.x, sub = tid & 7u, group = tid & 24u;
+    const unsigned gmask = 0xFFu << group;
+    const uint32_t count = h->node_count, prims = h->prim_count;
+    if (tid == 0) err = kinds_seen = 0u;
+    for (uint32_t i = tid; i < kRefitNodes; i += kRefitSmall) arrived[i] = 0u;
+    __syncthreads();
+    uint8_t* base = reinterpret_cast<uint8_t*>(h);
+    WideNode* nodes = reinterpret_cast<WideNode*>(base + h->nodes_offset);
+    const uint32_t* parents = reinterpret_cast<const uint32_t*>(base + h->parents_offset);
+    if (tid < n) {
+        InstRecord* recs = reinterpret_cast<InstRecord*>(base + h->prims_offset);
+        InstRecord rec;
+        const uint32_t id = recs[tid].instance_id;
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        if (id < n) {
+            const RtAccelerationStructureInstance r = inst[id];
+            if (fill_instance(r, id, &rec, lo, hi, &err)) atomicOr(&kinds_seen, blas_kind(rec.node_count));
+        } else {
+            rec = recs[tid];
+            rec.tri_count = 0;
+            atomicOr(&err, 1u << RT_ERR_INVALID);
+        }
+        recs[tid] = rec;
+        ibox[2 * tid] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+        ibox[2 * tid + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+    }
+    __syncthreads();
+    if (count > min(n + 2u, kRefitNodes)) {  // a TLAS of more instances than this update was given
+        if (tid == 0) atomicOr(&err, 1u << RT_ERR_INVALID);
+    } else {
+        for (uint32_t first = tid >> 3; first < count; first += kRefitSmall / 8u) {
+            uint32_t slot = first;
+            bool leaf_node = true;  // climbs start at the nodes without internal children
+            for (int guard = 0; guard < 64; guard++) {
+                WideNode* nd = &nodes[slot];
+                const uint32_t m = node_meta(nd->meta[0], nd->meta[1], (int)sub);
+                const bool inner = m == kMetaInternal;
+                if (leaf_node && __any_sync(gmask, inner)) break;
+                leaf_node = false;
+                uint32_t r = nd->child_ref[sub];
+                if (m != 0u && !inner) r &= 0x0FFFFFFFu;  // leaf: first primitive
+                float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                if (m != 0u) {
+                    if (inner ? r >= count : (m > 8u || r + m > prims || r + m > n)) {
+                        atomicOr(&err, 1u << RT_ERR_BAD_AS);  // malformed child: leave its box empty
+                    } else if (inner) {
+                        for (int k = 0; k < 6; k++) b[k] = *const_cast<volatile float*>(&nbox[r][k]);
+                    } else {
+                        for (uint32_t q = 0; q < m; q++) {
+                            const float4 l = ibox[2 * (r + q)], u = ibox[2 * (r + q) + 1];
+                            b[0] = fminf(b[0], l.x); b[1] = fminf(b[1], l.y); b[2] = fminf(b[2], l.z);
+                            b[3] = fmaxf(b[3], u.x); b[4] = fmaxf(b[4], u.y); b[5] = fmaxf(b[5], u.z);
+                        }
+                    }
+                    nd->lox[sub] = b[0]; nd->loy[sub] = b[1]; nd->loz[sub] = b[2];
+                    nd->hix[sub] = b[3]; nd->hiy[sub] = b[4]; nd->hiz[sub] = b[5];
+                }
+                for (int off = 1; off < 8; off <<= 1)
+                    for (int k = 0; k < 6; k++) {
+                        const float o = __shfl_xor_sync(gmask, b[k], off);
+                        b[k] = k < 3 ? fminf(b[k], o) : fmaxf(b[k], o);
+                    }
+                const uint32_t p = parents[slot];
+                const bool root = p == kNone || p >= count;
+                uint32_t last = 0;
+                if (sub == 0u) {
+                    if (root) {
+                        for (int k = 0; k < 3; k++) {
+                            h->bounds_lo[k] = b[k];
+                            h->bounds_hi[k] = b[3 + k];
+                        }
+                    } else {
+                        for (int k = 0; k < 6; k++) *const_cast<volatile float*>(&nbox[slot][k]) = b[k];
+                        __threadfence_block();
+                        uint32_t need = 0;
+                        for (int k = 0; k < 8; k++) need += node_meta(nodes[p].meta[0], nodes[p].meta[1], k) == kMetaInternal;
+                        last = atomicAdd(&arrived[p], 1u) + 1u >= need ? 1u : 0u;
+                        __threadfence_block();
+                    }
+                }
+                last = __shfl_sync(gmask, last, (int)group);
+                if (root || !last) break;
+                slot = p;
+                if (guard == 63 && sub == 0u) atomicOr(&err, 1u << RT_ERR_STACK_OVERFLOW);
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        if (kinds_seen) h->blas_kinds |= kinds_seen;  // a refit may add a BLAS kind, never drop one
+        if (err >> 1) h->status = (uint32_t)__ffs(err >> 1);  // the lowest RT_ERR_* bit
+    }
+}
+
 __device__ __forceinline__ int internal_children(const WideNode* nd) {
     uint32_t m0 = __ldcg(&nd->meta[0]), m1 = __ldcg(&nd->meta[1]);
     int c = 0;
@@ -2199,6 +2329,7 @@ __device__ __forceinline__ int internal_children(const WideNode* nd) {
 }
 
 __global__ void k_refit_nodes(AsHeader* h, const float4* sboxes, uint32_t* counters, uint32_t cap, uint32_t* err) {
+    after_previous();
     uint32_t count = h->node_count;
     uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (count > cap) {  // a TLAS of more instances than this update was given
@@ -2273,6 +2404,7 @@ __global__ void k_refit_nodes(AsHeader* h, const float4* sboxes, uint32_t* count
 }
 
 __global__ void k_refit_status(AsHeader* h, const uint32_t* err) {
+    after_previous();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     uint32_t e = *err;
     for (uint32_t b = 1; b < 32; b++)
@@ -2284,6 +2416,7 @@ __global__ void k_refit_status(AsHeader* h, const uint32_t* err) {
 
 // ---- AS copy (CLONE / COMPACT) ------------------------------------------------------
 __global__ void k_as_copy(const uint8_t* src, uint8_t* dst, uint64_t dst_size, uint32_t mode) {
+    after_previous();
     const AsHeader* h = reinterpret_cast<const AsHeader*>(src);
     if (h->magic != kAsMagic) {
         if (blockIdx.x == 0 && threadIdx.x == 0 && dst_size >= kHeaderBytes)
@@ -2470,8 +2603,10 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     unsigned long long* tasks = reinterpret_cast<unsigned long long*>(sl.ploc ? scratch + sl.iparent : scratch + sl.boxes);
     const uint32_t task_count = n > (top ? kTlasLeafMax : kBlasLeafMax) ? al.max_nodes : 0u;
     const ZeroedWords zero_ploc = {reinterpret_cast<unsigned long long*>(scratch + sl.ploc_nn), tasks,
-                                   sl.ploc ? blocks_for(n, kPlocTile) : 0u, sl.ploc ? task_count : 0u};
-    const ZeroedWords zero_karras = {nullptr, tasks, 0u, task_count};
+                                   reinterpret_cast<unsigned long long*>(hist), sl.ploc ? blocks_for(n, kPlocTile) : 0u,
+                                   sl.ploc ? task_count : 0u,
+                                   n > kSortBlockMax ? (uint32_t)(key_sort_state_bytes(n) / 8u) : 0u};
+    const ZeroedWords zero_karras = {nullptr, tasks, nullptr, 0u, task_count, 0u};
 
     HeaderStatic hs;
     hs.node_bytes = al.node_bytes;
@@ -2502,13 +2637,13 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         ta.n = n;
         ta.width = node_width(build_flags);
         ta.max_nodes = al.max_nodes;
-        note_launch(), k_tlas_small<<<1, kTlasSmall, sizeof(TlasSmallShared), stream>>>(ta, hs);
+        launch(k_tlas_small, 1, kTlasSmall, sizeof(TlasSmallShared), stream, ta, hs);
         return cudaGetLastError();
     }
-    note_launch(), k_init_state<<<1, 32, 0, stream>>>(st, n);
+    launch(k_init_state, 1, 32, 0, stream, st, n);
     if (n > 0) {
-        if (top) note_launch(), k_tlas_prims<<<blocks_for(n, T), T, 0, stream>>>(inst, n, boxes, temp, st, zero_ploc);
-        else note_launch(), k_blas_prims<<<blocks_for(n, T), T, 0, stream>>>(*blas, boxes, st, zero_ploc);
+        if (top) launch(k_tlas_prims, blocks_for(n, T), T, 0, stream, inst, n, boxes, temp, st, zero_ploc);
+        else launch(k_blas_prims, blocks_for(n, T), T, 0, stream, *blas, boxes, st, zero_ploc);
         // Morton codes and their stable order: the sorted pairs land in keys[0] / vals[0]
         const int cur = 0;
         if (cudaError_t e = launch_sort<true>(keys[0], vals[0], keys[1], vals[1], n, reinterpret_cast<uint8_t*>(hist),
@@ -2529,22 +2664,19 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
             pa.n = n;
             const int rounds = ploc_grid_rounds(n);
             for (int r = 0; r < rounds; r++)
-                note_launch(), k_ploc_round<<<ploc_round_blocks(n, r), kPlocThreads, 0, stream>>>(pa, r);
+                launch(k_ploc_round, ploc_round_blocks(n, r), kPlocThreads, 0, stream, pa, r);
             // a per-device attribute: set on every build (a host-side call, no device work)
             const cudaError_t smem_ok =
                 cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(PlocTailShared));
             if (smem_ok != cudaSuccess) return smem_ok;
-            note_launch(), k_ploc_tail<<<1, kPlocSmall, sizeof(PlocTailShared), stream>>>(pa, rounds);
+            launch(k_ploc_tail, 1, kPlocSmall, sizeof(PlocTailShared), stream, pa, rounds);
         } else {
-            note_launch(), k_gather_boxes<<<blocks_for(n, T), T, 0, stream>>>(boxes, vals[cur], n, sboxes);
+            launch(k_gather_boxes, blocks_for(n, T), T, 0, stream, boxes, vals[cur], n, sboxes);
         }
         if (!sl.ploc && n > 1) {
-            note_launch(), k_karras<<<blocks_for(n - 1, T), T, 0, stream>>>(keys[cur], n, inodes, iparent, lparent,
-                                                                             zero_karras);
-            cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, stream);
-            note_launch(), k_bottom_up<<<blocks_for(n, T), T, 0, stream>>>(inodes, lparent, iparent, sboxes, iboxes,
-                                                                             flags, n, &st->error);
+            launch(k_karras, blocks_for(n - 1, T), T, 0, stream, keys[cur], n, inodes, iparent, lparent, flags, zero_karras);
+            launch(k_bottom_up, blocks_for(n, T), T, 0, stream, inodes, lparent, iparent, sboxes, iboxes, flags, n, &st->error);
         }
         uint32_t* perm = reinterpret_cast<uint32_t*>(scratch + sl.perm);
         CollapseCtx cc;
@@ -2562,14 +2694,11 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         cc.n = n;
         // a group of 8 lanes per possible wide node, up to a full load of the SMs
         const uint32_t g = std::min<uint32_t>(blocks_for(al.max_nodes, kCollapseThreads / 8), kCollapseBlocks);
-        note_launch(), k_collapse<<<g, kCollapseThreads, 0, stream>>>(cc);
+        launch(k_collapse, g, kCollapseThreads, 0, stream, cc);
         if (top) {
-            note_launch(), k_write_insts<<<blocks_for(n, T), T, 0, stream>>>(temp, vals[cur], perm, n,
-                                                              reinterpret_cast<InstRecord*>(dst + al.prims));
+            launch(k_write_insts, blocks_for(n, T), T, 0, stream, temp, vals[cur], perm, n, reinterpret_cast<InstRecord*>(dst + al.prims));
         } else {
-            note_launch(), k_write_tris<<<blocks_for(n, T), T, 0, stream>>>(*blas, vals[cur], perm,
-                                                                             reinterpret_cast<TriRecord*>(dst + al.prims),
-                                                                             st);
+            launch(k_write_tris, blocks_for(n, T), T, 0, stream, *blas, vals[cur], perm, reinterpret_cast<TriRecord*>(dst + al.prims), st);
         }
     } else {
         CollapseCtx cc{};
@@ -2580,14 +2709,13 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
         cc.width = node_width(build_flags);
         cc.max_nodes = al.max_nodes;
         cc.n = n;
-        note_launch(), k_collapse<<<1, kCollapseThreads, 0, stream>>>(cc);
+        launch(k_collapse, 1, kCollapseThreads, 0, stream, cc);
     }
     if (quantized) {
         uint32_t g = blocks_for(al.max_nodes, 128);
-        note_launch(), k_quantize_nodes<<<g, 128, 0, stream>>>(fp32_nodes, st, al.max_nodes,
-                                                               reinterpret_cast<QNode*>(dst + al.nodes));
+        launch(k_quantize_nodes, g, 128, 0, stream, fp32_nodes, st, al.max_nodes, reinterpret_cast<QNode*>(dst + al.nodes));
     }
-    note_launch(), k_finish<<<1, kFinishThreads, 0, stream>>>(reinterpret_cast<AsHeader*>(dst), st, hs);
+    launch(k_finish, 1, kFinishThreads, 0, stream, reinterpret_cast<AsHeader*>(dst), st, hs);
     return cudaGetLastError();
 }
 
@@ -2604,7 +2732,7 @@ cudaError_t launch_tlas_build(const RtAccelerationStructureInstance* instances, 
 }
 
 cudaError_t launch_as_copy(const uint8_t* src, uint8_t* dst, uint64_t dst_size, uint32_t mode, cudaStream_t stream) {
-    note_launch(), k_as_copy<<<1024, 256, 0, stream>>>(src, dst, dst_size, mode);
+    launch(k_as_copy, 1024, 256, 0, stream, src, dst, dst_size, mode);
     return cudaGetLastError();
 }
 
@@ -2614,7 +2742,11 @@ cudaError_t launch_tlas_update(const RtAccelerationStructureInstance* instances,
     // node capacity of either node width: the grid and the counters cover any TLAS of n instances
     const uint32_t cap = (uint32_t)max_wide_nodes(n, 4);
     if (src != dst) {
-        note_launch(), k_as_copy<<<1024, 256, 0, stream>>>(src, dst, dst_size, RT_COPY_MODE_CLONE);
+        launch(k_as_copy, 1024, 256, 0, stream, src, dst, dst_size, RT_COPY_MODE_CLONE);
+    }
+    if (n > 0 && n <= kRefitSmall) {
+        launch(k_refit_small, 1, kRefitSmall, 0, stream, instances, n, reinterpret_cast<AsHeader*>(dst));
+        return cudaGetLastError();
     }
     float4* sboxes = reinterpret_cast<float4*>(scratch);
     uint32_t* counters = reinterpret_cast<uint32_t*>(scratch + sl.refit_counters);
@@ -2622,9 +2754,9 @@ cudaError_t launch_tlas_update(const RtAccelerationStructureInstance* instances,
     uint32_t* err = counters + cap;
     cudaMemsetAsync(counters, 0, (size_t)cap * 4 + 4, stream);
     AsHeader* h = reinterpret_cast<AsHeader*>(dst);
-    if (n > 0) note_launch(), k_refit_insts<<<blocks_for(n, 256), 256, 0, stream>>>(instances, n, h, sboxes, err);
-    note_launch(), k_refit_nodes<<<blocks_for(cap, 128), 128, 0, stream>>>(h, sboxes, counters, cap, err);
-    note_launch(), k_refit_status<<<1, 32, 0, stream>>>(h, err);
+    if (n > 0) launch(k_refit_insts, blocks_for(n, 256), 256, 0, stream, instances, n, h, sboxes, err);
+    launch(k_refit_nodes, blocks_for(cap, 128), 128, 0, stream, h, sboxes, counters, cap, err);
+    launch(k_refit_status, 1, 32, 0, stream, h, err);
     return cudaGetLastError();
 }
 

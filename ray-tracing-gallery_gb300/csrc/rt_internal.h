@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <utility>
 
 #include "rt_device.cuh"
 
@@ -10,6 +11,34 @@ namespace rt {
 
 // Counts every kernel this library launches (rt_kernel_launch_count).
 void note_launch();
+
+// Every kernel of the build and trace sequences begins with after_previous()
+// and is launched by launch(): it may become resident while the previous
+// kernel of its stream still runs, and waits there until that one has
+// completed and its writes are visible, so the launch latency of a short
+// kernel is hidden (programmatic dependent launch).  The next kernel may
+// become resident from then on; no block returns before the wait, so a kernel
+// that has completed implies that all before it have.
+__device__ __forceinline__ void after_previous() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
+template <class... Params, class... Args>
+void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    note_launch();
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = 1;
+    cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);  // an error stays for cudaGetLastError
+}
 
 // kBlasKind* bits of every BLAS node format this process has built.  A BLAS
 // blob only comes from a build here (or a copy of one), so a TLAS can only
@@ -142,7 +171,8 @@ struct RayBufferLaunch {
     uint32_t collect_stats;
     RtStats* stats;
     uint32_t* status;
-    uint32_t* work;            // device fetch counter for this launch (zeroed by the launcher)
+    uint32_t* work;            // device fetch counter for this launch, zero between launches
+    uint32_t* done;            // blocks that have finished, likewise
     uint32_t kinds_built;      // blas_kinds_built() when the launch was recorded
 };
 cudaError_t launch_trace_ray_buffer(const RayBufferLaunch& p, int num_sms, cudaStream_t stream);

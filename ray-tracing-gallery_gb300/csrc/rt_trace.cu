@@ -803,9 +803,14 @@ struct SetupParams {
 
 // Scene records of one chunk of the batch (TLAS header -> Env).
 __global__ void k_setup(const __grid_constant__ SetupParams P) {
+    after_previous();
     const uint32_t t = threadIdx.x;
-    if (P.copy_textures)
+    if (P.copy_textures) {  // the launch's first chunk: also zeroes its counters
         for (uint32_t i = t; i < RT_MAX_BOUND_IMAGES; i += blockDim.x) P.B.ctx_textures[i] = P.textures[i];
+        uint32_t* ctr = reinterpret_cast<uint32_t*>(P.B.ctr);
+        for (uint32_t i = t; i < sizeof(WfCounters) / 4; i += blockDim.x) ctr[i] = 0;
+        __syncthreads();
+    }
     if (t >= P.count) return;
     const TraceScene& d = P.d[t];
     SceneRec r;
@@ -835,6 +840,7 @@ __global__ void k_setup(const __grid_constant__ SetupParams P) {
 
 // ray_generation, lib.rs:126-142 (camera ray, fixed operation order)
 __global__ void k_raygen(const __grid_constant__ WfParams P) {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.total_slots) return;
     const uint32_t tile = i >> 5, l = i & 31u;
@@ -859,7 +865,10 @@ __global__ void k_raygen(const __grid_constant__ WfParams P) {
                     mat4_row(VI, 2, local.x, local.y, local.z, 0.0f));
         R[2 * (size_t)i] = make_float4(ro.x, ro.y, ro.z, 0.01f);
         R[2 * (size_t)i + 1] = make_float4(rd.x, rd.y, rd.z, 10000.0f);
-        P.B.ray_pixel[0][i] = S.pixel_begin + y * W + x;
+        const uint32_t p = S.pixel_begin + y * W + x;
+        P.B.ray_pixel[0][i] = p;
+        P.B.lit[p] = 0;
+        if (U.show_heatmap) P.B.heat[p] = 0;
     } else {
         R[2 * (size_t)i] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);  // tmin > tmax: never traversed
         R[2 * (size_t)i + 1] = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
@@ -1024,6 +1033,7 @@ __device__ __forceinline__ bool kinds_selected(uint32_t kinds_built, uint32_t tl
 template <int MODE, bool STATS, uint32_t KINDS, int SD, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, trace_warps_per_sm(KINDS) * 32 / BLOCK)
     k_trace(const __grid_constant__ WfParams P) {
+    after_previous();
     if (kinds_selected(P.kinds_built, P.B.ctr->kinds, KINDS)) trace_wavefront<MODE, STATS, KINDS, SD, BLOCK>(P);
 }
 
@@ -1302,6 +1312,7 @@ constexpr int packet_warps_per_sm(uint32_t kinds, int block) {
 template <int MODE, bool STATS, uint32_t KINDS, int BLOCK, bool LANE_BOUNCES>
 __global__ void __launch_bounds__(BLOCK, packet_warps_per_sm(KINDS, BLOCK) * 32 / BLOCK)
     k_trace_packet(const __grid_constant__ WfParams P) {
+    after_previous();
     if (kinds_selected(P.kinds_built, P.B.ctr->kinds, KINDS))
         trace_packets<MODE, STATS, KINDS, BLOCK, LANE_BOUNCES>(P);
 }
@@ -1316,6 +1327,7 @@ __global__ void __launch_bounds__(BLOCK, packet_warps_per_sm(KINDS, BLOCK) * 32 
 // dependent loads (instance -> model -> indices -> vertices -> textures);
 // 1080p frame 199 -> 170 us against the unconstrained 90 registers.
 __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ WfParams P) {
+    after_previous();
     const uint32_t b = P.bounce;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t p = kNoPixel, sc = 0, depth = 0, nshadow = 0;
@@ -1423,6 +1435,7 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ WfPara
 
 // sun_factor = lit / N; colour = brdf * sun_factor + ambient.
 __global__ void k_resolve(const __grid_constant__ WfParams P) {
+    after_previous();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.B.ctr->shade_count) return;
     const uint32_t p = P.B.shade_list[k];
@@ -1436,6 +1449,7 @@ __global__ void k_resolve(const __grid_constant__ WfParams P) {
 
 // Heatmap (lib.rs:174-186), linear_to_srgb and the RGBA8 image write.
 __global__ void k_output(const __grid_constant__ WfParams P) {
+    after_previous();
     const uint32_t gp = blockIdx.x * blockDim.x + threadIdx.x;
     if (gp >= P.total_pixels) return;
     if (gp == 0) {  // the shadow and bounce rays the shading launch appended
@@ -1475,8 +1489,8 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->traversals), (unsigned long long)L.count);
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->primary_rays), (unsigned long long)L.count);
     }
-    if ((threadIdx.x & 31u) >= rays_per_warp(L.count)) return;
-    for (;;) {
+    const bool spare = (threadIdx.x & 31u) >= rays_per_warp(L.count);
+    while (!spare) {
         uint32_t my = warp_append(L.work, item == kNoItem);
         if (item == kNoItem) {
             if (my >= L.count) break;
@@ -1519,11 +1533,20 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
 template <bool STATS, uint32_t KINDS>
 __global__ void __launch_bounds__(kTraceThreads, raybuf_warps_per_sm(KINDS) * 32 / kTraceThreads)
     k_trace_ray_buffer(const __grid_constant__ RayBufferParams P) {
+    after_previous();
     const Env e = make_env(P.L.tlas, P.L.push.model_info, P.L.textures, RT_MAX_BOUND_IMAGES, P.L.status);
-    if (kinds_selected(P.L.kinds_built, e.blas_kinds, KINDS)) trace_ray_buffer<STATS, KINDS>(P, e);
+    if (!kinds_selected(P.L.kinds_built, e.blas_kinds, KINDS)) return;
+    trace_ray_buffer<STATS, KINDS>(P, e);
+    // the last block to finish leaves the fetch counter at zero for its next launch
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(P.L.done, 1u) == gridDim.x - 1u) {
+        *P.L.work = 0u;
+        *P.L.done = 0u;
+    }
 }
 
 __global__ void k_debug_eval(uint32_t fn, const float* in, float* out, uint32_t count) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     switch (fn) {
@@ -1612,7 +1635,7 @@ void launch_trace_kernel(const WfParams& P, int num_sms, cudaStream_t stream) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         blocks = persistent_blocks(kern, BLOCK, num_sms, smem);
     }
-    note_launch(), kern<<<blocks, BLOCK, smem, stream>>>(P);
+    launch(kern, blocks, BLOCK, smem, stream, P);
 }
 
 template <int MODE, bool STATS, uint32_t KINDS, int BLOCK, bool LANE_BOUNCES = false>
@@ -1620,7 +1643,7 @@ void launch_packet_kernel(const WfParams& P, int num_sms, cudaStream_t stream) {
     const auto kern = k_trace_packet<MODE, STATS, KINDS, BLOCK, LANE_BOUNCES>;
     static int blocks = 0;
     if (!blocks) blocks = persistent_blocks(kern, BLOCK, num_sms);
-    note_launch(), kern<<<blocks, BLOCK, 0, stream>>>(P);
+    launch(kern, blocks, BLOCK, 0, stream, P);
 }
 
 // The traversal variants the autotuner chooses among: block size x depth of
@@ -1686,7 +1709,7 @@ template <bool STATS, uint32_t KINDS>
 void launch_ray_buffer_kernel(const RayBufferParams& P, int num_sms, cudaStream_t stream) {
     static int blocks = 0;
     if (!blocks) blocks = persistent_blocks(k_trace_ray_buffer<STATS, KINDS>, kTraceThreads, num_sms);
-    note_launch(), k_trace_ray_buffer<STATS, KINDS><<<blocks, kTraceThreads, 0, stream>>>(P);
+    launch(k_trace_ray_buffer<STATS, KINDS>, blocks, kTraceThreads, 0, stream, P);
 }
 
 }  // namespace
@@ -1816,10 +1839,6 @@ cudaError_t launch_trace_batch(const TraceBatch& tb, uint8_t* ws, int num_sms, c
     P.bounce = 0;
     P.kinds_built = tb.kinds_built;
     P.leaf_wait = tb.config.leaf_wait;
-    cudaError_t err = cudaMemsetAsync(P.B.ctr, 0, sizeof(WfCounters), stream);
-    if (err == cudaSuccess) err = cudaMemsetAsync(P.B.lit, 0, L.pixels * 4, stream);
-    if (err == cudaSuccess) err = cudaMemsetAsync(P.B.heat, 0, L.pixels * 8, stream);
-    if (err != cudaSuccess) return err;
     // scene records, kSetupChunk scenes per launch (their descriptions travel as kernel parameters)
     static SetupParams sp;  // 10 KB: kept off the stack; launches copy it
     static std::mutex sp_mu;
@@ -1838,28 +1857,28 @@ cudaError_t launch_trace_batch(const TraceBatch& tb, uint8_t* ws, int num_sms, c
             sp.status = tb.status;
             sp.first = first;
             sp.count = n;
-            note_launch(), k_setup<<<1, 128, 0, stream>>>(sp);
+            launch(k_setup, 1, 128, 0, stream, sp);
         }
     }
     const bool stats = tb.stats != 0;
     RtTraversalConfig config = tb.config;
     if (tb.choose_packets && L.slots >= kPacketSlots) config.packet_lists |= RT_TRAVERSAL_PACKET_PRIMARY;
-    note_launch(), k_raygen<<<(uint32_t)((L.slots + 255) / 256), 256, 0, stream>>>(P);
+    launch(k_raygen, (uint32_t)((L.slots + 255) / 256), 256, 0, stream, P);
     mark(kKernOther);
     // the traversal follows every mirror / portal bounce itself, so one closest-hit launch and one
     // shading launch cover all bounces
     P.bounce = 0;
     launch_trace_mode<kModeBounce>(P, config, stats, num_sms, stream);
     mark(kKernClosest);
-    note_launch(), k_shade<<<(uint32_t)((L.slots + 127) / 128), 128, 0, stream>>>(P);
+    launch(k_shade, (uint32_t)((L.slots + 127) / 128), 128, 0, stream, P);
     mark(kKernShade);
     if (L.any_shadow) {
         launch_trace_mode<kModeShadow>(P, config, stats, num_sms, stream);
         mark(kKernShadow);
-        note_launch(), k_resolve<<<(uint32_t)((L.pixels + 255) / 256), 256, 0, stream>>>(P);
+        launch(k_resolve, (uint32_t)((L.pixels + 255) / 256), 256, 0, stream, P);
         mark(kKernOther);
     }
-    note_launch(), k_output<<<(uint32_t)((L.pixels + 255) / 256), 256, 0, stream>>>(P);
+    launch(k_output, (uint32_t)((L.pixels + 255) / 256), 256, 0, stream, P);
     mark(kKernOther);
     return cudaGetLastError();
 }
@@ -1868,8 +1887,6 @@ cudaError_t launch_trace_ray_buffer(const RayBufferLaunch& p, int num_sms, cudaS
     RayBufferParams P;
     P.L = p;
     if (p.count == 0) return cudaSuccess;
-    cudaError_t err = cudaMemsetAsync(p.work, 0, sizeof(uint32_t), stream);
-    if (err != cudaSuccess) return err;
     for_each_variant(p.kinds_built, [&](auto k) {
         constexpr uint32_t K = decltype(k)::value;
         if (p.collect_stats) launch_ray_buffer_kernel<true, K>(P, num_sms, stream);
@@ -1880,7 +1897,7 @@ cudaError_t launch_trace_ray_buffer(const RayBufferLaunch& p, int num_sms, cudaS
 
 cudaError_t launch_debug_eval(uint32_t fn, const float* in, float* out, uint32_t count, cudaStream_t stream) {
     if (count == 0) return cudaSuccess;
-    note_launch(), k_debug_eval<<<(count + 127) / 128, 128, 0, stream>>>(fn, in, out, count);
+    launch(k_debug_eval, (count + 127) / 128, 128, 0, stream, fn, in, out, count);
     return cudaGetLastError();
 }
 

@@ -120,3 +120,28 @@ def test_tlas_sizes(device, n, flags):
                    for _ in range(n)])
     xf[n // 2] = 0.0  # a singular transform among them: never hit
     _check(device, _scene(_soup(12, "soup"), xf), TRACE, flags | abi.RT_BUILD_ALLOW_UPDATE, walk=False)
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 65, 511, 512, 513, 1500])
+@pytest.mark.parametrize("flags", [TRACE, TRACE | W4], ids=["w8", "w4"])
+def test_tlas_refit_sizes(device, n, flags):
+    """Every instance moved and the TLAS refitted in place: the hits of the oracle's fresh structure."""
+    host = _host()
+    rng = np.random.default_rng(n)
+
+    def transforms():
+        return np.stack([scenes.affine(scenes.rot_y(rng.uniform(0, 6)), rng.uniform(-4, 4, 3), rng.uniform(0.05, 0.4))
+                         for _ in range(n)])
+
+    model = _soup(12, "soup")
+    gs = host.GpuScene(device, _scene(model, transforms()), tlas_flags=flags | abi.RT_BUILD_ALLOW_UPDATE)
+    moved = _scene(model, transforms())
+    instances = host.Device.upload(gs.patch_instances(moved.instances))
+    gs.tlas.update_tlas(device, instances, n, gs.scratch)
+    rays = scenes.random_rays(3000, 23, 8.0)
+    rays["tmax"] = 1e4
+    g = host.trace_ray_buffer(device, gs, rays, with_models=False)
+    o, _ = O.OracleScene(moved).trace(rays, with_models=False)
+    for f in ("t", "u", "v", "instance_id", "primitive_index"):
+        assert (np.asarray(g[f]).view(np.uint32) == np.asarray(o[f]).view(np.uint32)).all(), f
+    assert gs.tlas.info(device).status == 0
