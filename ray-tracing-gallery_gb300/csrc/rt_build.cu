@@ -19,7 +19,7 @@
 //      follow each other in slot order, and a leaf child writes its
 //      primitives' positions (perm).
 //   6. primitive records written in that final order.
-// A TLAS of 2 to kTlasSmall instances goes through all of it in one block
+// A TLAS of up to kTlasSmall instances goes through all of it in one block
 // (k_tlas_small), whatever the build flags.
 // Everything runs on the caller's stream; no host synchronisation.
 //
@@ -1021,11 +1021,16 @@ __device__ __forceinline__ uint32_t ploc_take(const uint32_t* nbr, const float* 
     const float limit = best[x] * kPlocNear;
     float bd = INFINITY;
     uint32_t q = kNone;
+    // every place is read, whatever its neighbour says: short-circuited
+    // conditions made this 16 dependent reads (2,100 cycles of a 6,000-cycle round)
 #pragma unroll
     for (int o = 1 - kPlocRadius; o < kPlocRadius; o += 2) {  // odd offsets, ascending
-        const int y = x + o;
-        if (y >= first && y < last && nbr[y] == i && best[y] <= limit && best[y] < bd) {
-            bd = best[y];
+        const bool there = x + o >= first && x + o < last;
+        const int y = there ? x + o : x;
+        const uint32_t near = nbr[y];
+        const float b = best[y];
+        if (there & (near == i) & (b <= limit) & (b < bd)) {
+            bd = b;
             q = i + (uint32_t)o;
         }
     }
@@ -2093,7 +2098,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const Bu
 }
 
 // ---- small TLAS in one block ----------------------------------------------------------
-// A TLAS of 2 to 1,024 instances, one thread each: records and boxes, Morton
+// A TLAS of 1 to 1,024 instances, one thread each: records and boxes, Morton
 // sort, PLOC and the collapse in shared memory, one launch.  A frame rebuilds
 // such a TLAS before it traces, and eight launches that each work on a few
 // hundred instances were mostly launch and L2 latency.  Bound: latency, the
@@ -2176,7 +2181,11 @@ __global__ void __launch_bounds__(kTlasSmall) k_tlas_small(const __grid_constant
     c.width = a.width;
     c.max_nodes = a.max_nodes;
     c.n = n;
-    if ((tid >> 5) * 4u < a.max_nodes) collapse_loop<true>(c);  // a warp works on four nodes
+    if (n <= kTlasLeafMax) {
+        if (tid == 0) write_single_leaf(c);
+    } else if ((tid >> 5) * 4u < a.max_nodes) {  // a warp works on four nodes
+        collapse_loop<true>(c);
+    }
     __syncthreads();
     if (tid == 0) write_header(a.header, &s.st, hs);
     // eight lanes copy a record (temp was written by this block)
@@ -2622,7 +2631,7 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     hs.parents_offset = al.parents;
     hs.prim_bytes = top ? kInstBytes : kTriBytes;
 
-    if (top && n > kTlasLeafMax && n <= kTlasSmall) {
+    if (top && n > 0 && n <= kTlasSmall) {
         // a per-device attribute: set on every build (a host-side call, no device work)
         const cudaError_t smem_ok = cudaFuncSetAttribute(k_tlas_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          (int)sizeof(TlasSmallShared));
