@@ -1467,7 +1467,7 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
 // bounded.  Bound: latency, about seven dependent loads per level for small
 // structures; gathers of binary nodes for large ones.  (One launch per level
 // with one thread per task: 15-40 us a level; 163,840 triangles 290 us,
-// 10,485,760 triangles 1.3 ms.)
+X
 struct CollapseCtx {
     const uint4* inodes;
     const float4* iboxes;  // (lo, primitives below as bits), (hi, -) of each internal node
@@ -1545,7 +1545,7 @@ __device__ __forceinline__ void collapse_loop(const CollapseCtx& c) {
     const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, group = lane & 24u;
     const uint32_t lt = (1u << lane) - 1u;
     BuildState* st = c.st;
-    uint32_t slot = kNone, depth_seen = 0, spins = 0;
+    uint32_t slot = kNone, depth_seen = 0, spins = 0, unreported = 0;  // primitives this warp has placed
     for (;;) {
         // groups without a slot take the next ones
         const unsigned want = __ballot_sync(0xFFFFFFFFu, slot == kNone && sub == 0u);
@@ -1560,6 +1560,17 @@ __device__ __forceinline__ void collapse_loop(const CollapseCtx& c) {
         else if (slot < c.max_nodes) task = queue_load<SHARED>(&c.tasks[slot]);
         const bool ready = task != 0;
         if (!__any_sync(0xFFFFFFFFu, ready)) {
+            if (unreported) {  // before waiting: the warp that reports the last ones ends the launch
+                if (lane == 0) {
+                    const unsigned long long before = atomicAdd(&st->progress, (unsigned long long)unreported << 32);
+                    if ((uint32_t)(before >> 32) + unreported >= c.n) {
+                        st->node_count = (uint32_t)before;
+                        queue_store<SHARED>(&st->collapse_done, 1u);
+                    }
+                }
+                unreported = 0;
+                __syncwarp();
+            }
             if (queue_load<SHARED>(&st->collapse_done)) break;
             if (++spins > kCollapseSpinLimit) {
                 if (lane == 0) atomicOr(&st->error, 1u << RT_ERR_TIMEOUT);
@@ -1642,16 +1653,15 @@ __device__ __forceinline__ void collapse_loop(const CollapseCtx& c) {
         const unsigned inners = __ballot_sync(0xFFFFFFFFu, inner);
         uint32_t placed = leaf ? size : 0u;
         if (bad && sub == 0u) placed = bref + 1u < c.n ? __float_as_uint(c.iboxes[2 * (size_t)bref].w) : c.n;
-        placed = __reduce_add_sync(0xFFFFFFFFu, placed);
-        unsigned long long before = 0;
-        if (lane == 0) {
-            before = atomicAdd(&st->progress, ((unsigned long long)placed << 32) | (uint32_t)__popc(inners));
-            if ((uint32_t)(before >> 32) + placed >= c.n) {  // the last primitives: no task is left
-                st->node_count = (uint32_t)before + (uint32_t)__popc(inners);
-                queue_store<SHARED>(&st->collapse_done, 1u);
-            }
+        // Every warp adds to one counter: placed primitives are kept until the
+        // warp has nothing to do, and an iteration without internal children
+        // (most of them: the lowest nodes) leaves it alone.
+        unreported += __reduce_add_sync(0xFFFFFFFFu, placed);
+        uint32_t cs = 0;
+        if (inners) {
+            if (lane == 0) cs = (uint32_t)atomicAdd(&st->progress, (unsigned long long)__popc(inners));
+            cs = __shfl_sync(0xFFFFFFFFu, cs, 0) + (uint32_t)__popc(inners & lt);
         }
-        const uint32_t cs = (uint32_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)before, 0) + (uint32_t)__popc(inners & lt);
         bool used = child;
         uint32_t meta = 0, entry = 0;
         if (inner) {
