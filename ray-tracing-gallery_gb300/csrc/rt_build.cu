@@ -962,7 +962,7 @@ __device__ __forceinline__ float merged_half_area(float ax, float ay, float az, 
                                                   float cx, float cy, float cz, float dx, float dy, float dz) {
     // boxes (a, b) and (c, d) as lo, hi corners
     float ex = fmaxf(bx, dx) - fminf(ax, cx), ey = fmaxf(by, dy) - fminf(ay, cy), ez = fmaxf(bz, dz) - fminf(az, cz);
-    return ex * ey + ey * ez + ez * ex;
+    return fmaf(ex, ey + ez, ey * ez);
 }
 
 // The internal node of a merge: children a and b, the merged box, the primitives below.
@@ -1015,30 +1015,54 @@ __device__ uint32_t ploc_look_back(const unsigned long long* desc, uint32_t roun
     }
 }
 
-// The asker that position i (even, without a mutual neighbour) takes: of the
-// odd positions within R whose nearest neighbour is i, the one with the
-// smallest area, the lower one on ties; kNone if there is none near enough.
-// x: i's place in nbr / best; the places x - R .. x + R that lie in
-// [first, last) are looked at.
-__device__ __forceinline__ uint32_t ploc_take(const uint32_t* nbr, const float* best, uint32_t i, int x, int first,
-                                              int last) {
-    const float limit = best[x] * kPlocNear;
-    float bd = INFINITY;
-    uint32_t q = kNone;
-    // every place is read, whatever its neighbour says: short-circuited
-    // conditions made this 16 dependent reads (2,100 cycles of a 6,000-cycle round)
+// A neighbour and the area of the merge with it as one word: the area's bits
+// without the lowest five (a merge is chosen by the area to 2^-18 of itself),
+// and there the neighbour's offset, -R..-1 as 0..15 and 1..R as 16..31.  The
+// smallest word is the nearest neighbour, the lower position on ties.  No
+// finite area reaches kPlocNoKey (infinity and NaN are above it).
+static_assert(kPlocRadius == 16, "32 offsets");
+constexpr uint32_t kPlocNoKey = 0x7F800000u;
+__device__ __forceinline__ uint32_t ploc_key(uint32_t area_bits, int offset) {
+    return area_bits | (uint32_t)(offset < 0 ? offset + kPlocRadius : offset + kPlocRadius - 1);
+}
+__device__ __forceinline__ int ploc_offset(uint32_t key) {
+    const int k = (int)(key & 31u);
+    return k < kPlocRadius ? k - kPlocRadius : k - kPlocRadius + 1;
+}
+// The place of place x's nearest neighbour; x itself if it has none.
+__device__ __forceinline__ int ploc_near(const uint32_t* keys, int x) {
+    const uint32_t k = keys[x];
+    return k < kPlocNoKey ? x + ploc_offset(k) : x;
+}
+// The nearest neighbour of place x of position i, whose neighbours' areas are
+// in area[o - 1][place of the lower].  FIRST: place 0 is the first position;
+// otherwise there are R places before x.
+template <bool FIRST, int STRIDE>
+__device__ __forceinline__ uint32_t ploc_nearest(const uint32_t (*area)[STRIDE], int x) {
+    uint32_t best = 0xFFFFFFFFu;
 #pragma unroll
-    for (int o = 1 - kPlocRadius; o < kPlocRadius; o += 2) {  // odd offsets, ascending
-        const bool there = x + o >= first && x + o < last;
-        const int y = there ? x + o : x;
-        const uint32_t near = nbr[y];
-        const float b = best[y];
-        if (there & (near == i) & (b <= limit) & (b < bd)) {
-            bd = b;
-            q = i + (uint32_t)o;
-        }
+    for (int o = 1; o <= kPlocRadius; o++) {
+        const uint32_t down = !FIRST || x >= o ? ploc_key(area[o - 1][x - o], -o) : 0xFFFFFFFFu;
+        best = min(best, min(down, ploc_key(area[o - 1][x], o)));
     }
-    return q;
+    return best;
+}
+// Place x (its neighbour at y, odd position, not mutual) asks y when y's
+// position is even, it has no mutual neighbour either and its own nearest is
+// hardly nearer.
+__device__ __forceinline__ void ploc_ask(const uint32_t* keys, uint32_t* take, int x, int y) {
+    const uint32_t mine = keys[x], theirs = keys[y];
+    const int z = ploc_near(keys, y);
+    if (z != y && ploc_near(keys, z) == y) return;
+    if (__uint_as_float(mine & ~31u) <= __uint_as_float(theirs & ~31u) * kPlocNear)
+        atomicMin(&take[y], ploc_key(mine & ~31u, x - y));
+}
+// The place that place x merges with (x itself: none).  odd: of its position.
+__device__ __forceinline__ int ploc_partner(const uint32_t* keys, const uint32_t* take, int x, int y, bool mutual,
+                                            bool odd) {
+    if (mutual) return y;
+    if (!odd) return take[x] != 0xFFFFFFFFu ? x + ploc_offset(take[x]) : x;
+    return y != x && take[y] == ploc_key(keys[x] & ~31u, x - y) ? y : x;
 }
 
 // One round over more than kPlocSmall clusters.  A block takes tiles in
@@ -1046,8 +1070,7 @@ __device__ __forceinline__ uint32_t ploc_take(const uint32_t* nbr, const float* 
 // 3 R on each side a halo: boxes for all 512, the areas of the pairs
 // (p, p + 1..R) once each (they do not depend on the order of the boxes) in
 // shared memory, the nearest neighbour (smallest area, the lower position on
-// ties) of the positions within 2 R of an own one, the askers taken by those
-// within R, then the merges of the own positions: the lower of a pair keeps
+// ties) of the positions within 2 R of an own one, which ask those within R, then the merges of the own positions: the lower of a pair keeps
 // the new node, the higher drops out.  The tile claims its merges' node ids with one atomic
 // (counting down from n - 2) and finds its survivors' output position by
 // look-back over the earlier tiles, so one launch reads each cluster once and
@@ -1070,10 +1093,9 @@ __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_con
     float4* cout = a.cbox[(word & kPlocParity) ? 0 : 1];
     __shared__ float4 s0[T];          // lo, hi.x
     __shared__ float2 s1[T];          // hi.y, hi.z
-    __shared__ float area[R][T - R];  // area[o - 1][t] = area of the pair (t, t + o)
-    __shared__ uint32_t nbr[T];       // nearest neighbour (position in the round)
-    __shared__ float best_area[T];    // its area
-    uint32_t* take = reinterpret_cast<uint32_t*>(&area[0][0]);  // the asker a position takes (once area is done with)
+    __shared__ uint32_t area[R][T - R];  // area[o - 1][t] = area of the pair (t, t + o), its bits as in ploc_key
+    __shared__ uint32_t keys[T];         // nearest neighbours
+    __shared__ uint32_t take[T];         // the asker a place takes
     __shared__ uint32_t warp_sums[2 * T / 32];  // each warp's total, then the totals before it
     __shared__ uint32_t s_tile, s_claim, s_prefix;
     const int t = (int)threadIdx.x;
@@ -1087,7 +1109,8 @@ __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_con
         const int i = (int)(tile * kPlocTile) - 3 * R + t;  // this thread's position
         const bool inside = i >= 0 && i < (int)count;
         const bool own = inside && t >= 3 * R && t < T - 3 * R;
-        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+        // outside the round: a box whose merges have infinite area
+        float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = lo;
         if (inside) {
             if (round == 0) {
                 const size_t p = a.vals[i];
@@ -1112,57 +1135,36 @@ __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_con
             for (int o = 1; o <= R; o++) {
                 const float4 c = s0[t + o];
                 const float2 d = s1[t + o];
-                const float h = merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y, c.z, c.w, d.x, d.y);
-                area[o - 1][t] = i >= 0 && i + o < (int)count ? h : INFINITY;
+                area[o - 1][t] = __float_as_uint(merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y, c.z,
+                                                                  c.w, d.x, d.y)) & ~31u;
             }
         }
         __syncthreads();
-        uint32_t near = kNone;
         if (t >= R && t < T - R) {
-            int best = i;
-            float bd = INFINITY;
-            if (inside && forced) {
-                if ((i ^ 1) < (int)count) best = i ^ 1;
-            } else if (inside) {
-#pragma unroll
-                for (int o = R; o >= 1; o--) {  // candidates i - R .. i - 1
-                    const float h = area[o - 1][t - o];
-                    if (h < bd) {  // ties keep the lower position
-                        bd = h;
-                        best = i - o;
-                    }
-                }
-#pragma unroll
-                for (int o = 1; o <= R; o++) {  // candidates i + 1 .. i + R
-                    const float h = area[o - 1][t];
-                    if (h < bd) {
-                        bd = h;
-                        best = i + o;
-                    }
-                }
-            }
-            near = inside ? (uint32_t)best : kNone;
-            nbr[t] = near;
-            best_area[t] = bd;
+            uint32_t key = 0xFFFFFFFFu;
+            if (!forced) key = ploc_nearest<false, T - R>(area, t);
+            else if ((i ^ 1) < (int)count) key = ploc_key(0u, (i ^ 1) - i);
+            keys[t] = inside ? key : 0xFFFFFFFFu;
         }
+        take[t] = 0xFFFFFFFFu;
         __syncthreads();
+        int near = t;
         bool mutual = false;
-        if (t >= 2 * R && t < T - 2 * R && inside) {
-            mutual = near != (uint32_t)i && nbr[t + ((int)near - i)] == (uint32_t)i;
-            take[t] = !mutual && !(i & 1) ? ploc_take(nbr, best_area, (uint32_t)i, t, R, T - R) : kNone;
+        if (t >= R && t < T - R && inside) {
+            near = ploc_near(keys, t);
+            if (near >= 2 * R && near < T - 2 * R) {  // the neighbours that an own place can have
+                mutual = near != t && ploc_near(keys, near) == t;
+                if (near != t && !mutual && (i & 1) && !((i + near - t) & 1)) ploc_ask(keys, take, t, near);
+            }
         }
         __syncthreads();
         uint32_t k = 0u;
         bool merging = false;
         int tj = t;
         if (own) {
-            uint32_t j = (uint32_t)i;  // the cluster to merge with; i itself: none
-            if (mutual) j = near;
-            else if (!(i & 1)) j = take[t] != kNone ? take[t] : j;
-            else if (take[t + ((int)near - i)] == (uint32_t)i) j = near;
-            tj = t + ((int)j - i);
-            merging = (int)j > i;
-            k = (int)j < i ? 0u : 1u;
+            tj = ploc_partner(keys, take, t, near, mutual, (i & 1) != 0);  // t itself: no merge
+            merging = tj > t;
+            k = tj < t ? 0u : 1u;
         }
         // one scan counts survivors (low 16 bits) and merges (high 16 bits)
         const uint32_t v = k | (merging ? 1u << 16 : 0u);
@@ -1244,13 +1246,12 @@ __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_con
 // left more than kPlocSmall clusters, neighbour pairs are merged in global
 // memory until that few remain.
 struct PlocTailShared {
-    float4 s0[kPlocSmall];   // lo, hi.x
-    float2 s1[kPlocSmall];   // hi.y, hi.z
-    uint2 ref[kPlocSmall];   // binary reference, primitives below
-    uint32_t nbr[kPlocSmall];
-    float best[kPlocSmall];
-    // area[o - 1][i] = area of the pair (i, i + o); then row 0 holds the asker each position takes
-    float area[kPlocRadius][kPlocSmall];
+    float4 s0[kPlocSmall + kPlocRadius];  // lo, hi.x; behind the last cluster, boxes of infinite area
+    float2 s1[kPlocSmall + kPlocRadius];  // hi.y, hi.z
+    uint2 ref[kPlocSmall];                // binary reference, primitives below
+    uint32_t keys[kPlocSmall];            // nearest neighbours
+    uint32_t take[kPlocSmall];            // the asker a position takes
+    uint32_t area[kPlocRadius][kPlocSmall];  // area[o - 1][i] = area of the pair (i, i + o), its bits as in ploc_key
     uint32_t warp_sums[32];
 };
 // Rounds until one of the `count` clusters in s is left; returns the merges
@@ -1261,6 +1262,12 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
     constexpr int R = kPlocRadius;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     bool forced = false;
+    const float inf = INFINITY;
+    if (tid < (uint32_t)R) {
+        s.s0[count + tid] = make_float4(inf, inf, inf, inf);
+        s.s1[count + tid] = make_float2(inf, inf);
+    }
+    __syncthreads();
     while (count > 1u) {  // a round after one with next to no merges merges pairs: it ends
         const uint32_t blocks = (count + 31u) >> 5;  // of 32 clusters
         if (!forced) {
@@ -1273,48 +1280,30 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
                 const uint32_t step = 1u << lg;
 #pragma unroll 4
                 for (uint32_t o = 1u + (warp & (step - 1u)); o <= (uint32_t)R; o += step) {
-                    const uint32_t j = (i + o) & (kPlocSmall - 1u);
-                    const float4 u = s.s0[j];
-                    const float2 v = s.s1[j];
-                    const float h = merged_half_area(p.x, p.y, p.z, p.w, q.x, q.y, u.x, u.y, u.z, u.w, v.x, v.y);
-                    s.area[o - 1u][i] = i + o < count ? h : INFINITY;
+                    const float4 u = s.s0[i + o];
+                    const float2 v = s.s1[i + o];
+                    s.area[o - 1u][i] =
+                        __float_as_uint(merged_half_area(p.x, p.y, p.z, p.w, q.x, q.y, u.x, u.y, u.z, u.w, v.x, v.y)) &
+                        ~31u;
                 }
             }
         }
         __syncthreads();
         const bool here = tid < count;
-        uint32_t near = tid;
         if (here) {
-            float bd = INFINITY;
-            if (forced) {
-                if ((tid ^ 1u) < count) near = tid ^ 1u;
-            } else {
-#pragma unroll
-                for (int o = R; o >= 1; o--) {  // candidates i - R .. i - 1
-                    const float h = tid >= (uint32_t)o ? s.area[o - 1][tid - o] : INFINITY;
-                    if (h < bd) {  // ties keep the lower position
-                        bd = h;
-                        near = tid - o;
-                    }
-                }
-#pragma unroll
-                for (int o = 1; o <= R; o++) {  // candidates i + 1 .. i + R
-                    const float h = s.area[o - 1][tid];
-                    if (h < bd) {
-                        bd = h;
-                        near = tid + o;
-                    }
-                }
-            }
-            s.nbr[tid] = near;
-            s.best[tid] = bd;
+            uint32_t key = 0xFFFFFFFFu;
+            if (!forced) key = ploc_nearest<true, kPlocSmall>(s.area, (int)tid);
+            else if ((tid ^ 1u) < count) key = ploc_key(0u, (int)(tid ^ 1u) - (int)tid);
+            s.keys[tid] = key;
+            s.take[tid] = 0xFFFFFFFFu;
         }
         __syncthreads();
-        uint32_t* take = reinterpret_cast<uint32_t*>(&s.area[0][0]);
+        int near = (int)tid;
         bool mutual = false;
         if (here) {
-            mutual = near != tid && s.nbr[near] == tid;
-            take[tid] = !mutual && !(tid & 1u) ? ploc_take(s.nbr, s.best, tid, (int)tid, 0, (int)count) : kNone;
+            near = ploc_near(s.keys, (int)tid);
+            mutual = near != (int)tid && ploc_near(s.keys, near) == (int)tid;
+            if (near != (int)tid && !mutual && (tid & 1u) && !(near & 1)) ploc_ask(s.keys, s.take, (int)tid, near);
         }
         __syncthreads();
         bool keep = false, merge = false;
@@ -1323,11 +1312,8 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
         uint2 r = make_uint2(0u, 0u);
         uint32_t partner = 0u;
         if (here) {
-            uint32_t j = tid;  // the cluster to merge with; tid itself: none
-            if (mutual) j = near;
-            else if (!(tid & 1u)) j = take[tid] != kNone ? take[tid] : j;
-            else if (take[near] == tid) j = near;
-            merge = j > tid;
+            const uint32_t j = (uint32_t)ploc_partner(s.keys, s.take, (int)tid, near, mutual, (tid & 1u) != 0u);
+            merge = j > tid;  // tid itself: no merge
             keep = j >= tid;
             p = s.s0[tid];
             q = s.s1[tid];
@@ -1371,6 +1357,10 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
         merges += total >> 16;
         forced = (total & 0xFFFFu) > count - 1u - count / 32u;
         count = total & 0xFFFFu;
+        if (tid < (uint32_t)R) {
+            s.s0[count + tid] = make_float4(inf, inf, inf, inf);
+            s.s1[count + tid] = make_float2(inf, inf);
+        }
         __syncthreads();
     }
     return merges;
