@@ -942,7 +942,7 @@ constexpr float kPlocNear = 1.25f;
 constexpr double kPlocFirstRate = 0.62, kPlocRate = 0.765;  // survivors of the first and of later rounds, at most
 constexpr uint32_t kPlocThreads = 512;
 constexpr uint32_t kPlocTile = kPlocThreads - 6 * kPlocRadius;  // clusters a block owns per tile
-constexpr uint32_t kPlocMaxBlocks = 152 * 3;
+constexpr uint32_t kPlocMaxBlocks = 152 * 4;
 constexpr uint32_t kPlocParity = 1u << 31, kPlocForced = 1u << 30, kPlocCount = (1u << 28) - 1u;
 constexpr uint32_t kPlocSpinLimit = 1u << 22;
 
@@ -1079,7 +1079,12 @@ __device__ __forceinline__ int ploc_partner(const uint32_t* keys, const uint32_t
 // cluster: PLOC of 10.5M triangles 3.6 ms; of 164k triangles 410 us.)  Bound:
 // shared-memory and arithmetic issue for large counts, latency for small.
 // The first round gathers the Morton-ordered primitive boxes itself.
-__global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_round(const __grid_constant__ PlocArgs a, int round) {
+// PER_SM: resident blocks, 4 (32 registers) where there are tiles for them
+// all, which overlaps one tile's gathers with more others' arithmetic (10.5M
+// triangles: pass 3.86 -> 3.64 ms), 3 (38 registers) for rounds bound by
+// the latency of one tile (163,840 triangles 0.5 % faster so).
+template <int PER_SM>
+__global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __grid_constant__ PlocArgs a, int round) {
     after_previous();
     BuildState* st = a.st;
     const uint32_t word = st->ploc_round[round], count = word & kPlocCount;
@@ -2678,8 +2683,12 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
             pa.desc = zero_ploc.desc;
             pa.n = n;
             const int rounds = ploc_grid_rounds(n);
-            for (int r = 0; r < rounds; r++)
-                launch(k_ploc_round, ploc_round_blocks(n, r), kPlocThreads, 0, stream, pa, r);
+            for (int r = 0; r < rounds; r++) {
+                if (const uint32_t g = ploc_round_blocks(n, r); g == kPlocMaxBlocks)
+                    launch(k_ploc_round<4>, g, kPlocThreads, 0, stream, pa, r);
+                else
+                    launch(k_ploc_round<3>, g, kPlocThreads, 0, stream, pa, r);
+            }
             // a per-device attribute: set on every build (a host-side call, no device work)
             const cudaError_t smem_ok =
                 cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
