@@ -268,12 +268,20 @@ __device__ __forceinline__ void rt_sincos(float x, float* s, float* c) {
     *c = co;
 }
 
+__device__ __forceinline__ V3 safe_inv(V3 d) {
+    const float e = 1e-20f;
+    return mk3(1.0f / (fabsf(d.x) < e ? copysignf(e, d.x) : d.x), 1.0f / (fabsf(d.y) < e ? copysignf(e, d.y) : d.y),
+               1.0f / (fabsf(d.z) < e ? copysignf(e, d.z) : d.z));
+}
+
 // Watertight ray setup (Woop, Benthin & Wald 2013).
 struct WtRay {
     int kx, ky, kz;
     float sx, sy, sz;
 };
-__device__ __forceinline__ WtRay wt_setup(V3 d) {
+// inv = safe_inv(d): kz is the largest component, so inv holds 1 / dz unless
+// every component is tiny.
+__device__ __forceinline__ WtRay wt_setup(V3 d, V3 inv) {
     float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     int kz = 0;
     if (ay > ax) kz = 1;
@@ -282,7 +290,8 @@ __device__ __forceinline__ WtRay wt_setup(V3 d) {
     if (kx == 3) kx = 0;
     int ky = kx + 1;
     if (ky == 3) ky = 0;
-    if (get3(d, kz) < 0.0f) {
+    float dz = get3(d, kz);
+    if (dz < 0.0f) {
         int t = kx;
         kx = ky;
         ky = t;
@@ -291,10 +300,9 @@ __device__ __forceinline__ WtRay wt_setup(V3 d) {
     w.kx = kx;
     w.ky = ky;
     w.kz = kz;
-    float dz = get3(d, kz);
     w.sx = get3(d, kx) / dz;
     w.sy = get3(d, ky) / dz;
-    w.sz = 1.0f / dz;
+    w.sz = fabsf(dz) < 1e-20f ? 1.0f / dz : get3(inv, kz);
     return w;
 }
 
@@ -345,10 +353,5 @@ __device__ __forceinline__ bool tri_intersect(V3 o, const WtRay& w, V3 v0, V3 v1
 // Conservative slab-test scale on the far distance (Ize 2013, 1 + 2*gamma(3)).
 constexpr float kBoxFarScale = 1.0000004f;
 
-__device__ __forceinline__ V3 safe_inv(V3 d) {
-    const float e = 1e-20f;
-    return mk3(1.0f / (fabsf(d.x) < e ? copysignf(e, d.x) : d.x), 1.0f / (fabsf(d.y) < e ? copysignf(e, d.y) : d.y),
-               1.0f / (fabsf(d.z) < e ? copysignf(e, d.z) : d.z));
-}
 
 }  // namespace rt

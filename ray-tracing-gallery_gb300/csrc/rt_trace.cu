@@ -157,6 +157,7 @@ __device__ __forceinline__ void sort8(uint32_t k[8]) {
 // ---------------------------------------------------------------------------
 struct Trav {
     V3 wo, wd;                 // world ray
+    V3 winv;                   // 1 / wd, kept for the return from an instance
     V3 o, d, inv;              // ray in the current space (world or object)
     uint32_t oct;              // octant_offsets(inv)
     WtRay wt;                  // watertight shear of the object-space ray
@@ -182,6 +183,7 @@ __device__ __forceinline__ void trav_begin(Trav& s, const Env& e, V3 o, V3 d, fl
     s.o = o;
     s.d = d;
     s.inv = safe_inv(d);
+    s.winv = s.inv;
     s.oct = octant_offsets(s.inv);
     s.wt.kx = s.wt.ky = s.wt.kz = 0;
     s.wt.sx = s.wt.sy = s.wt.sz = 0.0f;
@@ -239,7 +241,7 @@ __device__ __forceinline__ void trav_restore_world(Trav& s, const Env& e) {
     s.quant = false;
     s.o = s.wo;
     s.d = s.wd;
-    s.inv = safe_inv(s.wd);
+    s.inv = s.winv;
     s.oct = octant_offsets(s.inv);
 }
 
@@ -258,6 +260,16 @@ __device__ __forceinline__ float2 slab2(float a0, float a1, float neg_o, float i
         "add.rn.f32x2 p, p, q;\n\tmul.rn.f32x2 p, p, i;\n\tmov.b64 {%0, %1}, p;\n\t}"
         : "=f"(r.x), "=f"(r.y)
         : "f"(a0), "f"(a1), "f"(neg_o), "f"(inv));
+    return r;
+}
+
+// a * s + n of two values at once.
+__device__ __forceinline__ float2 fma2(float a0, float a1, float s, float n) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, i;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tmov.b64 i, {%5, %5};\n\t"
+        "fma.rn.f32x2 p, p, q, i;\n\tmov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a0), "f"(a1), "f"(s), "f"(n));
     return r;
 }
 
@@ -384,16 +396,21 @@ __device__ __forceinline__ const uint32_t* qnode_keys(const Trav& s, uint32_t en
     const float Nx = fmaf(-kQuantMargin, ax, Cx), Ny = fmaf(-kQuantMargin, ay, Cy), Nz = fmaf(-kQuantMargin, az, Cz);
     const float Fx = fmaf(kQuantMargin, ax, Cx), Fy = fmaf(kQuantMargin, ay, Cy), Fz = fmaf(kQuantMargin, az, Cz);
     const float tcap = s.t, tlo = s.tmin;
+    auto key = [&](float tn, float tf, int k) {
+        return child_key(fmaxf(fmaf(-kQuantRelative, fabsf(tn), tn), tlo), fminf(fmaf(kQuantRelative, fabsf(tf), tf), tcap),
+                         refs[k], k);
+    };
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < 8; k += 2) {
         const int j = k & 3;
         const uint32_t wnx = k < 4 ? nx.x : nx.y, wfx = k < 4 ? fx.x : fx.y;
         const uint32_t wny = k < 4 ? ny.x : ny.y, wfy = k < 4 ? fy.x : fy.y;
         const uint32_t wnz = k < 4 ? nz.x : nz.y, wfz = k < 4 ? fz.x : fz.y;
-        const float tn = fmax3(fmaf(qbyte(wnx, j), Sx, Nx), fmaf(qbyte(wny, j), Sy, Ny), fmaf(qbyte(wnz, j), Sz, Nz));
-        const float tf = fmin3(fmaf(qbyte(wfx, j), Sx, Fx), fmaf(qbyte(wfy, j), Sy, Fy), fmaf(qbyte(wfz, j), Sz, Fz));
-        keys[k] = child_key(fmaxf(fmaf(-kQuantRelative, fabsf(tn), tn), tlo),
-                            fminf(fmaf(kQuantRelative, fabsf(tf), tf), tcap), refs[k], k);
+        const float2 ax2 = fma2(qbyte(wnx, j), qbyte(wnx, j + 1), Sx, Nx), bx2 = fma2(qbyte(wfx, j), qbyte(wfx, j + 1), Sx, Fx);
+        const float2 ay2 = fma2(qbyte(wny, j), qbyte(wny, j + 1), Sy, Ny), by2 = fma2(qbyte(wfy, j), qbyte(wfy, j + 1), Sy, Fy);
+        const float2 az2 = fma2(qbyte(wnz, j), qbyte(wnz, j + 1), Sz, Nz), bz2 = fma2(qbyte(wfz, j), qbyte(wfz, j + 1), Sz, Fz);
+        keys[k] = key(fmax3(ax2.x, ay2.x, az2.x), fmin3(bx2.x, by2.x, bz2.x), k);
+        keys[k + 1] = key(fmax3(ax2.y, ay2.y, az2.y), fmin3(bx2.y, by2.y, bz2.y), k + 1);
     }
     return child_ref;
 }
@@ -418,7 +435,7 @@ __device__ __forceinline__ void enter_instance(Trav& s, const InstRecord* ir, ui
     s.d = xform_dir(w, s.wd);
     s.inv = safe_inv(s.d);
     s.oct = octant_offsets(s.inv);
-    s.wt = wt_setup(s.d);
+    s.wt = wt_setup(s.d, s.inv);
     const uint8_t* blas = reinterpret_cast<const uint8_t*>(((uint64_t)q0.y << 32) | q0.x);
     s.nodes = reinterpret_cast<const WideNode*>(blas + kHeaderBytes);
     s.tris = reinterpret_cast<const TriRecord*>(blas + (uint64_t)q1.w * 256u);
@@ -1584,7 +1601,7 @@ __global__ void k_debug_eval(uint32_t fn, const float* in, float* out, uint32_t 
         case RT_FN_WATERTIGHT: {
             const float* p = in + 16 * (size_t)i;
             V3 o = mk3(p[0], p[1], p[2]), d = mk3(p[3], p[4], p[5]);
-            WtRay w = wt_setup(d);
+            WtRay w = wt_setup(d, safe_inv(d));
             float t = 0, u = 0, v = 0;
             bool front = false;
             bool hit = tri_intersect(o, w, mk3(p[6], p[7], p[8]), mk3(p[9], p[10], p[11]), mk3(p[12], p[13], p[14]),
