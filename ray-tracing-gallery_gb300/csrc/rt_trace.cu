@@ -165,6 +165,7 @@ struct Trav {
     float t, u, v;             // best hit so far (t = tmax before any hit)
     uint32_t hit_inst;         // sorted TLAS index of the best hit, kNoHit if none
     uint32_t hit_geom, hit_prim;
+    uint32_t hit_sbt_flags;    // of the best hit's instance
     bool front, in_blas;
     bool quant;                // current nodes are QNodes (a quantised BLAS)
     uint32_t entry;            // what the next step processes
@@ -192,6 +193,7 @@ __device__ __forceinline__ void trav_begin(Trav& s, const Env& e, V3 o, V3 d, fl
     s.u = s.v = 0.0f;
     s.hit_inst = kNoHit;
     s.hit_geom = s.hit_prim = kNoHit;
+    s.hit_sbt_flags = 0;
     s.front = false;
     s.in_blas = false;
     s.sp = 0;
@@ -494,6 +496,7 @@ __device__ __forceinline__ bool try_triangle(Trav& s, const SV& sv, const RtShad
     s.hit_inst = s.c_inst;
     s.hit_geom = geom;
     s.hit_prim = prim;
+    s.hit_sbt_flags = s.c_sbt_flags;
     s.front = front;
     return true;
 }
@@ -526,12 +529,13 @@ struct alignas(128) SceneRec {
     uint32_t* image;           // RGBA8, may be null
     float4* radiance;          // may be null
     uint32_t width, height, max_depth, shadow_count;
-    uint32_t flags;            // RT_TRACE_FLAG_* of this scene
+    uint32_t flags;            // RT_TRACE_FLAG_* of this scene, kSceneHeat
     uint32_t tiles_x;          // 8x4 tiles per row
     uint32_t tile_begin;       // first tile of the batch's tile list
     uint32_t pixel_begin;      // first pixel of the batch's pixel list
 };
 static_assert(sizeof(SceneRec) == 128, "scene record size");
+constexpr uint32_t kSceneHeat = 1u << 31;  // its uniforms ask for the heatmap
 
 struct OneScene {
     Env e;
@@ -841,7 +845,7 @@ __global__ void k_setup(const __grid_constant__ SetupParams P) {
     r.height = d.desc.height;
     r.max_depth = d.desc.max_trace_depth;
     r.shadow_count = d.desc.shadow_ray_count;
-    r.flags = d.desc.flags;
+    r.flags = (d.desc.flags & ~kSceneHeat) | (r.uniforms->show_heatmap ? kSceneHeat : 0u);
     r.tiles_x = P.lay[t].tiles_x;
     r.tile_begin = P.lay[t].tile_begin;
     r.pixel_begin = P.lay[t].pixel_begin;
@@ -927,6 +931,13 @@ __device__ __forceinline__ NextRay next_bounce_ray(const Env& e, const RtShaderB
     return r;
 }
 
+// Whether the closest-hit program of a hit continues the ray: asked with the
+// flags that came with the hit, before anything is read for it.
+__device__ __forceinline__ bool continues(const RtShaderBindingTable* sbt, uint32_t sbt_flags) {
+    const RtHitGroup* g = hit_group(sbt, sbt_flags, 0u);
+    return g && (g->closest_hit == RT_PROGRAM_CLOSEST_HIT_MIRROR || g->closest_hit == RT_PROGRAM_CLOSEST_HIT_PORTAL);
+}
+
 // Ray-list scene words carry the ray's bounce depth in their top byte.
 constexpr uint32_t kSceneBits = 24;
 constexpr uint32_t kSceneMask = (1u << kSceneBits) - 1u;
@@ -997,7 +1008,7 @@ __device__ __forceinline__ void trace_wavefront(const WfParams& P) {
                 trav_begin(s, sv(sc), mk3(a.x, a.y, a.z), mk3(c.x, c.y, c.z), a.w, c.w);
             }
             s.scene = sc;
-            heat = pix != kNoPixel && P.B.scenes[sc].uniforms->show_heatmap != 0;
+            heat = pix != kNoPixel && (P.B.scenes[sc].flags & kSceneHeat) != 0u;
             if (heat) t0 = (uint32_t)clock();
         }
         const int phase = node_phase(s.entry, P.leaf_wait) ? 1 : 0;
@@ -1005,7 +1016,8 @@ __device__ __forceinline__ void trace_wavefront(const WfParams& P) {
             continue;
         // the ray is finished
         if (MODE == kModeBounce) {
-            if (s.hit_inst != kNoHit && (depth & 0xFFu) + 1 < P.B.scenes[s.scene].max_depth) {
+            if (s.hit_inst != kNoHit && continues(&P.sbt, s.hit_sbt_flags) &&
+                (depth & 0xFFu) + 1 < P.B.scenes[s.scene].max_depth) {
                 const NextRay nr =
                     next_bounce_ray(P.B.scenes[s.scene].env, &P.sbt, s.hit_inst, s.hit_geom, s.hit_prim, s.t, s.u,
                                     s.v, s.wo, s.wd);
@@ -1248,7 +1260,7 @@ __device__ __forceinline__ void trace_packets(const WfParams& P) {
             }
             s.scene = sc;
         }
-        const bool heat = pix != kNoPixel && P.B.scenes[s.scene].uniforms->show_heatmap != 0;
+        const bool heat = pix != kNoPixel && (P.B.scenes[s.scene].flags & kSceneHeat) != 0u;
         const uint32_t t0 = heat ? (uint32_t)clock() : 0u;
         unsigned pending = __ballot_sync(0xFFFFFFFFu, s.entry != kNoEntry);
         while (pending) {
@@ -1263,7 +1275,8 @@ __device__ __forceinline__ void trace_packets(const WfParams& P) {
                     // every further bounce of the lane's ray, traced by the lane
                     // alone (the closest-hit program's arithmetic, bit for bit)
                     TravStack<0, BLOCK> stk;
-                    while (s.hit_inst != kNoHit && depth + 1 < P.B.scenes[s.scene].max_depth) {
+                    while (s.hit_inst != kNoHit && continues(&P.sbt, s.hit_sbt_flags) &&
+                           depth + 1 < P.B.scenes[s.scene].max_depth) {
                         const NextRay nr = next_bounce_ray(P.B.scenes[s.scene].env, &P.sbt, s.hit_inst, s.hit_geom,
                                                            s.hit_prim, s.t, s.u, s.v, s.wo, s.wd);
                         if (nr.d.x == 0.0f && nr.d.y == 0.0f && nr.d.z == 0.0f) break;
@@ -1275,7 +1288,7 @@ __device__ __forceinline__ void trace_packets(const WfParams& P) {
                                                         cnt, -1)) {
                         }
                     }
-                } else if (MODE == kModeBounce && s.hit_inst != kNoHit &&
+                } else if (MODE == kModeBounce && s.hit_inst != kNoHit && continues(&P.sbt, s.hit_sbt_flags) &&
                            depth + 1 < P.B.scenes[s.scene].max_depth) {
                     // a mirror / portal hit with depth left: the lane's next ray
                     // joins the chunk's next sub-packet
