@@ -12,14 +12,23 @@ namespace rt {
 // Counts every kernel this library launches (rt_kernel_launch_count).
 void note_launch();
 
-// Every kernel of the build and trace sequences begins with after_previous()
+// Every kernel of the build and trace sequences begins with one of these two
 // and is launched by launch(): it may become resident while the previous
 // kernel of its stream still runs, and waits there until that one has
 // completed and its writes are visible, so the launch latency of a short
-// kernel is hidden (programmatic dependent launch).  The next kernel may
-// become resident from then on; no block returns before the wait, so a kernel
-// that has completed implies that all before it have.
-__device__ __forceinline__ void after_previous() {
+// kernel is hidden (programmatic dependent launch).  No block returns before
+// the wait, so a kernel that has completed implies that all before it have.
+//
+// A kernel that lets the next one become resident early gives it the places
+// of its own finished blocks to wait in.  Behind a traversal, whose last
+// blocks end long after the first, those places are what another stream's
+// kernels would run in: with two frames in flight on two streams the frames
+// stopped overlapping (1280x720 default scene 0.52 -> 0.70 ms a frame,
+// 1920x1080 4.07 -> 4.26; 0.45 and 3.67 when the traversal kernels only wait).
+__device__ __forceinline__ void after_previous_alone() {  // traversals
+    cudaGridDependencySynchronize();
+}
+__device__ __forceinline__ void after_previous() {  // all others
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
 }

@@ -1062,7 +1062,7 @@ __device__ __forceinline__ bool kinds_selected(uint32_t kinds_built, uint32_t tl
 template <int MODE, bool STATS, uint32_t KINDS, int SD, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, trace_warps_per_sm(KINDS) * 32 / BLOCK)
     k_trace(const __grid_constant__ WfParams P) {
-    after_previous();
+    after_previous_alone();
     if (kinds_selected(P.kinds_built, P.B.ctr->kinds, KINDS)) trace_wavefront<MODE, STATS, KINDS, SD, BLOCK>(P);
 }
 
@@ -1342,7 +1342,7 @@ constexpr int packet_warps_per_sm(uint32_t kinds, int block) {
 template <int MODE, bool STATS, uint32_t KINDS, int BLOCK, bool LANE_BOUNCES>
 __global__ void __launch_bounds__(BLOCK, packet_warps_per_sm(KINDS, BLOCK) * 32 / BLOCK)
     k_trace_packet(const __grid_constant__ WfParams P) {
-    after_previous();
+    after_previous_alone();
     if (kinds_selected(P.kinds_built, P.B.ctr->kinds, KINDS))
         trace_packets<MODE, STATS, KINDS, BLOCK, LANE_BOUNCES>(P);
 }
@@ -1563,7 +1563,7 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
 template <bool STATS, uint32_t KINDS>
 __global__ void __launch_bounds__(kTraceThreads, raybuf_warps_per_sm(KINDS) * 32 / kTraceThreads)
     k_trace_ray_buffer(const __grid_constant__ RayBufferParams P) {
-    after_previous();
+    after_previous_alone();
     const Env e = make_env(P.L.tlas, P.L.push.model_info, P.L.textures, RT_MAX_BOUND_IMAGES, P.L.status);
     if (!kinds_selected(P.L.kinds_built, e.blas_kinds, KINDS)) return;
     trace_ray_buffer<STATS, KINDS>(P, e);
