@@ -1044,18 +1044,23 @@ __device__ __forceinline__ int ploc_near(const uint32_t* keys, int x) {
     const uint32_t k = keys[x];
     return k < kPlocNoKey ? x + ploc_offset(k) : x;
 }
-// The nearest neighbour of place x of position i, whose neighbours' areas are
-// in area[o - 1][place of the lower].  FIRST: place 0 is the first position;
-// otherwise there are R places before x.
+// The smaller of `best` and the keys of the neighbours below place x, whose
+// areas are in area[o - 1][place of the lower].  FIRST: place 0 is the first
+// position; otherwise there are R places before x.
+template <bool FIRST, int STRIDE>
+__device__ __forceinline__ uint32_t ploc_below(const uint32_t (*area)[STRIDE], int x, uint32_t best) {
+#pragma unroll
+    for (int o = 1; o <= kPlocRadius; o++)
+        best = min(best, !FIRST || x >= o ? ploc_key(area[o - 1][x - o], -o) : 0xFFFFFFFFu);
+    return best;
+}
+// The nearest of all neighbours.
 template <bool FIRST, int STRIDE>
 __device__ __forceinline__ uint32_t ploc_nearest(const uint32_t (*area)[STRIDE], int x) {
     uint32_t best = 0xFFFFFFFFu;
 #pragma unroll
-    for (int o = 1; o <= kPlocRadius; o++) {
-        const uint32_t down = !FIRST || x >= o ? ploc_key(area[o - 1][x - o], -o) : 0xFFFFFFFFu;
-        best = min(best, min(down, ploc_key(area[o - 1][x], o)));
-    }
-    return best;
+    for (int o = 1; o <= kPlocRadius; o++) best = min(best, ploc_key(area[o - 1][x], o));
+    return ploc_below<FIRST, STRIDE>(area, x, best);
 }
 // Place x (its neighbour at y, odd position, not mutual) asks y when y's
 // position is even, it has no mutual neighbour either and its own nearest is
@@ -1080,8 +1085,12 @@ __device__ __forceinline__ int ploc_partner(const uint32_t* keys, const uint32_t
 // 3 R on each side a halo: boxes for all 512, the areas of the pairs
 // (p, p + 1..R) once each (they do not depend on the order of the boxes) in
 // shared memory, the nearest neighbour (smallest area, the lower position on
-// ties) of the positions within 2 R of an own one, which ask those within R, then the merges of the own positions: the lower of a pair keeps
-// the new node, the higher drops out.  The tile claims its merges' node ids with one atomic
+// ties) of the positions within 2 R of an own one, which ask those within R,
+// then the merges of the own positions: the lower of a pair keeps the new
+// node, the higher drops out.  A position keeps its minimum over those above
+// it in a register and reads back only the areas below (0.3 % of a pass at
+// 163,840 triangles and 0.5 % at 10.5M against reading all 32).  The tile
+// claims its merges' node ids with one atomic
 // (counting down from n - 2) and finds its survivors' output position by
 // look-back over the earlier tiles, so one launch reads each cluster once and
 // writes each survivor once: 32 + 0.8 x 32 bytes per cluster.  (Neighbour
@@ -1145,20 +1154,22 @@ __global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __gri
         s0[t] = make_float4(lo.x, lo.y, lo.z, hi.x);
         s1[t] = make_float2(hi.y, hi.z);
         __syncthreads();
+        uint32_t key = 0xFFFFFFFFu;  // the nearest so far: first of the positions above
         if (t < T - R) {
 #pragma unroll
             for (int o = 1; o <= R; o++) {
                 const float4 c = s0[t + o];
                 const float2 d = s1[t + o];
-                area[o - 1][t] = __float_as_uint(merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y, c.z,
-                                                                  c.w, d.x, d.y)) & ~31u;
+                const uint32_t bits = __float_as_uint(merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y,
+                                                                       c.z, c.w, d.x, d.y)) & ~31u;
+                area[o - 1][t] = bits;
+                key = min(key, ploc_key(bits, o));
             }
         }
         __syncthreads();
         if (t >= R && t < T - R) {
-            uint32_t key = 0xFFFFFFFFu;
-            if (!forced) key = ploc_nearest<false, T - R>(area, t);
-            else if ((i ^ 1) < (int)count) key = ploc_key(0u, (i ^ 1) - i);
+            if (!forced) key = ploc_below<false, T - R>(area, t, key);
+            else key = (i ^ 1) < (int)count ? ploc_key(0u, (i ^ 1) - i) : 0xFFFFFFFFu;
             keys[t] = inside ? key : 0xFFFFFFFFu;
         }
         take[t] = 0xFFFFFFFFu;
