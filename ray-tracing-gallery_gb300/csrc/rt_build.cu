@@ -2264,6 +2264,7 @@ constexpr uint32_t kRefitSmall = 512;
 constexpr uint32_t kRefitNodes = kRefitSmall + 2;  // max_wide_nodes(n, 4)
 __global__ void __launch_bounds__(kRefitSmall) k_refit_small(const RtAccelerationStructureInstance* inst, uint32_t n,
                                                              AsHeader* h) {
+    after_previous();
     __shared__ float4 ibox[2 * kRefitSmall];
     __shared__ float nbox[kRefitNodes][6];
     __shared__ uint32_t arrived[kRefitNodes];
