@@ -443,9 +443,7 @@ RTCORE_API int32_t rt_cmd_trace_rays_batched(rt_ctx* ctx, const RtBatchScene* sc
  *                       large coherent frames; for small images a request
  *                       lasts as long as its slowest tile, so they are
  *                       opt-in (rt_ctx_autotune tries them)
- * Default {128, 0, 20, 0}.  Until a configuration is set (here or by
- * rt_ctx_autotune), a launch of 1.5 M or more ray slots traverses its camera
- * rays as packets; a configuration that was set is used as it is. */
+ * Default {128, 0, 20, 0}. */
 #define RT_TRAVERSAL_PACKET_PRIMARY 0x1u /* camera rays (8x4 pixel tiles) and their mirror / portal bounces */
 #define RT_TRAVERSAL_PACKET_SHADOW 0x2u  /* the shadow rays of each shaded pixel, appended per shading warp */
 /* with PACKET_PRIMARY: the mirror / portal continuation rays of a packet are

@@ -112,7 +112,6 @@ struct rt_ctx {
     std::vector<Workspace> workspaces;
     KernelTimer timer;
     RtTraversalConfig traversal{128, 0, 20, 0};
-    bool traversal_set = false;  // by the caller or the autotuner: used as it is
     // rt_trace_ray_buffer_host: two streams and their device staging (rays, then hits)
     struct HostQuery {
         std::mutex mu;
@@ -600,7 +599,6 @@ int32_t trace_scenes(rt_ctx* ctx, const std::vector<TraceScene>& scenes, const R
     b.status = &ctx->dev->stats.status;
     b.kinds_built = blas_kinds_built();
     b.config = ctx->traversal;
-    b.choose_packets = !ctx->traversal_set;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     uint8_t* ws = nullptr;
     cudaError_t e = ctx_workspace(ctx, s, trace_workspace_bytes(b.scenes, b.count), &ws);
@@ -674,7 +672,6 @@ RTCORE_API int32_t rt_ctx_set_traversal_config(rt_ctx* ctx, const RtTraversalCon
                     config->shared_stack_depth, config->leaf_wait, config->packet_lists);
     MaybeLock l(ctx);
     ctx->traversal = *config;
-    ctx->traversal_set = true;
     return RT_OK;
 }
 
@@ -700,15 +697,10 @@ RTCORE_API int32_t rt_ctx_autotune(rt_ctx* ctx, const RtBatchScene* scenes, uint
         for (uint32_t d : kDepths)
             for (uint32_t w : kWaits) cands.push_back(RtTraversalConfig{b, d, w, 0});
     const RtTraversalConfig saved = ctx->traversal;
-    const bool saved_set = ctx->traversal_set;
-    ctx->traversal_set = true;  // every candidate is timed as it is
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t ce = cudaEventCreate(&e0);
     if (ce == cudaSuccess) ce = cudaEventCreate(&e1);
-    if (ce != cudaSuccess) {
-        ctx->traversal_set = saved_set;
-        return cuda_fail(ce, "rt_ctx_autotune (events)");
-    }
+    if (ce != cudaSuccess) return cuda_fail(ce, "rt_ctx_autotune (events)");
     std::vector<float> med;
     int32_t r = RT_OK;
     auto time_cands = [&](size_t from) {
@@ -751,7 +743,6 @@ RTCORE_API int32_t rt_ctx_autotune(rt_ctx* ctx, const RtBatchScene* scenes, uint
     cudaEventDestroy(e1);
     if (r != RT_OK) {
         ctx->traversal = saved;
-        ctx->traversal_set = saved_set;
         return r;
     }
     const size_t best = fastest();

@@ -139,7 +139,6 @@ struct TraceBatch {
     uint32_t* status;               // device (same block)
     uint32_t kinds_built;           // blas_kinds_built() when the launch was recorded
     RtTraversalConfig config;       // launch shape of the traversal kernels
-    bool choose_packets;            // no configuration was set: packets by the size of the camera-ray list
 };
 // Whether the traversal kernels are built for `c` (block size, shared stack depth, leaf_wait <= 32).
 bool traversal_config_supported(const RtTraversalConfig& c);

@@ -1717,16 +1717,6 @@ void launch_trace_config(const WfParams& P, const RtTraversalConfig& c, bool sta
     launch_trace_kernel<MODE, false, K, 0, kTraceThreads>(P, num_sms, stream);
 }
 
-// Ray slots from which a launch without a set configuration traverses its
-// camera rays as packets.  A packet kernel walks one chunk of 32 rays per warp
-// at a time, so it needs some 16 chunks for each of its 3,040 resident warps
-// before the last ones do not stand out.  Traces in us, one ray per lane /
-// packets, of four scenes (17, 34, 105 and 256 instances): 1280x720 (9 chunks
-// a warp) 370 / 328, 473 / 505, 622 / 693, 1986 / 2045; 1920x1080 (21) 681 /
-// 568, 807 / 827, 1099 / 1026, 4112 / 3617; 3840x2160 (85) 2200 / 1794, 2632 /
-// 2339, 3425 / 2960, 14405 / 11413.
-constexpr uint64_t kPacketSlots = 1500000;
-
 template <int MODE>
 void launch_trace_mode(const WfParams& P, const RtTraversalConfig& c, bool stats, int num_sms, cudaStream_t stream) {
     for_each_variant(P.kinds_built, [&](auto k) {
@@ -1891,19 +1881,17 @@ cudaError_t launch_trace_batch(const TraceBatch& tb, uint8_t* ws, int num_sms, c
         }
     }
     const bool stats = tb.stats != 0;
-    RtTraversalConfig config = tb.config;
-    if (tb.choose_packets && L.slots >= kPacketSlots) config.packet_lists |= RT_TRAVERSAL_PACKET_PRIMARY;
     launch(k_raygen, (uint32_t)((L.slots + 255) / 256), 256, 0, stream, P);
     mark(kKernOther);
     // the traversal follows every mirror / portal bounce itself, so one closest-hit launch and one
     // shading launch cover all bounces
     P.bounce = 0;
-    launch_trace_mode<kModeBounce>(P, config, stats, num_sms, stream);
+    launch_trace_mode<kModeBounce>(P, tb.config, stats, num_sms, stream);
     mark(kKernClosest);
     launch(k_shade, (uint32_t)((L.slots + 127) / 128), 128, 0, stream, P);
     mark(kKernShade);
     if (L.any_shadow) {
-        launch_trace_mode<kModeShadow>(P, config, stats, num_sms, stream);
+        launch_trace_mode<kModeShadow>(P, tb.config, stats, num_sms, stream);
         mark(kKernShadow);
         launch(k_resolve, (uint32_t)((L.pixels + 255) / 256), 256, 0, stream, P);
         mark(kKernOther);

@@ -1,27 +1,10 @@
 """Launch rules by size: what a size rule picks gives the bytes of the general path."""
-import ctypes as C
-
 import numpy as np
 import pytest
 
-from rtgallery import abi, scenes
+from rtgallery import scenes
 
 pytestmark = pytest.mark.gpu
-
-
-@pytest.mark.parametrize("size", [(1496, 1000), (1505, 1003)])  # ray slots just below and above 1.5 M
-def test_unset_configuration_renders_the_same_image(device, size):
-    from rtgallery import host
-
-    scene = scenes.scene_gallery(*size)
-    fresh = host.Device()  # no configuration set: packets for large camera-ray lists
-    image, _, stats = host.render(fresh, scene, radiance=False)
-    config = abi.RtTraversalConfig(128, 0, 20, 0)
-    fresh.check(fresh.lib.rt_ctx_set_traversal_config(fresh.ctx, C.byref(config)))
-    per_lane, _, per_lane_stats = host.render(fresh, scene, radiance=False)
-    fresh.close()
-    assert stats == per_lane_stats and stats["status"] == 0
-    assert np.array_equal(image, per_lane)
 
 
 @pytest.mark.parametrize("count", [1, 31, 33, 3647, 3649, 7300, 20_000, 116_735, 116_737, 130_001])
