@@ -1483,7 +1483,7 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
 // bounded.  Bound: latency, about seven dependent loads per level for small
 // structures; gathers of binary nodes for large ones.  (One launch per level
 // with one thread per task, 15-40 us a level: 163,840 triangles 340 -> 80 us,
-// 10,485,760 triangles 1.3 ms -> 0.4 ms.)
+// 10,485,760 triangles 1.3 -> 0.92 ms.)
 struct CollapseCtx {
     const uint4* inodes;
     const float4* iboxes;  // (lo, primitives below as bits), (hi, -) of each internal node
