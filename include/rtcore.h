@@ -551,7 +551,9 @@ RTCORE_API int32_t rt_server_stats(rt_server* server, RtServeStats* out);
 
 /* Traversal only: one traceRay per RtRay against `tlas`, writing RtHit.
  * `push` may be NULL (then any-hit programs cannot run and candidates are
- * accepted as if opaque). */
+ * accepted as if opaque).  Can be captured into a CUDA graph; replays of one
+ * captured call must not run at the same time as each other (the counter that
+ * hands out its rays is fixed in the graph). */
 RTCORE_API int32_t rt_cmd_trace_ray_buffer(rt_ctx* ctx, uint64_t tlas, const RtPushConstantBufferAddresses* push,
                                            const RtShaderBindingTable* sbt, uint32_t ray_flags,
                                            uint32_t cull_mask, uint32_t sbt_offset, uint64_t rays,

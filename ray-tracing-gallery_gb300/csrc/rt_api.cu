@@ -21,11 +21,16 @@ using namespace rt;
 
 namespace {
 
-constexpr uint32_t kWorkSlots = 256;
+// Fetch counters of ray-buffer launches.  A launch zeroes its own first, on its
+// stream, so one counter serves launch after launch; only two launches that run
+// at the same time must not share one.  Direct launches take the next of
+// kWorkSlots (more than streams keep queued), and captured ones, whose counter
+// stays in their graph, the next of as many others.
+constexpr uint32_t kWorkSlots = 1u << 14;
 
 struct CtxDevice {
     RtStats stats;
-    uint32_t work[kWorkSlots], done[kWorkSlots];  // ray-buffer launches (zero between them)
+    uint32_t work[2][kWorkSlots];  // [captured]
 };
 
 thread_local std::string g_last_error;
@@ -107,7 +112,7 @@ struct rt_ctx {
     int num_sms = 1;
     RtTextureDesc textures[RT_MAX_BOUND_IMAGES];
     CtxDevice* dev = nullptr;
-    std::atomic<uint32_t> work_slot{0};
+    std::atomic<uint32_t> work_slot[2] = {{0}, {0}};  // [captured]
     std::mutex mu;
     std::vector<Workspace> workspaces;
     KernelTimer timer;
@@ -788,9 +793,8 @@ RTCORE_API int32_t rt_cmd_trace_ray_buffer(rt_ctx* ctx, uint64_t tlas, const RtP
     p.collect_stats = (ray_flags & RT_RAY_FLAG_EXT_COLLECT_STATS) ? 1u : 0u;
     p.stats = &ctx->dev->stats;
     p.status = &ctx->dev->stats.status;
-    const uint32_t slot = ctx->work_slot.fetch_add(1) % kWorkSlots;
-    p.work = &ctx->dev->work[slot];
-    p.done = &ctx->dev->done[slot];
+    const int captured = stream_capturing(reinterpret_cast<cudaStream_t>(stream)) ? 1 : 0;
+    p.work = &ctx->dev->work[captured][ctx->work_slot[captured].fetch_add(1) % kWorkSlots];
     p.kinds_built = blas_kinds_built();
     cudaError_t e = launch_trace_ray_buffer(p, ctx->num_sms, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "rt_cmd_trace_ray_buffer");

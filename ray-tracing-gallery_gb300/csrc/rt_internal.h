@@ -179,8 +179,7 @@ struct RayBufferLaunch {
     uint32_t collect_stats;
     RtStats* stats;
     uint32_t* status;
-    uint32_t* work;            // device fetch counter for this launch, zero between launches
-    uint32_t* done;            // blocks that have finished, likewise
+    uint32_t* work;            // device fetch counter for this launch (zeroed by the launcher where it is used)
     uint32_t kinds_built;      // blas_kinds_built() when the launch was recorded
 };
 cudaError_t launch_trace_ray_buffer(const RayBufferLaunch& p, int num_sms, cudaStream_t stream);

@@ -1519,9 +1519,19 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->traversals), (unsigned long long)L.count);
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->primary_rays), (unsigned long long)L.count);
     }
-    const bool spare = (threadIdx.x & 31u) >= rays_per_warp(L.count);
-    while (!spare) {
-        uint32_t my = warp_append(L.work, item == kNoItem);
+    // A list no longer than the grid's lanes: one ray for each lane, warp by
+    // warp, no counter.  Longer ones are fetched from the launch's counter.
+    const uint32_t per_warp = rays_per_warp(L.count), lane = threadIdx.x & 31u;
+    const bool one_each = L.count <= gridDim.x * blockDim.x;
+    uint32_t mine = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp + lane;
+    if (lane >= per_warp) mine = kNoItem;  // (only of a list of one each)
+    for (;;) {
+        uint32_t my = mine;
+        if (one_each) {
+            if (item == kNoItem) mine = kNoItem;
+        } else {
+            my = warp_append(L.work, item == kNoItem);
+        }
         if (item == kNoItem) {
             if (my >= L.count) break;
             item = my;
@@ -1567,12 +1577,6 @@ __global__ void __launch_bounds__(kTraceThreads, raybuf_warps_per_sm(KINDS) * 32
     const Env e = make_env(P.L.tlas, P.L.push.model_info, P.L.textures, RT_MAX_BOUND_IMAGES, P.L.status);
     if (!kinds_selected(P.L.kinds_built, e.blas_kinds, KINDS)) return;
     trace_ray_buffer<STATS, KINDS>(P, e);
-    // the last block to finish leaves the fetch counter at zero for its next launch
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(P.L.done, 1u) == gridDim.x - 1u) {
-        *P.L.work = 0u;
-        *P.L.done = 0u;
-    }
 }
 
 __global__ void k_debug_eval(uint32_t fn, const float* in, float* out, uint32_t count) {
@@ -1725,11 +1729,20 @@ void launch_trace_mode(const WfParams& P, const RtTraversalConfig& c, bool stats
     });
 }
 
+// The fetch counter is zeroed on the launch's own stream, ahead of it, where
+// the list is longer than the grid's lanes: whatever used the counter before,
+// and however that ended, the launch starts at the first ray.
 template <bool STATS, uint32_t KINDS>
-void launch_ray_buffer_kernel(const RayBufferParams& P, int num_sms, cudaStream_t stream) {
+cudaError_t launch_ray_buffer_kernel(const RayBufferParams& P, bool* zeroed, int num_sms, cudaStream_t stream) {
     static int blocks = 0;
     if (!blocks) blocks = persistent_blocks(k_trace_ray_buffer<STATS, KINDS>, kTraceThreads, num_sms);
+    if (!*zeroed && P.L.count > (uint32_t)blocks * kTraceThreads) {
+        const cudaError_t e = cudaMemsetAsync(P.L.work, 0, sizeof(uint32_t), stream);
+        if (e != cudaSuccess) return e;
+        *zeroed = true;
+    }
     launch(k_trace_ray_buffer<STATS, KINDS>, blocks, kTraceThreads, 0, stream, P);
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -1905,12 +1918,15 @@ cudaError_t launch_trace_ray_buffer(const RayBufferLaunch& p, int num_sms, cudaS
     RayBufferParams P;
     P.L = p;
     if (p.count == 0) return cudaSuccess;
+    bool zeroed = false;
+    cudaError_t err = cudaSuccess;
     for_each_variant(p.kinds_built, [&](auto k) {
         constexpr uint32_t K = decltype(k)::value;
-        if (p.collect_stats) launch_ray_buffer_kernel<true, K>(P, num_sms, stream);
-        else launch_ray_buffer_kernel<false, K>(P, num_sms, stream);
+        if (err != cudaSuccess) return;
+        if (p.collect_stats) err = launch_ray_buffer_kernel<true, K>(P, &zeroed, num_sms, stream);
+        else err = launch_ray_buffer_kernel<false, K>(P, &zeroed, num_sms, stream);
     });
-    return cudaGetLastError();
+    return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 cudaError_t launch_debug_eval(uint32_t fn, const float* in, float* out, uint32_t count, cudaStream_t stream) {
