@@ -33,7 +33,11 @@ __device__ __forceinline__ void after_previous() {  // all others
     cudaTriggerProgrammaticLaunchCompletion();
 }
 
-template <class... Params, class... Args>
+// OVERLAP false: the kernel starts when the one before it has completed.  For
+// kernels that read through the non-coherent cache (ld.global.nc, __ldg) what
+// the kernel before may have written: such loads are only defined for data that
+// nothing writes while the kernel is resident.
+template <bool OVERLAP = true, class... Params, class... Args>
 void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     note_launch();
     cudaLaunchAttribute attr{};
@@ -45,7 +49,7 @@ void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaS
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     config.attrs = &attr;
-    config.numAttrs = 1;
+    config.numAttrs = OVERLAP ? 1 : 0;
     cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);  // an error stays for cudaGetLastError
 }
 

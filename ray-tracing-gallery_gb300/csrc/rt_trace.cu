@@ -1741,7 +1741,8 @@ cudaError_t launch_ray_buffer_kernel(const RayBufferParams& P, bool* zeroed, int
         if (e != cudaSuccess) return e;
         *zeroed = true;
     }
-    launch(k_trace_ray_buffer<STATS, KINDS>, blocks, kTraceThreads, 0, stream, P);
+    // the rays, nodes and records that it reads with __ldg can be the work of the kernel before it
+    launch<false>(k_trace_ray_buffer<STATS, KINDS>, blocks, kTraceThreads, 0, stream, P);
     return cudaSuccess;
 }
 
