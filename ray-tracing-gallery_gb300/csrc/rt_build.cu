@@ -881,10 +881,19 @@ __device__ __forceinline__ void load_box_cg(const float4* b, size_t i, float lo[
     hi[0] = h.x; hi[1] = h.y; hi[2] = h.z;
 }
 
+// Adds 1 to a node's arrivals and returns how many came before.  What the
+// caller wrote is visible to whoever arrives later, and what those before it
+// wrote is visible to the caller.
+__device__ __forceinline__ uint32_t arrive(uint32_t* arrivals) {
+    uint32_t before;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(arrivals) : "memory");
+    return before;
+}
+
 // Boxes from the leaves up: a thread climbs until it is the first at a node;
 // the second carries the box of its own child in registers, reads the
 // other's, and goes on.  What the next step needs of the hierarchy is read
-// beside the arrival, so a step waits for the fence, the arrival and one box.
+// beside the arrival, so a step waits for the arrival and one box.
 // (4,096 leaves: 29 -> 22 us.)
 __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const uint32_t* iparent,
                             const float4* sboxes, float4* iboxes, uint32_t* flags, uint32_t n, uint32_t* err) {
@@ -901,8 +910,7 @@ __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const 
         }
         const uint4 nd = inodes[p];
         const uint32_t above = iparent[p];
-        if (!(self & kLeafBit)) __threadfence();  // this thread's box before its arrival
-        if (atomicAdd(&flags[p], 1u) == 0u) return;
+        if (arrive(&flags[p]) == 0u) return;
         const uint32_t other = nd.x == self ? nd.y : nd.x;
         float olo[3], ohi[3];
         if (other & kLeafBit) load_box_cg(sboxes, other & ~kLeafBit, olo, ohi);
@@ -2350,6 +2358,7 @@ __global__ void __launch_bounds__(kRefitSmall) k_refit_small(const RtAcceleratio
                     }
                 }
                 last = __shfl_sync(gmask, last, (int)group);
+                __syncwarp(gmask);  // the first lane has seen the children's boxes: so do the others
                 if (root || !last) break;
                 slot = p;
                 if (guard == 63 && sub == 0u) atomicOr(&err, 1u << RT_ERR_STACK_OVERFLOW);
@@ -2429,7 +2438,6 @@ __global__ void k_refit_nodes(AsHeader* h, const float4* sboxes, uint32_t* count
                 uhi[a] = fmaxf(uhi[a], hi[a]);
             }
         }
-        __threadfence();
         uint32_t p = __ldcg(&parents[slot]);
         if (p == kNone || p >= count) {
             for (int a = 0; a < 3; a++) {
@@ -2439,7 +2447,7 @@ __global__ void k_refit_nodes(AsHeader* h, const float4* sboxes, uint32_t* count
             return;
         }
         int need = internal_children(&nodes[p]);
-        if ((int)atomicAdd(&counters[p], 1u) + 1 < need) return;
+        if ((int)arrive(&counters[p]) + 1 < need) return;
         slot = p;
     }
     atomicOr(err, 1u << RT_ERR_STACK_OVERFLOW);
