@@ -1921,7 +1921,7 @@ struct HeaderStatic {
     uint64_t prim_bytes;
 };
 
-// The header of a finished build but for the 14-DOP (one thread).
+// The header of a finished build, without a 14-DOP (one thread).
 __device__ void write_header(AsHeader* h, const BuildState* st, const HeaderStatic& hs) {
     h->magic = kAsMagic;
     h->type = hs.type;
@@ -1956,6 +1956,7 @@ __device__ void write_header(AsHeader* h, const BuildState* st, const HeaderStat
     const bool sphere = hs.type == kAsTypeBottom && hs.prim_count > 0 && st->radius_bits != 0u && rad <= FLT_MAX;
     for (int k = 0; k < 3; k++) h->sphere_center[k] = sphere ? bounds_center(st, k) : 0.0f;
     h->sphere_radius = sphere ? __fmul_ru(rad, 1.0000010f) : 0.0f;
+    h->dop_count = 0;
     uint64_t nodes_end = hs.nodes_offset + (uint64_t)nc * hs.node_bytes;
     uint64_t par = hs.parents_offset ? align_up(nodes_end, 256) : 0;
     uint64_t par_end = par ? par + (uint64_t)nc * 4 : nodes_end;
@@ -2014,10 +2015,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const Bu
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
     if (t == kFinishThreads - 1) write_header(h, st, hs);
-    if (hs.type != kAsTypeBottom || hs.prim_count == 0u) {
-        if (t == 0) h->dop_count = 0;
-        return;
-    }
+    if (hs.type != kAsTypeBottom || hs.prim_count == 0u) return;
     if (t == 0) {
         bool good = true;
         for (int k = 0; k < 7; k++) {
@@ -2027,9 +2025,8 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const Bu
             phf[2 * k + 1] = -lo;
         }
         ok = good;
-        h->dop_count = 0;
     }
-    __syncthreads();
+    __syncthreads();  // and the header is written: its dop_count can be set below
     if (!ok) return;
     float scale_f = 0.0f;
     for (int j = 0; j < 14; j++) scale_f = fmaxf(scale_f, fabsf(phf[j]));
