@@ -53,9 +53,10 @@ struct BuildState {
     uint32_t depth;
     uint32_t blas_kinds;  // TLAS: kBlasKind* bits of the BLASes its instances enter
     uint32_t merge_counter;  // PLOC merges so far (internal node ids count down from n - 2)
+    uint32_t pair_merges;    // and those of k_ploc_pairs
     uint32_t radius_bits;    // BLAS: largest vertex distance from the bounds centre (float bits, rounded up)
     uint32_t dop_hi[7], dop_lo[7];  // BLAS: largest / smallest vertex projection on each 14-DOP axis (ordered uint)
-    uint32_t ploc_round[kPlocMaxRounds + 1];  // PLOC clusters entering each round | kPloc* bits
+    uint32_t ploc_round[kPlocMaxRounds + 2];  // PLOC clusters entering each round, k_ploc_pairs, the tail | kPloc* bits
     uint32_t ploc_ticket[kPlocMaxRounds];     // next tile of each round
     // collapse: one cache line each for the two counters that every warp adds
     // to and the flag that waiting warps read
@@ -168,6 +169,7 @@ __device__ __forceinline__ void init_state(BuildState* st, uint32_t n) {
         st->depth = 1;
         st->blas_kinds = 0;
         st->merge_counter = 0;
+        st->pair_merges = 0;
         st->radius_bits = 0;
         for (int k = 0; k < 7; k++) {
             st->dop_hi[k] = 0u;
@@ -950,7 +952,8 @@ __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const 
 // builder gave up and merged neighbour pairs, 54 instead of 61.
 //
 // Rounds over more than kPlocSmall clusters are one grid-wide launch each
-// (k_ploc_round; the cluster count stays on the device).  One CTA with every
+// (k_ploc_round; the cluster count stays on the device), and k_ploc_pairs
+// takes a mesh that needs more rounds than were launched.  One CTA with every
 // cluster in shared memory finishes (k_ploc_tail).  When a round leaves more
 // than 31/32 of its clusters (many equal or NaN areas), the next one merges
 // neighbour pairs (i, i ^ 1) instead.
@@ -1267,6 +1270,81 @@ __global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __gri
     }
 }
 
+// What the grid-wide rounds have left above kPlocSmall clusters: neighbour
+// pairs, pairs of pairs and so on until kPlocSmall remain, in one grid-wide
+// launch.  A block takes 2^k consecutive clusters, 2^k the least that leaves
+// kPlocSmall groups, and merges them level by level in their own places; a
+// merge's node id follows from its level and position, so the tree is the one
+// that whole levels would give.  Almost always there is nothing to do: the
+// rounds are enough for any mesh whose clusters merge at about the rates below,
+// and a mesh for which they are not (every cluster's nearest neighbour has a
+// nearer one, round after round: nested shells, each around the last) still
+// takes one pass over its clusters instead of many by one block.
+constexpr uint32_t kPlocPairThreads = 256;
+constexpr uint32_t kPlocPairBlocks = 152 * 2;
+__global__ void __launch_bounds__(kPlocPairThreads) k_ploc_pairs(const __grid_constant__ PlocArgs a, int round) {
+    after_previous();
+    BuildState* st = a.st;
+    const uint32_t word = st->ploc_round[round], count = word & kPlocCount;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (count <= kPlocSmall) {
+        if (first) st->ploc_round[round + 1] = word;
+        return;
+    }
+    float4* cin = a.cbox[(word & kPlocParity) ? 1 : 0];
+    float4* cout = a.cbox[(word & kPlocParity) ? 0 : 1];
+    const uint32_t levels = 32u - (uint32_t)__clz((count - 1u) / kPlocSmall);
+    const uint32_t groups = (uint32_t)(((unsigned long long)count + (1ull << levels) - 1ull) >> levels);
+    const uint32_t merges = st->merge_counter;
+    if (first) {
+        st->ploc_round[round + 1] = groups | ((word & kPlocParity) ^ kPlocParity);
+        st->pair_merges = count - groups;
+    }
+    for (uint32_t g = blockIdx.x; g < groups; g += gridDim.x) {
+        float4* c = cin + 2 * ((size_t)g << levels);  // the group's clusters
+        uint32_t left = min(count - (g << levels), 1u << levels);
+        for (uint32_t level = 0; level < levels; level++) {
+            const uint32_t all = (count + (1u << level) - 1u) >> level;  // clusters of every group at this level
+            const uint32_t claimed = merges + (count - all) + (g << (levels - 1u - level));
+            const uint32_t pairs = (left + 1u) / 2u;  // the last may be one cluster alone
+            float4* out = level + 1u == levels ? cout + 2 * (size_t)g : c;
+            for (uint32_t base = 0; base < pairs; base += blockDim.x) {  // q is stored behind every later read
+                const uint32_t q = base + threadIdx.x;
+                const bool on = q < pairs, two = on && 2u * q + 1u < left;
+                float4 lo, hi, l2, h2;
+                if (on) {
+                    lo = c[4 * (size_t)q];
+                    hi = c[4 * (size_t)q + 1];
+                }
+                if (two) {
+                    l2 = c[4 * (size_t)q + 2];
+                    h2 = c[4 * (size_t)q + 3];
+                }
+                __syncthreads();
+                if (two) {
+                    const uint32_t claim = claimed + q;
+                    const uint32_t ra = __float_as_uint(lo.w), rb = __float_as_uint(l2.w);
+                    const uint32_t size = __float_as_uint(hi.w) + __float_as_uint(h2.w);
+                    if (claim + 2u <= a.n) {
+                        const uint32_t id = a.n - 2u - claim;
+                        lo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), __uint_as_float(id));
+                        hi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), __uint_as_float(size));
+                        ploc_write_node(a, id, ra, rb, lo, hi, size);
+                    } else {  // more merges than a binary tree over n primitives has
+                        atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
+                    }
+                }
+                if (on) {
+                    out[2 * (size_t)q] = lo;
+                    out[2 * (size_t)q + 1] = hi;
+                }
+                __syncthreads();
+            }
+            left = pairs;
+        }
+    }
+}
+
 // The last rounds, in one CTA with every cluster (at most kPlocSmall, one
 // per thread) in shared memory; node ids follow from the round's prefix sums.
 // The areas of the pairs (i, i + 1..R) are computed once each: warp w takes
@@ -1276,9 +1354,7 @@ __global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __gri
 // latency between them, about 1 us a round.  Meshes with fans of slivers (the
 // poles of a sphere) take many rounds: 163,840 triangles 75, 4,096 triangles
 // 40.  (With both directions evaluated by every thread of the block in each
-// round, the tail of those took 535 and 290 us.)  If the grid-wide rounds
-// left more than kPlocSmall clusters, neighbour pairs are merged in global
-// memory until that few remain.
+// round, the tail of those took 535 and 290 us.)
 struct PlocTailShared {
     float4 s0[kPlocSmall + kPlocRadius];  // lo, hi.x; behind the last cluster, boxes of infinite area
     float2 s1[kPlocSmall + kPlocRadius];  // hi.y, hi.z
@@ -1406,48 +1482,12 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
     BuildState* st = a.st;
     const uint32_t tid = threadIdx.x;
     const uint32_t word = st->ploc_round[round];
-    uint32_t count = word & kPlocCount, merges = st->merge_counter;
-    float4* c = a.cbox[(word & kPlocParity) ? 1 : 0];
-    if (count == 0u) {
+    const uint32_t count = word & kPlocCount;
+    uint32_t merges = st->merge_counter + st->pair_merges;
+    const float4* c = a.cbox[(word & kPlocParity) ? 1 : 0];
+    if (count == 0u || count > kPlocSmall) {  // neither ever leaves the rounds and k_ploc_pairs
         if (tid == 0) atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
         return;
-    }
-    while (count > kPlocSmall) {  // pair q takes positions 2q, 2q + 1 and is stored at q (behind every later read)
-        const uint32_t pairs = (count + 1u) / 2u;
-        for (uint32_t base = 0; base < pairs; base += blockDim.x) {
-            const uint32_t q = base + tid;
-            float4 lo, hi, l2, h2;
-            const bool on = q < pairs, two = on && 2u * q + 1u < count;
-            if (on) {
-                lo = __ldcg(&c[4 * (size_t)q]);
-                hi = __ldcg(&c[4 * (size_t)q + 1]);
-            }
-            if (two) {
-                l2 = __ldcg(&c[4 * (size_t)q + 2]);
-                h2 = __ldcg(&c[4 * (size_t)q + 3]);
-            }
-            __syncthreads();
-            if (two) {
-                const uint32_t claim = merges + q;
-                const uint32_t ra = __float_as_uint(lo.w), rb = __float_as_uint(l2.w);
-                const uint32_t size = __float_as_uint(hi.w) + __float_as_uint(h2.w);
-                if (claim + 2u <= a.n) {
-                    const uint32_t id = a.n - 2u - claim;
-                    lo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), __uint_as_float(id));
-                    hi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), __uint_as_float(size));
-                    ploc_write_node(a, id, ra, rb, lo, hi, size);
-                } else {
-                    atomicOr(&st->error, 1u << RT_ERR_BAD_AS);
-                }
-            }
-            if (on) {
-                c[2 * (size_t)q] = lo;
-                c[2 * (size_t)q + 1] = hi;
-            }
-            __syncthreads();
-        }
-        merges += count / 2u;
-        count = pairs;
     }
     if (tid < count) {
         float4 lo, hi;
@@ -2524,8 +2564,8 @@ inline bool uses_ploc(uint32_t n, bool top, uint32_t build_flags) {
 
 // Grid-wide PLOC rounds for n > kPlocSmall primitives: enough to reach
 // kPlocSmall clusters at the measured survival rates, and 2 more.  A round
-// that finds kPlocSmall or fewer does nothing (2.5 us); k_ploc_tail finishes
-// any count.
+// that finds kPlocSmall or fewer does nothing (2.5 us); k_ploc_pairs takes
+// what is above it after the last.
 inline int ploc_grid_rounds(uint32_t n) {
     if (n <= kPlocSmall) return 0;
     const double x = kPlocFirstRate * (double)n / (double)kPlocSmall;
@@ -2721,7 +2761,8 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
                 cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(PlocTailShared));
             if (smem_ok != cudaSuccess) return smem_ok;
-            launch(k_ploc_tail, 1, kPlocSmall, sizeof(PlocTailShared), stream, pa, rounds);
+            if (rounds > 0) launch(k_ploc_pairs, kPlocPairBlocks, kPlocPairThreads, 0, stream, pa, rounds);
+            launch(k_ploc_tail, 1, kPlocSmall, sizeof(PlocTailShared), stream, pa, rounds > 0 ? rounds + 1 : 0);
         } else {
             launch(k_gather_boxes, blocks_for(n, T), T, 0, stream, boxes, vals[cur], n, sboxes);
         }
