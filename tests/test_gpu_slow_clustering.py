@@ -20,7 +20,7 @@ SHELLS, RADIUS, TAIL = 30, 16, 1024
 def _rounds(n):
     """Grid-wide clustering rounds of a build of n primitives (more than the tail takes)."""
     x = 0.62 * n / TAIL
-    return 1 + (math.ceil(math.log(x) / -math.log(0.765)) if x > 1 else 0) + 2
+    return 1 + (math.ceil(math.log(x) / -math.log(0.765)) if x > 1 else 0) + 6
 
 
 def _round(areas, first):
@@ -68,13 +68,13 @@ def _shells(stacks):
     return scenes.Model(pos, np.zeros_like(pos), np.zeros((len(pos), 2), np.float32), [scenes.Geometry(idx)], "shells")
 
 
-@pytest.mark.parametrize("stacks", [40, 64, 200, 4096])
+@pytest.mark.parametrize("stacks", [46, 64, 200, 4096])
 def test_the_rounds_leave_too_many(stacks):
     assert stacks * _left(_rounds(stacks * SHELLS)) > TAIL
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("stacks", [40, 64, 200, 4096])
+@pytest.mark.parametrize("stacks", [46, 64, 200, 4096])
 @pytest.mark.parametrize("flags", [TRACE, TRACE | W4, TRACE | Q], ids=["w8", "w4", "q8"])
 def test_nested_shells(device, stacks, flags):
     _check(device, _scene(_shells(stacks), scenes.affine(np.eye(3), [0, 0, 0])[None]), flags,
