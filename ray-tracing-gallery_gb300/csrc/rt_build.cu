@@ -946,10 +946,11 @@ __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const 
 // neighbour also merges with its nearest neighbour j when j is at an even
 // position, has no mutual neighbour either, and its own nearest is hardly
 // nearer (kPlocNear): j takes the best of those that ask.  That leaves 0.75
-// per round (2.6M-triangle sphere: 26 rounds to 1024 clusters instead of 134)
-// at the same surface-area cost: on ten meshes and instance sets within 1 %
-// of mutual pairs only, simulated on the host; for the spheres, where the old
-// builder gave up and merged neighbour pairs, 54 instead of 61.
+// per round (2.6M-triangle sphere: 26 rounds to 1024 clusters instead of 134).
+// Nodes visited a ray, random rays, mutual pairs only -> now: spheres of 164k /
+// 1M / 10.5M triangles 8.75 / 9.91 / 13.98 -> 8.70 / 9.66 / 12.24, 300k
+// scattered triangles 91.2 -> 85.2, hair 25.5 -> 24.1, a torus 9.28 -> 9.53,
+// 200k triangles of very different sizes 82.4 -> 83.9.
 //
 // Rounds over more than kPlocSmall clusters are one grid-wide launch each
 // (k_ploc_round; the cluster count stays on the device), and k_ploc_pairs
@@ -1036,59 +1037,91 @@ __device__ uint32_t ploc_look_back(const unsigned long long* desc, uint32_t roun
     }
 }
 
-// A neighbour and the area of the merge with it as one word: the area's bits
-// without the lowest five (a merge is chosen by the area to 2^-18 of itself),
-// and there the neighbour's offset, -R..-1 as 0..15 and 1..R as 16..31.  The
-// smallest word is the nearest neighbour, the lower position on ties.  No
-// finite area reaches kPlocNoKey (infinity and NaN are above it).
-static_assert(kPlocRadius == 16, "32 offsets");
-constexpr uint32_t kPlocNoKey = 0x7F800000u;
-__device__ __forceinline__ uint32_t ploc_key(uint32_t area_bits, int offset) {
-    return area_bits | (uint32_t)(offset < 0 ? offset + kPlocRadius : offset + kPlocRadius - 1);
-}
-__device__ __forceinline__ int ploc_offset(uint32_t key) {
-    const int k = (int)(key & 31u);
-    return k < kPlocRadius ? k - kPlocRadius : k - kPlocRadius + 1;
-}
-// The place of place x's nearest neighbour; x itself if it has none.
-__device__ __forceinline__ int ploc_near(const uint32_t* keys, int x) {
-    const uint32_t k = keys[x];
-    return k < kPlocNoKey ? x + ploc_offset(k) : x;
-}
-// The smaller of `best` and the keys of the neighbours below place x, whose
-// areas are in area[o - 1][place of the lower].  FIRST: place 0 is the first
-// position; otherwise there are R places before x.
+// The best of the neighbours looked at so far: the area of the merge with it
+// (float bits) and its offset.  Areas are compared whole; the lower position
+// wins ties.  Areas from kPlocNoArea on (infinity and NaN) are no neighbour.
+constexpr uint32_t kPlocNoArea = 0x7F800000u;
+struct PlocBest {
+    uint32_t area = 0xFFFFFFFFu;
+    int offset = 0;
+    // neighbours in ascending position above all seen so far
+    __device__ __forceinline__ void higher(uint32_t a, int o) {
+        bool keep;
+        area = __vibmin_u32(area, a, &keep);
+        offset = keep ? offset : o;
+    }
+    // neighbours in descending position below all seen so far
+    __device__ __forceinline__ void lower(uint32_t a, int o) {
+        bool take;
+        area = __vibmin_u32(a, area, &take);
+        offset = take ? o : offset;
+    }
+};
+// The nearest neighbours of a round: `area` of the merge, `offset` of its place (0: none).
+struct PlocNear {
+    const uint32_t* area;
+    const int8_t* offset;
+    __device__ __forceinline__ int operator()(int x) const { return x + offset[x]; }  // x itself if it has none
+};
+// The neighbours below place x, whose areas are in area[o - 1][place of the
+// lower].  FIRST: place 0 is the first position; otherwise there are R places
+// before x.
 template <bool FIRST, int STRIDE>
-__device__ __forceinline__ uint32_t ploc_below(const uint32_t (*area)[STRIDE], int x, uint32_t best) {
+__device__ __forceinline__ void ploc_below(const uint32_t (*area)[STRIDE], int x, int from, int to, PlocBest& best) {
 #pragma unroll
-    for (int o = 1; o <= kPlocRadius; o++)
-        best = min(best, !FIRST || x >= o ? ploc_key(area[o - 1][x - o], -o) : 0xFFFFFFFFu);
+    for (int o = from; o <= to; o++) best.lower(!FIRST || x >= o ? area[o - 1][x - o] : 0xFFFFFFFFu, -o);
+}
+// The nearest of all neighbours (of the tail's clusters).  Four runs at once:
+// the comparisons of one wait for each other.
+template <int STRIDE>
+__device__ __forceinline__ PlocBest ploc_nearest(const uint32_t (*area)[STRIDE], int x) {
+    constexpr int R = kPlocRadius, H = R / 2;
+    PlocBest best, far, below, far_below;
+#pragma unroll
+    for (int o = 1; o <= H; o++) {
+        best.higher(area[o - 1][x], o);
+        far.higher(area[o + H - 1][x], o + H);
+    }
+    ploc_below<true>(area, x, 1, H, below);
+    ploc_below<true>(area, x, H + 1, R, far_below);
+    best.higher(far.area, far.offset);
+    best.lower(below.area, below.offset);
+    best.lower(far_below.area, far_below.offset);
     return best;
 }
-// The nearest of all neighbours.
-template <bool FIRST, int STRIDE>
-__device__ __forceinline__ uint32_t ploc_nearest(const uint32_t (*area)[STRIDE], int x) {
-    uint32_t best = 0xFFFFFFFFu;
-#pragma unroll
-    for (int o = 1; o <= kPlocRadius; o++) best = min(best, ploc_key(area[o - 1][x], o));
-    return ploc_below<FIRST, STRIDE>(area, x, best);
+__device__ __forceinline__ void ploc_store(uint32_t* area, int8_t* offset, int x, const PlocBest& best) {
+    area[x] = best.area;
+    offset[x] = (int8_t)(best.area < kPlocNoArea ? best.offset : 0);
+}
+// An asker in one word, the best the smallest (PLOC++, Benthin et al., 2022,
+// packs a distance and an offset so, but drops bits of the distance): how much
+// its area is above the asked place's own nearest, in units in the last place,
+// and in the low five bits its offset from there (-R..-1 as 0..15, 1..R as
+// 16..31), so that the lower position wins ties.  The difference is not
+// negative, since the asker is among the asked place's neighbours, and
+// kPlocNear keeps it below 2^22.
+__device__ __forceinline__ uint32_t ploc_asker(const PlocNear& near, int x, int y) {
+    const int o = x - y;
+    return (near.area[x] - near.area[y]) << 5 | (uint32_t)(o < 0 ? o + kPlocRadius : o + kPlocRadius - 1);
 }
 // Place x (its neighbour at y, odd position, not mutual) asks y when y's
 // position is even, it has no mutual neighbour either and its own nearest is
 // hardly nearer.
-__device__ __forceinline__ void ploc_ask(const uint32_t* keys, uint32_t* take, int x, int y) {
-    const uint32_t mine = keys[x], theirs = keys[y];
-    const int z = ploc_near(keys, y);
-    if (z != y && ploc_near(keys, z) == y) return;
-    if (__uint_as_float(mine & ~31u) <= __uint_as_float(theirs & ~31u) * kPlocNear)
-        atomicMin(&take[y], ploc_key(mine & ~31u, x - y));
+__device__ __forceinline__ void ploc_ask(const PlocNear& near, uint32_t* take, int x, int y) {
+    const int z = near(y);
+    if (z != y && near(z) == y) return;
+    if (__uint_as_float(near.area[x]) <= __uint_as_float(near.area[y]) * kPlocNear)
+        atomicMin(&take[y], ploc_asker(near, x, y));
 }
-// The place that place x merges with (x itself: none).  odd: of its position.
-__device__ __forceinline__ int ploc_partner(const uint32_t* keys, const uint32_t* take, int x, int y, bool mutual,
+// The place that place x merges with (x itself: none).  y: its nearest (x
+// itself if it has none); odd: of its position.
+__device__ __forceinline__ int ploc_partner(const PlocNear& near, const uint32_t* take, int x, int y, bool mutual,
                                             bool odd) {
     if (mutual) return y;
-    if (!odd) return take[x] != 0xFFFFFFFFu ? x + ploc_offset(take[x]) : x;
-    return y != x && take[y] == ploc_key(keys[x] & ~31u, x - y) ? y : x;
+    if (odd) return y != x && take[y] == ploc_asker(near, x, y) ? y : x;
+    const uint32_t k = take[x];
+    const int o = (int)(k & 31u);
+    return k == 0xFFFFFFFFu ? x : x + (o < kPlocRadius ? o - kPlocRadius : o - kPlocRadius + 1);
 }
 
 // One round over more than kPlocSmall clusters.  A block takes tiles in
@@ -1101,17 +1134,17 @@ __device__ __forceinline__ int ploc_partner(const uint32_t* keys, const uint32_t
 // node, the higher drops out.  A position keeps its minimum over those above
 // it in a register and reads back only the areas below (0.3 % of a pass at
 // 163,840 triangles and 0.5 % at 10.5M against reading all 32).  The tile
-// claims its merges' node ids with one atomic
-// (counting down from n - 2) and finds its survivors' output position by
-// look-back over the earlier tiles, so one launch reads each cluster once and
-// writes each survivor once: 32 + 0.8 x 32 bytes per cluster.  (Neighbour
+// claims its merges' node ids with one atomic (counting down from n - 2) and
+// finds its survivors' output position by look-back over the earlier tiles, so
+// one launch reads each cluster once and writes each survivor once: 32 + 0.8 x
+// 32 bytes per cluster.  (Neighbour
 // search, merge and compaction as three launches moved about 200 bytes per
 // cluster: PLOC of 10.5M triangles 3.6 ms; of 164k triangles 410 us.)  Bound:
 // shared-memory and arithmetic issue for large counts, latency for small.
 // The first round gathers the Morton-ordered primitive boxes itself.
 // PER_SM: resident blocks, 4 (32 registers) where there are tiles for them
 // all, which overlaps one tile's gathers with more others' arithmetic (10.5M
-// triangles: pass 3.86 -> 3.64 ms), 3 (38 registers) for rounds bound by
+// triangles: pass 3.86 -> 3.64 ms), 3 (39 registers) for rounds bound by
 // the latency of one tile (163,840 triangles 0.5 % faster so).
 template <int PER_SM>
 __global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __grid_constant__ PlocArgs a, int round) {
@@ -1128,9 +1161,11 @@ __global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __gri
     float4* cout = a.cbox[(word & kPlocParity) ? 0 : 1];
     __shared__ float4 s0[T];          // lo, hi.x
     __shared__ float2 s1[T];          // hi.y, hi.z
-    __shared__ uint32_t area[R][T - R];  // area[o - 1][t] = area of the pair (t, t + o), its bits as in ploc_key
-    __shared__ uint32_t keys[T];         // nearest neighbours
+    __shared__ uint32_t area[R][T - R];  // area[o - 1][t] = area of the pair (t, t + o), its bits
+    __shared__ uint32_t near_area[T];    // nearest neighbours
+    __shared__ int8_t near_offset[T];
     __shared__ uint32_t take[T];         // the asker a place takes
+    const PlocNear nearest{near_area, near_offset};
     __shared__ uint32_t warp_sums[2 * T / 32];  // each warp's total, then the totals before it
     __shared__ uint32_t s_tile, s_claim, s_prefix;
     const int t = (int)threadIdx.x;
@@ -1166,41 +1201,40 @@ __global__ void __launch_bounds__(kPlocThreads, PER_SM) k_ploc_round(const __gri
         s0[t] = make_float4(lo.x, lo.y, lo.z, hi.x);
         s1[t] = make_float2(hi.y, hi.z);
         __syncthreads();
-        uint32_t key = 0xFFFFFFFFu;  // the nearest so far: first of the positions above
+        PlocBest best;  // first of the positions above
         if (t < T - R) {
 #pragma unroll
             for (int o = 1; o <= R; o++) {
                 const float4 c = s0[t + o];
                 const float2 d = s1[t + o];
-                const uint32_t bits = __float_as_uint(merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y,
-                                                                       c.z, c.w, d.x, d.y)) & ~31u;
+                const uint32_t bits = __float_as_uint(
+                    merged_half_area(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, c.x, c.y, c.z, c.w, d.x, d.y));
                 area[o - 1][t] = bits;
-                key = min(key, ploc_key(bits, o));
+                best.higher(bits, o);
             }
         }
         __syncthreads();
         if (t >= R && t < T - R) {
-            if (!forced) key = ploc_below<false, T - R>(area, t, key);
-            else key = (i ^ 1) < (int)count ? ploc_key(0u, (i ^ 1) - i) : 0xFFFFFFFFu;
-            keys[t] = inside ? key : 0xFFFFFFFFu;
+            if (!forced) ploc_below<false>(area, t, 1, R, best);
+            else best.area = 0u, best.offset = (i ^ 1) < (int)count ? (i ^ 1) - i : 0;
+            if (!inside) best.offset = 0;
+            ploc_store(near_area, near_offset, t, best);
         }
         take[t] = 0xFFFFFFFFu;
         __syncthreads();
-        int near = t;
-        bool mutual = false;
-        if (t >= R && t < T - R && inside) {
-            near = ploc_near(keys, t);
-            if (near >= 2 * R && near < T - 2 * R) {  // the neighbours that an own place can have
-                mutual = near != t && ploc_near(keys, near) == t;
-                if (near != t && !mutual && (i & 1) && !((i + near - t) & 1)) ploc_ask(keys, take, t, near);
-            }
+        if (t >= R && t < T - R && inside && (i & 1)) {
+            const int near = nearest(t);
+            if (near >= 2 * R && near < T - 2 * R &&  // the neighbours that an own place can have
+                ((near - t) & 1) && nearest(near) != t)
+                ploc_ask(nearest, take, t, near);
         }
         __syncthreads();
         uint32_t k = 0u;
         bool merging = false;
         int tj = t;
         if (own) {
-            tj = ploc_partner(keys, take, t, near, mutual, (i & 1) != 0);  // t itself: no merge
+            const int near = nearest(t);
+            tj = ploc_partner(nearest, take, t, near, near != t && nearest(near) == t, (i & 1) != 0);  // t itself: no merge
             merging = tj > t;
             k = tj < t ? 0u : 1u;
         }
@@ -1360,9 +1394,10 @@ struct PlocTailShared {
     float4 s0[kPlocSmall + kPlocRadius];  // lo, hi.x; behind the last cluster, boxes of infinite area
     float2 s1[kPlocSmall + kPlocRadius];  // hi.y, hi.z
     uint2 ref[kPlocSmall];                // binary reference, primitives below
-    uint32_t keys[kPlocSmall];            // nearest neighbours
+    uint32_t near_area[kPlocSmall];       // nearest neighbours
+    int8_t near_offset[kPlocSmall];
     uint32_t take[kPlocSmall];            // the asker a position takes
-    uint32_t area[kPlocRadius][kPlocSmall];  // area[o - 1][i] = area of the pair (i, i + o), its bits as in ploc_key
+    uint32_t area[kPlocRadius][kPlocSmall];  // area[o - 1][i] = area of the pair (i, i + o), its bits
     uint32_t warp_sums[32];
 };
 // Rounds until one of the `count` clusters in s is left; returns the merges
@@ -1372,6 +1407,7 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
                                                      uint32_t* error, W write_node) {
     constexpr int R = kPlocRadius;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const PlocNear nearest{s.near_area, s.near_offset};
     bool forced = false;
     const float inf = INFINITY;
     if (tid < (uint32_t)R) {
@@ -1394,27 +1430,26 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
                     const float4 u = s.s0[i + o];
                     const float2 v = s.s1[i + o];
                     s.area[o - 1u][i] =
-                        __float_as_uint(merged_half_area(p.x, p.y, p.z, p.w, q.x, q.y, u.x, u.y, u.z, u.w, v.x, v.y)) &
-                        ~31u;
+                        __float_as_uint(merged_half_area(p.x, p.y, p.z, p.w, q.x, q.y, u.x, u.y, u.z, u.w, v.x, v.y));
                 }
             }
         }
         __syncthreads();
         const bool here = tid < count;
         if (here) {
-            uint32_t key = 0xFFFFFFFFu;
-            if (!forced) key = ploc_nearest<true, kPlocSmall>(s.area, (int)tid);
-            else if ((tid ^ 1u) < count) key = ploc_key(0u, (int)(tid ^ 1u) - (int)tid);
-            s.keys[tid] = key;
+            PlocBest best;
+            if (!forced) best = ploc_nearest(s.area, (int)tid);
+            else best.area = 0u, best.offset = (tid ^ 1u) < count ? (int)(tid ^ 1u) - (int)tid : 0;
+            ploc_store(s.near_area, s.near_offset, (int)tid, best);
             s.take[tid] = 0xFFFFFFFFu;
         }
         __syncthreads();
         int near = (int)tid;
         bool mutual = false;
         if (here) {
-            near = ploc_near(s.keys, (int)tid);
-            mutual = near != (int)tid && ploc_near(s.keys, near) == (int)tid;
-            if (near != (int)tid && !mutual && (tid & 1u) && !(near & 1)) ploc_ask(s.keys, s.take, (int)tid, near);
+            near = nearest((int)tid);
+            mutual = near != (int)tid && nearest(near) == (int)tid;
+            if (near != (int)tid && !mutual && (tid & 1u) && !(near & 1)) ploc_ask(nearest, s.take, (int)tid, near);
         }
         __syncthreads();
         bool keep = false, merge = false;
@@ -1423,7 +1458,7 @@ __device__ __forceinline__ uint32_t ploc_tail_rounds(PlocTailShared& s, uint32_t
         uint2 r = make_uint2(0u, 0u);
         uint32_t partner = 0u;
         if (here) {
-            const uint32_t j = (uint32_t)ploc_partner(s.keys, s.take, (int)tid, near, mutual, (tid & 1u) != 0u);
+            const uint32_t j = (uint32_t)ploc_partner(nearest, s.take, (int)tid, near, mutual, (tid & 1u) != 0u);
             merge = j > tid;  // tid itself: no merge
             keep = j >= tid;
             p = s.s0[tid];
