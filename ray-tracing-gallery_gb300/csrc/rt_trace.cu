@@ -1507,7 +1507,9 @@ struct RayBufferParams {
     RayBufferLaunch L;
 };
 
-template <bool STATS, uint32_t KINDS>
+// ONE_EACH: a list no longer than the grid's lanes, one ray for each lane, warp
+// by warp.  Longer lists are fetched from the launch's counter.
+template <bool STATS, uint32_t KINDS, bool ONE_EACH>
 __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const Env& e) {
     const RayBufferLaunch& L = P.L;
     const OneScene sv{e};
@@ -1519,26 +1521,28 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->traversals), (unsigned long long)L.count);
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.stats->primary_rays), (unsigned long long)L.count);
     }
-    // A list no longer than the grid's lanes: one ray for each lane, warp by
-    // warp, no counter.  Longer ones are fetched from the launch's counter.
-    const uint32_t per_warp = rays_per_warp(L.count), lane = threadIdx.x & 31u;
-    const bool one_each = L.count <= gridDim.x * blockDim.x;
-    uint32_t mine = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp + lane;
-    if (lane >= per_warp) mine = kNoItem;  // (only of a list of one each)
-    for (;;) {
-        uint32_t my = mine;
-        if (one_each) {
-            if (item == kNoItem) mine = kNoItem;
-        } else {
-            my = warp_append(L.work, item == kNoItem);
-        }
-        if (item == kNoItem) {
-            if (my >= L.count) break;
+    const auto begin = [&] {
+        const float4* rp = reinterpret_cast<const float4*>(L.rays + item);
+        float4 a = __ldg(rp), c = __ldg(rp + 1);
+        trav_begin(s, e, mk3(a.x, a.y, a.z), mk3(c.x, c.y, c.z), a.w, c.w);
+        s.scene = 0;
+    };
+    if (ONE_EACH) {
+        const uint32_t per_warp = rays_per_warp(L.count), lane = threadIdx.x & 31u;
+        const uint32_t my = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp + lane;
+        if (lane < per_warp && my < L.count) {
             item = my;
-            const float4* rp = reinterpret_cast<const float4*>(L.rays + item);
-            float4 a = __ldg(rp), c = __ldg(rp + 1);
-            trav_begin(s, e, mk3(a.x, a.y, a.z), mk3(c.x, c.y, c.z), a.w, c.w);
-            s.scene = 0;
+            begin();
+        }
+    }
+    while (!ONE_EACH || item != kNoItem) {
+        if (!ONE_EACH) {
+            uint32_t my = warp_append(L.work, item == kNoItem);
+            if (item == kNoItem) {
+                if (my >= L.count) break;
+                item = my;
+                begin();
+            }
         }
         const int phase = node_phase(s.entry, RT_TRACE_LEAF_WAIT) ? 1 : 0;
         if (!trav_step<STATS, KINDS>(s, stack, sv, &L.sbt, L.status, L.ray_flags, L.cull_mask, L.sbt_offset, cnt,
@@ -1570,13 +1574,13 @@ __device__ __forceinline__ void trace_ray_buffer(const RayBufferParams& P, const
     flush_counters(L.stats, cnt);
 }
 
-template <bool STATS, uint32_t KINDS>
+template <bool STATS, uint32_t KINDS, bool ONE_EACH>
 __global__ void __launch_bounds__(kTraceThreads, raybuf_warps_per_sm(KINDS) * 32 / kTraceThreads)
     k_trace_ray_buffer(const __grid_constant__ RayBufferParams P) {
     after_previous_alone();
     const Env e = make_env(P.L.tlas, P.L.push.model_info, P.L.textures, RT_MAX_BOUND_IMAGES, P.L.status);
     if (!kinds_selected(P.L.kinds_built, e.blas_kinds, KINDS)) return;
-    trace_ray_buffer<STATS, KINDS>(P, e);
+    trace_ray_buffer<STATS, KINDS, ONE_EACH>(P, e);
 }
 
 __global__ void k_debug_eval(uint32_t fn, const float* in, float* out, uint32_t count) {
@@ -1729,20 +1733,31 @@ void launch_trace_mode(const WfParams& P, const RtTraversalConfig& c, bool stats
     });
 }
 
-// The fetch counter is zeroed on the launch's own stream, ahead of it, where
-// the list is longer than the grid's lanes: whatever used the counter before,
-// and however that ended, the launch starts at the first ray.
+// The rays, nodes and records that the kernel reads with __ldg can be the work of the kernel before it.
+template <bool STATS, uint32_t KINDS, bool ONE_EACH>
+void launch_ray_buffer_kernel(const RayBufferParams& P, int blocks, cudaStream_t stream) {
+    launch<false>(k_trace_ray_buffer<STATS, KINDS, ONE_EACH>, blocks, kTraceThreads, 0, stream, P);
+}
+
+// A list longer than the grid's lanes is fetched from a counter, which is
+// zeroed on the launch's own stream, ahead of it: whatever used the counter
+// before, and however that ended, the launch starts at the first ray.  (Both
+// kinds of list in one kernel, asked in each iteration: 2 % slower.)
 template <bool STATS, uint32_t KINDS>
-cudaError_t launch_ray_buffer_kernel(const RayBufferParams& P, bool* zeroed, int num_sms, cudaStream_t stream) {
-    static int blocks = 0;
-    if (!blocks) blocks = persistent_blocks(k_trace_ray_buffer<STATS, KINDS>, kTraceThreads, num_sms);
-    if (!*zeroed && P.L.count > (uint32_t)blocks * kTraceThreads) {
+cudaError_t launch_ray_buffer_list(const RayBufferParams& P, bool* zeroed, int num_sms, cudaStream_t stream) {
+    static int one_each = 0, fetched = 0;
+    if (!one_each) one_each = persistent_blocks(k_trace_ray_buffer<STATS, KINDS, true>, kTraceThreads, num_sms);
+    if (P.L.count <= (uint32_t)one_each * kTraceThreads) {
+        launch_ray_buffer_kernel<STATS, KINDS, true>(P, one_each, stream);
+        return cudaSuccess;
+    }
+    if (!fetched) fetched = persistent_blocks(k_trace_ray_buffer<STATS, KINDS, false>, kTraceThreads, num_sms);
+    if (!*zeroed) {
         const cudaError_t e = cudaMemsetAsync(P.L.work, 0, sizeof(uint32_t), stream);
         if (e != cudaSuccess) return e;
         *zeroed = true;
     }
-    // the rays, nodes and records that it reads with __ldg can be the work of the kernel before it
-    launch<false>(k_trace_ray_buffer<STATS, KINDS>, blocks, kTraceThreads, 0, stream, P);
+    launch_ray_buffer_kernel<STATS, KINDS, false>(P, fetched, stream);
     return cudaSuccess;
 }
 
@@ -1924,8 +1939,8 @@ cudaError_t launch_trace_ray_buffer(const RayBufferLaunch& p, int num_sms, cudaS
     for_each_variant(p.kinds_built, [&](auto k) {
         constexpr uint32_t K = decltype(k)::value;
         if (err != cudaSuccess) return;
-        if (p.collect_stats) err = launch_ray_buffer_kernel<true, K>(P, &zeroed, num_sms, stream);
-        else err = launch_ray_buffer_kernel<false, K>(P, &zeroed, num_sms, stream);
+        if (p.collect_stats) err = launch_ray_buffer_list<true, K>(P, &zeroed, num_sms, stream);
+        else err = launch_ray_buffer_list<false, K>(P, &zeroed, num_sms, stream);
     });
     return err != cudaSuccess ? err : cudaGetLastError();
 }
