@@ -2641,6 +2641,14 @@ AsLayout AsLayout::make(uint32_t n, bool top, uint32_t build_flags) {
     return l;
 }
 
+// The look-back descriptors of a PLOC build, 8 bytes for each tile of its first
+// round, in a region of about 24 bytes a primitive: what a build with several
+// launches a round once needed.  The scratch sizes that callers query, and the
+// triangle limit of the static-scratch build that follows from them, stay so.
+static uint64_t ploc_desc_bytes(uint64_t n) {
+    return 5 * align_up(n * 4, 256) + align_up((n + 1023) / 1024 * 4, 256) + align_up((n - 1) * 4, 256);
+}
+
 ScratchLayout ScratchLayout::make(uint32_t n, bool top, uint32_t build_flags) {
     const bool quantized = !top && (build_flags & RT_BUILD_QUANTIZED_NODES) != 0;
     const uint64_t cap = max_wide_nodes(n, node_width(build_flags));
@@ -2653,7 +2661,6 @@ ScratchLayout ScratchLayout::make(uint32_t n, bool top, uint32_t build_flags) {
         o = align_up(o + bytes, 256);
         return r;
     };
-    s.sort_blocks = onesweep_partitions((uint32_t)nn);
     s.state = take(kBuildStateBytes);
     s.boxes = take(nn * 32);
     s.sboxes = take(nn * 32);
@@ -2672,15 +2679,9 @@ ScratchLayout ScratchLayout::make(uint32_t n, bool top, uint32_t build_flags) {
     s.perm = take(nn * 4);
     s.ploc = uses_ploc(n, top, build_flags);
     if (s.ploc) {
-        s.ploc_ref0 = take(nn * 4);
-        s.ploc_ref1 = take(nn * 4);
         s.ploc_box0 = take(nn * 32);
         s.ploc_box1 = take(nn * 32);
-        s.ploc_nn = take(nn * 4);
-        s.ploc_keep = take(nn * 4);
-        s.ploc_scan = take(nn * 4);
-        s.ploc_blk = take(((nn + 1023) / 1024) * 4);
-        s.counts = take(ni * 4);
+        s.ploc_desc = take(ploc_desc_bytes(nn));
     }
     s.refit_counters = 0;
     s.build_total = o;
@@ -2727,7 +2728,7 @@ cudaError_t build_common(uint32_t n, bool top, uint32_t build_flags, uint32_t ge
     // once gathered) in Karras builds, so the scratch holds nothing more for them.
     unsigned long long* tasks = reinterpret_cast<unsigned long long*>(sl.ploc ? scratch + sl.iparent : scratch + sl.boxes);
     const uint32_t task_count = n > (top ? kTlasLeafMax : kBlasLeafMax) ? al.max_nodes : 0u;
-    const ZeroedWords zero_ploc = {reinterpret_cast<unsigned long long*>(scratch + sl.ploc_nn), tasks,
+    const ZeroedWords zero_ploc = {reinterpret_cast<unsigned long long*>(scratch + sl.ploc_desc), tasks,
                                    reinterpret_cast<unsigned long long*>(hist), sl.ploc ? blocks_for(n, kPlocTile) : 0u,
                                    sl.ploc ? task_count : 0u,
                                    n > kSortBlockMax ? (uint32_t)(key_sort_state_bytes(n) / 8u) : 0u};

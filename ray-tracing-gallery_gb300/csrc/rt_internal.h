@@ -86,14 +86,12 @@ struct ScratchLayout {
     uint64_t state, temp_inst, refit_counters;
     uint64_t fp32_nodes;       // quantised builds: FP32 nodes before quantisation
     uint64_t perm;             // final primitive order
-    // PLOC builds (RT_BUILD_PREFER_FAST_TRACE): cluster refs / boxes (two
-    // buffers), neighbours, survivor flags and their scan, block totals,
-    // primitives per internal node
-    uint64_t ploc_ref0, ploc_ref1, ploc_box0, ploc_box1, ploc_nn, ploc_keep, ploc_scan, ploc_blk, counts;
+    // PLOC builds (RT_BUILD_PREFER_FAST_TRACE): clusters (two buffers) and the
+    // look-back descriptors of a round's tiles
+    uint64_t ploc_box0, ploc_box1, ploc_desc;
     bool ploc;
     uint64_t build_total;
     uint64_t update_total;
-    uint32_t sort_blocks;
     static ScratchLayout make(uint32_t n, bool top_level, uint32_t build_flags = 0);
 };
 
