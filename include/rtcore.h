@@ -432,7 +432,7 @@ RTCORE_API int32_t rt_cmd_trace_rays_batched(rt_ctx* ctx, const RtBatchScene* sc
  *   block_size          threads per block: 64, 128 or 256 (24 warps per SM each;
  *                       packet kernels 20 for 64 / 128)
  *   shared_stack_depth  traversal-stack entries kept in shared memory: 0, 16,
- *                       24 or 32 (the rest of the 64 live in local memory)
+ *                       24 or 32 (the rest of the 80 live in local memory)
  *   leaf_wait           0..32: a warp runs leaf steps once leaf_wait/32 of its
  *                       lanes wait on one, else node steps
  *   packet_lists        RT_TRAVERSAL_PACKET_* bits: the ray lists a warp
