@@ -179,7 +179,8 @@ __device__ __forceinline__ void init_state(BuildState* st, uint32_t n) {
 }
 __global__ void k_init_state(BuildState* st, uint32_t n) {
     after_previous();
-    init_state(st, n); }
+    init_state(st, n);
+}
 
 __device__ __forceinline__ int find_geometry(const BlasInput& in, uint32_t i) {
     int lo = 0, hi = (int)in.geometry_count - 1;
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_block(uint32_t* k, uint32
 // 8-bit digits, then one kernel per digit.  In a digit pass each block takes
 // the next partition of kOsTile keys from a counter (so every earlier
 // partition belongs to a block that is already running), ranks its keys
-// stably per digit (warp match_any, warps over consecutive chunks), publishes
+// stably per digit (one ballot per bit, warps over consecutive chunks), publishes
 // its per-digit counts, and finds the keys of each digit in all earlier
 // partitions by decoupled look-back: it walks back over their descriptors,
 // adding aggregates until one carries the inclusive prefix.  The tile is then
@@ -961,7 +962,7 @@ __global__ void k_bottom_up(const uint4* inodes, const uint32_t* lparent, const 
 constexpr int kPlocRadius = 16;
 constexpr uint32_t kPlocSmall = 1024;  // clusters the one-CTA tail holds, one per thread
 constexpr float kPlocNear = 1.25f;
-constexpr double kPlocFirstRate = 0.62, kPlocRate = 0.765;  // survivors of the first and of later rounds, at most
+constexpr double kPlocFirstRate = 0.62, kPlocRate = 0.765;  // survivors of the first and of later rounds of closed meshes
 constexpr uint32_t kPlocThreads = 512;
 constexpr uint32_t kPlocTile = kPlocThreads - 6 * kPlocRadius;  // clusters a block owns per tile
 constexpr uint32_t kPlocMaxBlocks = 152 * 4;
@@ -1140,7 +1141,10 @@ __device__ __forceinline__ int ploc_partner(const PlocNear& near, const uint32_t
 // 32 bytes per cluster.  (Neighbour
 // search, merge and compaction as three launches moved about 200 bytes per
 // cluster: PLOC of 10.5M triangles 3.6 ms; of 164k triangles 410 us.)  Bound:
-// shared-memory and arithmetic issue for large counts, latency for small.
+// the barriers between a tile's phases (first round of 2.6M triangles, 132 us:
+// 22.5 of the warps' 38 cycles per issue at a barrier, 28 of 32 lanes, issue 40
+// %, L1 and shared memory 57 %, DRAM 21 %); for small counts the latency of one
+// tile.
 // The first round gathers the Morton-ordered primitive boxes itself.
 // PER_SM: resident blocks, 4 (32 registers) where there are tiles for them
 // all, which overlaps one tile's gathers with more others' arithmetic (10.5M
@@ -1389,7 +1393,8 @@ __global__ void __launch_bounds__(kPlocPairThreads) k_ploc_pairs(const __grid_co
 // latency between them, about 1 us a round.  Meshes with fans of slivers (the
 // poles of a sphere) take many rounds: 163,840 triangles 75, 4,096 triangles
 // 40.  (With both directions evaluated by every thread of the block in each
-// round, the tail of those took 535 and 290 us.)
+// round, the tail of those took 535 and 290 us.)  A tail of 51 us: issue 46 %,
+// 7.9 of the warps' 16 cycles per issue at a barrier.
 struct PlocTailShared {
     float4 s0[kPlocSmall + kPlocRadius];  // lo, hi.x; behind the last cluster, boxes of infinite area
     float2 s1[kPlocSmall + kPlocRadius];  // hi.y, hi.z
@@ -1565,7 +1570,8 @@ __global__ void __launch_bounds__(kPlocSmall) k_ploc_tail(const __grid_constant_
 // a lower slot, which is running too; the launch ends when every primitive is
 // in a leaf (the count travels with the node counter), and every wait is
 // bounded.  Bound: latency, about seven dependent loads per level for small
-// structures; gathers of binary nodes for large ones.  (One launch per level
+// structures; gathers of binary nodes for large ones (2.6M triangles, 215 us:
+// 20.6 cycles per issue on global loads, L2 hits 30 %, DRAM 16 %, issue 28 %).  (One launch per level
 // with one thread per task, 15-40 us a level: 163,840 triangles 340 -> 80 us,
 // 10,485,760 triangles 1.3 -> 0.92 ms.)
 struct CollapseCtx {
@@ -2217,7 +2223,10 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(AsHeader* h, const Bu
 // hundred instances were mostly launch and L2 latency.  Bound: latency, the
 // rounds of the clustering first.  (17 instances 117 -> 33 us,
 // 256 instances 190 -> 66 us.)  Above 1,024 the grid-wide path takes over, with
-// its first round on more than one SM.
+// its first round on more than one SM.  The block needs an SM of its own; behind
+// a query of another stream that fills the GPU it is done 1,019 us (256
+// instances 1,045) after it was queued, the eight launches were after 1,105
+// (1,170): they waited for the same SMs to drain.
 constexpr uint32_t kTlasSmall = 1024;
 static_assert(kTlasSmall == kPlocSmall && kTlasSmall == kSortThreads, "one thread per instance");
 struct TlasSmallArgs {

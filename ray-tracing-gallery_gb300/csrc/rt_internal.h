@@ -18,6 +18,8 @@ void note_launch();
 // completed and its writes are visible, so the launch latency of a short
 // kernel is hidden (programmatic dependent launch).  No block returns before
 // the wait, so a kernel that has completed implies that all before it have.
+// (The ray-buffer query starts behind the kernel before it, see launch(); its
+// wait ends at once.)
 //
 // A kernel that lets the next one become resident early gives it the places
 // of its own finished blocks to wait in.  Behind a traversal, whose last
