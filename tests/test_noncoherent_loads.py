@@ -48,3 +48,11 @@ def test_frames_put_two_kernels_before_the_traversal():
     order = _body(text, "cudaError_t launch_trace_batch(")
     places = [order.index(s) for s in ("launch(k_setup", "launch(k_raygen", "launch_trace_mode<kModeBounce>")]
     assert places == sorted(places)
+
+
+def test_traversals_do_not_let_the_next_kernel_in_early():
+    """Shading samples textures with them, and starts when the traversal before it has completed."""
+    text = _code("rt_trace.cu")
+    for kernel in ("k_trace", "k_trace_packet", "k_trace_ray_buffer"):
+        body = _body(text, kernel + "(const __grid_constant__")
+        assert "after_previous_alone();" in body and "after_previous();" not in body
