@@ -2610,11 +2610,11 @@ inline bool uses_ploc(uint32_t n, bool top, uint32_t build_flags) {
 // Grid-wide PLOC rounds for n > kPlocSmall primitives: enough to reach
 // kPlocSmall clusters at the measured survival rates, and 6 more.  A round
 // that finds kPlocSmall or fewer does nothing (1 us); k_ploc_pairs takes
-// what is above it after the last.  Closed meshes need 4 to 6 rounds fewer;
-// with 2 more instead of 6, scattered triangles, hair and the 10.5M-triangle
-// sphere were left to the pairs, whose trees are worse: 300,000 scattered
-// triangles 89.8 nodes a ray instead of 84.5, 3,000,000 of them (many
-// overlapping) deeper than the traversal's stack.
+// what is above it after the last.  Spheres of up to 1M triangles need 8 rounds
+// fewer, the one of 10.5M 3; with 2 more instead of 6, scattered triangles, hair
+// and the 10.5M-triangle sphere were left to the pairs, whose trees are worse:
+// 300,000 scattered triangles 89.8 nodes a ray instead of 84.5, 3,000,000 of
+// them (many overlapping) deeper than the traversal's stack then was.
 inline int ploc_grid_rounds(uint32_t n) {
     if (n <= kPlocSmall) return 0;
     const double x = kPlocFirstRate * (double)n / (double)kPlocSmall;
